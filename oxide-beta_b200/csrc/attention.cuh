@@ -28,9 +28,10 @@ constexpr int kAttnThreads = 512;
 constexpr int kAttnWarps = kAttnThreads / 32;
 
 struct AttnArgs {
-    const float* qkv;        // [qkv_splits, B, qkv_n] QKV projection output (K-split partials), columns q | k | v
+    const float* qkv;        // [qkv_splits, split_rows, qkv_n] QKV projection output (K-split partials), columns q | k | v
     int qkv_n;
     int qkv_splits;          // partials to add (1 for the small-batch kernels)
+    int split_rows;          // rows between two partials
     uint16_t* out_bf16;      // optional BF16 copy of the output, [B, Nq * D] (input of the tcgen05 O projection)
     int B, Nq, Nkv;
     const float* q_norm;     // [D]
@@ -273,7 +274,7 @@ DEVINL void attn_cta(const AttnArgs& a, float* sm, const int s, const int kvh, c
             for (int e = 0; e < EPT; ++e) {
                 float v = 0.0f;
                 for (int sp = 0; sp < a.qkv_splits; ++sp)
-                    v += __ldcg(a.qkv + ((size_t)sp * a.B + b) * a.qkv_n + col + lane * EPT + e);
+                    v += __ldcg(a.qkv + ((size_t)sp * a.split_rows + b) * a.qkv_n + col + lane * EPT + e);
                 t[e] = v;
                 ss += v * v;
             }

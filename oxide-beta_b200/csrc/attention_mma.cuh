@@ -465,8 +465,8 @@ __global__ void __launch_bounds__(128) attn_merge_kernel(const AttnMmaArgs a) {
 // BF16 high and low parts for attn_mma_kernel. With `q_hl` null only the K/V rows are produced (the
 // SIMT attention kernel norms its own queries); with `write_kv` 0 only the queries (KV-shared layers).
 struct QkvPostArgs {
-    const float* qkv;            // [splits, R, qkv_n] projection output (K-split partials), columns q | k | v
-    int qkv_n, splits, R, Nq, Nkv;
+    const float* qkv;            // [splits, split_rows, qkv_n] projection output (K-split partials), columns q | k | v
+    int qkv_n, splits, split_rows, R, Nq, Nkv;   // split_rows: rows between two partials
     const float* q_norm;
     const float* k_norm;
     const float* inv_freq;
@@ -536,7 +536,7 @@ __global__ void __launch_bounds__(128) qkv_post_kernel(const QkvPostArgs a) {
     for (int e = 0; e < EPT; ++e) t[e] = 0.0f;
     for (int sp = 0; sp < a.splits; ++sp) {                    // K-split partials, in split order
         float v[EPT];
-        ld_f32_vec<EPT>(a.qkv + ((size_t)sp * a.R + row) * a.qkv_n + col + lane * EPT, v);
+        ld_f32_vec<EPT>(a.qkv + ((size_t)sp * a.split_rows + row) * a.qkv_n + col + lane * EPT, v);
 #pragma unroll
         for (int e = 0; e < EPT; ++e) t[e] += v[e];
     }

@@ -112,14 +112,9 @@ DEVINL Cand warp_best(Cand c) {
 // kernel_module.rs:1441-1458 — tanh-GELU through expf, times the up projection.
 DEVINL float gelu_mul(float x, float up) {
     float inner = 0.7978846f * (x + 0.044715f * x * x * x);
-    float t;
-    if (inner >= 0.0f) {
-        float e = expf(-2.0f * inner);
-        t = (1.0f - e) / (1.0f + e);
-    } else {
-        float e = expf(2.0f * inner);
-        t = (e - 1.0f) / (e + 1.0f);
-    }
+    // tanh from e = exp(-2 |inner|) on either side of zero; the sign comes last, so that no lane of a warp branches
+    const float e = expf(-2.0f * fabsf(inner));
+    const float t = copysignf((1.0f - e) / (1.0f + e), inner);
     float gelu = 0.5f * x * (1.0f + t);
     return gelu * up;
 }

@@ -26,6 +26,7 @@
 #include "sampling.cuh"
 #include "batch_ops.cuh"
 #include "tc_gemm.cuh"
+#include "pair_gemm.cuh"
 #include "layered_ops.cuh"
 #include "latent_mma.cuh"
 #include "head_mma.cuh"
@@ -764,18 +765,18 @@ struct oxg4_cache {
     std::vector<void*> owned;                 // every device allocation, for destroy
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     unsigned long long* ts_buf = nullptr;     // [kMaxTimeline][4] optional device timeline
-    // rows a pass over the layers may carry: the batch for a decode step, up to kPrefillRows prompt tokens for a chunk
-    int rows_cap = 0;
-    // prompt chunks: per-row metadata (token, position, sequence) and the attention groups, device + pinned host
-    uint32_t *pf_tok = nullptr, *h_pf_tok = nullptr;
-    int32_t *pf_pos = nullptr, *pf_seq = nullptr, *h_pf_meta = nullptr;
-    int32_t *pf_grp_row0[2] = {nullptr, nullptr}, *pf_grp_n[2] = {nullptr, nullptr};   // attention groups of a chunk, per layer kind (sliding, global)
+    // rows a pass over the layers may carry: the batch for a decode step, up to chunk_rows prompt tokens for a chunk
+    int rows_cap = 0, chunk_rows = 0;
+    bool wide = false;                        // prompt chunks may use the SM-pair projections (csrc/pair_gemm.cuh)
+    size_t part_rows = 0;                     // rows of partial outputs that qkv_part, o_part and down_part hold
+    // prompt chunks: per-row metadata (token, position, sequence), the attention groups per layer kind (sliding, global) and
+    // the runs, chunk_rows entries each, one device block and its pinned image (ChunkMeta)
+    int32_t *pf_meta = nullptr, *h_pf_meta = nullptr;
     // per-layer embeddings: embedding rows (f32 + BF16), context projection output, packed per-layer inputs, scratch
     float *ple_emb = nullptr, *ple_ctx = nullptr, *ple_packed = nullptr, *ple_h = nullptr, *ple_gate = nullptr, *ple_act = nullptr,
           *ple_raw = nullptr;
 
-    // layered models: runs of a chunk (one per sequence in it), recurrent states and token-shift states per layer, scratch
-    int32_t *pf_run_row0 = nullptr, *pf_run_n = nullptr;
+    // layered models: recurrent states and token-shift states per layer, scratch
     std::vector<float*> state, shift;
     void *mix_x = nullptr, *mix_y = nullptr, *x_q = nullptr, *x_u = nullptr, *x_l = nullptr;
     float *xf = nullptr, *in_buf = nullptr, *q_buf = nullptr, *uk_buf = nullptr, *uv_buf = nullptr, *wdec = nullptr, *lat_q = nullptr,
@@ -827,7 +828,28 @@ static int32_t dalloc(oxg4_cache* c, T** p, size_t count, bool zero = true) {
     return OXG4_OK;
 }
 
-constexpr int kPrefillRows = 256;             // most prompt tokens one pass over the layers carries
+constexpr int kPrefillRows = 256;             // prompt tokens whose K/V are appended before they attend (the spare rows of a sliding ring)
+constexpr int kChunkRows = 2048;              // most prompt tokens one pass over the layers carries with the SM-pair projections
+// Prompt chunks of more rows than this take the SM-pair projections. Their tile holds 256 rows whether they exist or not, the
+// weight-streaming kernel (csrc/tc_gemm.cuh) blocks of 16 .. 256 rows. Whole prompts in ms, streaming / pairs: 97 rows ~1B 2.82 /
+// 2.55, ~4B 5.23 / 4.73, six layers of ~27B 1.70 / 1.65; a pass of 64 rows takes as long as one of 97 on the pairs, streaming
+// 2.42, 4.49 and 1.51.
+constexpr int kWideRows = 96;
+
+// The metadata block of a prompt chunk: nine arrays of `cap` 32-bit entries.
+struct ChunkMeta {
+    int32_t* base;
+    int cap;
+    int32_t* at(int i) const { return base + (size_t)i * cap; }
+    uint32_t* tok() const { return (uint32_t*)at(0); }
+    int32_t* pos() const { return at(1); }
+    int32_t* seq() const { return at(2); }
+    int32_t* grp_row0(int kind) const { return at(3 + kind); }
+    int32_t* grp_n(int kind) const { return at(5 + kind); }
+    int32_t* run_row0() const { return at(7); }
+    int32_t* run_n() const { return at(8); }
+    static constexpr int kArrays = 9;
+};
 
 static int32_t tc_gemm_setup();
 static int32_t attn_mma_setup();
@@ -921,7 +943,16 @@ static int32_t cache_build(oxg4_cache* c) {
         part_floats = std::max(part_floats, p.Nkv * c->attn_splits[l] * p.G * (p.D + 2));
         ticket_n = std::max(ticket_n, p.Nkv);
     }
-    const int R = c->rows_cap = std::max(B, kPrefillRows);
+    // models with per-layer embeddings run through the small-batch kernels only (the extra projections per layer
+    // are tiny and have no tcgen05 variant)
+    c->tc_ok = m->es == 2 && m->P == 0 && (m->layered || getenv("OXG4_DISABLE_TCGEN05") == nullptr);
+    // a KV-shared layer attends after its source layer has appended a whole pass, so a pass may not outgrow the ring's spare rows
+    c->wide = c->tc_ok && !m->layered && m->tp == 1 && m->cfg.num_kv_shared_layers == 0;
+    int64_t all_tokens = 0;
+    for (int b = 0; b < B; ++b) all_tokens += c->max_seq[b];
+    c->chunk_rows = c->wide ? (int)std::max<int64_t>(kPrefillRows, std::min<int64_t>(kChunkRows, (all_tokens + 255) / 256 * 256)) : kPrefillRows;
+    c->part_rows = std::max(2 * c->chunk_rows, 2048);
+    const int R = c->rows_cap = std::max(B, c->chunk_rows), A = std::max(B, kPrefillRows);    // A: rows of one attention launch
     const int qw = m->qw_max;
     TRY(dalloc(c, &c->tokens, B));
     TRY(dalloc(c, &c->pos, B));
@@ -936,8 +967,8 @@ static int32_t cache_build(oxg4_cache* c) {
     TRY(dalloc(c, &c->gu_raw, (size_t)R * m->I));
     TRY(dalloc(c, &c->down_raw, (size_t)R * H));
     TRY(dalloc(c, &c->logits, (size_t)B * m->V));
-    TRY(dalloc(c, &c->attn_part, (size_t)R * part_floats));
-    TRY(dalloc(c, &c->attn_ticket, (size_t)R * ticket_n));
+    TRY(dalloc(c, &c->attn_part, (size_t)A * part_floats));
+    TRY(dalloc(c, &c->attn_ticket, (size_t)A * ticket_n));
     TRY(dalloc(c, &c->lm_ticket, (size_t)B + 1));
     TRY(dalloc(c, &c->blk_best, (size_t)B * m->num_sms));
     const int chunks = (m->V + kTopkChunk - 1) / kTopkChunk;
@@ -954,20 +985,11 @@ static int32_t cache_build(oxg4_cache* c) {
     TRY(dalloc(c, &c->topk_scores, (size_t)B * 64));
     if (m->timeline) TRY(dalloc(c, &c->ts_buf, (size_t)kMaxTimeline * 4));
     // prompt chunks
-    TRY(dalloc(c, &c->pf_tok, kPrefillRows));
-    TRY(dalloc(c, &c->pf_pos, kPrefillRows));
-    TRY(dalloc(c, &c->pf_seq, kPrefillRows));
-    for (int k = 0; k < 2; ++k) {
-        TRY(dalloc(c, &c->pf_grp_row0[k], kAmMaxGroups));
-        TRY(dalloc(c, &c->pf_grp_n[k], kAmMaxGroups));
-    }
+    TRY(dalloc(c, &c->pf_meta, (size_t)ChunkMeta::kArrays * c->chunk_rows));
     TRY(dalloc(c, &c->last_h, (size_t)B * H));
     TRY(dalloc(c, &c->last_raw, (size_t)B * H));
     TRY(dalloc(c, &c->last_x, (size_t)B * H));
-    CK(cudaMallocHost(&c->h_pf_tok, sizeof(uint32_t) * kPrefillRows));
-    TRY(dalloc(c, &c->pf_run_row0, kPrefillRows));
-    TRY(dalloc(c, &c->pf_run_n, kPrefillRows));
-    CK(cudaMallocHost(&c->h_pf_meta, sizeof(int32_t) * (4 * kPrefillRows + 4 * kAmMaxGroups)));
+    CK(cudaMallocHost(&c->h_pf_meta, sizeof(int32_t) * ChunkMeta::kArrays * c->chunk_rows));
     {
         std::vector<int32_t> r0(B), ones(B, 1);
         for (int b = 0; b < B; ++b) r0[b] = b;
@@ -981,14 +1003,11 @@ static int32_t cache_build(oxg4_cache* c) {
         TRY(attn_mma_setup());
         int kvh_max = 1;
         for (auto& p : m->layers) kvh_max = std::max(kvh_max, p.Nkv);
-        TRY(dalloc(c, &c->q_hl, (size_t)R * 2 * m->qw_max));
+        TRY(dalloc(c, &c->q_hl, (size_t)A * 2 * m->qw_max));
         const int warps = m->num_sms * 4;                       // upper bound of the consumer warps of a launch
-        TRY(dalloc(c, &c->am_part, ((size_t)std::min(R, kAmMaxGroups) * kvh_max + warps) * kAmRows * (m->Dmax + 2)));
+        TRY(dalloc(c, &c->am_part, ((size_t)std::min(A, kAmMaxGroups) * kvh_max + warps) * kAmRows * (m->Dmax + 2)));
         TRY(dalloc(c, &c->am_pre, (size_t)kAmMaxGroups + 1));
     }
-    // models with per-layer embeddings run through the small-batch kernels only (the extra projections per layer
-    // are tiny and have no tcgen05 variant)
-    c->tc_ok = m->es == 2 && m->P == 0 && (m->layered || getenv("OXG4_DISABLE_TCGEN05") == nullptr);
     c->use_tc = c->tc_ok && B >= (m->layered ? 2 : 8) && B <= kPrefillRows;       // up to 256 sequences: row blocks of 128 / 256 (UMMA N)
     c->ls_qkv.assign(L, 1);
     c->ls_o.assign(L, 1);
@@ -1013,29 +1032,36 @@ static int32_t cache_build(oxg4_cache* c) {
         auto kbs = [](int k) { return (k + kTcTileK - 1) / kTcTileK; };
         const int Bd = std::min(B, kPrefillRows);
         size_t qkv_part_n = 1, o_part_n = 1;
-        auto rows_splits = [&](int sd, int sp) { return (size_t)std::max(sd * B, sp * kPrefillRows); };
+        // chunks that the weight-streaming kernel takes: all of them, or the short ones
+        const int chunk_tc = c->wide ? kWideRows : kPrefillRows;
+        auto rows_splits = [&](int sd, int sp) { return (size_t)std::max(sd * B, sp * chunk_tc); };
+        auto part_rows = [&](int sd, int sp) { return std::max(rows_splits(sd, sp), c->wide ? c->part_rows : 0); };
+        if (c->wide) {
+            TRY(allow_big_smem(pair_gemm_kernel<PG_STORE>));
+            TRY(allow_big_smem(pair_gemm_kernel<PG_GLU>));
+        }
         for (int l = 0; l < L; ++l) {
             const LayerPlan& p = m->layers[l];
             c->ls_qkv[l] = tc_pick_splits(tiles(p.qkv_n), kbs(H), sms, Bd, p.qkv_n, H);
             c->ls_o[l] = tc_pick_splits(tiles(H), kbs(p.qw), sms, Bd, H, p.qw);
             // a full chunk is one 256-row block per weight tile (UMMA N = 256): K-splits fill the SMs where a projection
             // has few tiles; their partial outputs are cheap next to the tensor-core work of 256 rows
-            c->lps_qkv[l] = tc_pick_splits(tiles(p.qkv_n), kbs(H), sms, kPrefillRows, p.qkv_n, H, 1.0);
-            c->lps_o[l] = tc_pick_splits(tiles(H), kbs(p.qw), sms, kPrefillRows, H, p.qw, 1.0);
-            qkv_part_n = std::max(qkv_part_n, rows_splits(c->ls_qkv[l], c->lps_qkv[l]) * p.qkv_n);
-            o_part_n = std::max(o_part_n, rows_splits(c->ls_o[l], c->lps_o[l]) * H);
+            c->lps_qkv[l] = tc_pick_splits(tiles(p.qkv_n), kbs(H), sms, chunk_tc, p.qkv_n, H, 1.0);
+            c->lps_o[l] = tc_pick_splits(tiles(H), kbs(p.qw), sms, chunk_tc, H, p.qw, 1.0);
+            qkv_part_n = std::max(qkv_part_n, part_rows(c->ls_qkv[l], c->lps_qkv[l]) * p.qkv_n);
+            o_part_n = std::max(o_part_n, part_rows(c->ls_o[l], c->lps_o[l]) * H);
         }
         c->s_gu = tc_pick_splits(2 * tiles(m->I), kbs(H), sms, Bd, 2 * m->I, H);
         c->s_down = tc_pick_splits(tiles(H), kbs(m->I), sms, Bd, H, m->I);
-        c->ps_gu = tc_pick_splits(2 * tiles(m->I), kbs(H), sms, kPrefillRows, 2 * m->I, H, 1.0);
-        c->ps_down = tc_pick_splits(tiles(H), kbs(m->I), sms, kPrefillRows, H, m->I, 1.0);
+        c->ps_gu = tc_pick_splits(2 * tiles(m->I), kbs(H), sms, chunk_tc, 2 * m->I, H, 1.0);
+        c->ps_down = tc_pick_splits(tiles(H), kbs(m->I), sms, chunk_tc, H, m->I, 1.0);
         TRY(dalloc(c, &c->x_h, (size_t)R * H));
         TRY(dalloc(c, &c->x_a, (size_t)R * qw));
         TRY(dalloc(c, &c->x_i, (size_t)R * m->I));
         TRY(dalloc(c, &c->qkv_part, qkv_part_n));
         TRY(dalloc(c, &c->o_part, o_part_n));
         TRY(dalloc(c, &c->gu_part, rows_splits(c->s_gu, c->ps_gu) * 2 * m->I));
-        TRY(dalloc(c, &c->down_part, rows_splits(c->s_down, c->ps_down) * H));
+        TRY(dalloc(c, &c->down_part, part_rows(c->s_down, c->ps_down) * H));
         if (m->tp > 1 && c->use_tc && B <= 64) {
             const size_t bytes = sizeof(float) * 2 * (size_t)m->tp * B * H + sizeof(unsigned int) * 2 * kMaxTp;
             CK(cudaMalloc(&c->px_block, bytes));          // own allocation: its IPC handle is exported
@@ -1070,7 +1096,6 @@ extern "C" void oxg4_cache_destroy(oxg4_cache* c) {
     if (c->px_block) cudaFree(c->px_block);
     for (void* p : c->owned) cudaFree(p);
     if (c->h_tokens) cudaFreeHost(c->h_tokens);
-    if (c->h_pf_tok) cudaFreeHost(c->h_pf_tok);
     if (c->h_pf_meta) cudaFreeHost(c->h_pf_meta);
     if (c->h_ctl) cudaFreeHost(c->h_ctl);
     if (c->h_ids) cudaFreeHost(c->h_ids);
@@ -1304,6 +1329,36 @@ static int32_t tc_gemm_launch(const void* w_dev, const void* w1_dev, const void*
     return OXG4_OK;
 }
 
+// Projection of many rows on SM pairs by `plan` (csrc/pair_gemm.cuh): partials out[plan.S, M, ld], or with w1 (gate and up)
+// out_bf16[M, ld] = bf16(act(gate) * up)
+static int32_t pair_gemm_launch(const PairPlan& plan, const void* w, const void* w1, const void* x, int M, int N, int K, int seg_rows,
+                                float* out, uint16_t* out_bf16, int ld, int act, int* err, cudaStream_t st, bool pdl) {
+    if (M < 1 || K % 8 != 0) return fail(OXG4_INVALID_SHAPE, "tcgen05 projection: at least one row and K %% 8 == 0 required");
+    const int n_segs = seg_rows > 0 ? (N + seg_rows - 1) / seg_rows : 1;
+    CUtensorMap mx, mw, mw1;
+    TRY(encode_bf16_2d(&mx, x, (uint64_t)M * n_segs, (uint64_t)K, 128));
+    TRY(encode_bf16_2d(&mw, w, (uint64_t)N, (uint64_t)K, (uint32_t)plan.bn / 2));
+    TRY(encode_bf16_2d(&mw1, w1 ? w1 : w, (uint64_t)N, (uint64_t)K, (uint32_t)plan.bn / 2));
+    PairGemmArgs a{};
+    a.M = M; a.N = N; a.K = K;
+    a.bn = plan.bn; a.cut = plan.cut; a.S = plan.S;
+    a.seg_rows = seg_rows;
+    a.out = out; a.out_bf16 = out_bf16; a.ld = ld; a.act = act;
+    a.err = err;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * plan.pairs);
+    cfg.blockDim = dim3(kPgThreads);
+    cfg.dynamicSmemBytes = pair_gemm_smem_bytes();
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    CK(w1 ? cudaLaunchKernelEx(&cfg, pair_gemm_kernel<PG_GLU>, mx, mw, mw1, a) : cudaLaunchKernelEx(&cfg, pair_gemm_kernel<PG_STORE>, mx, mw, mw1, a));
+    return OXG4_OK;
+}
+
 static int32_t tc_gemm_setup() {
     TRY(allow_big_smem(tc_gemm_kernel<16>));
     TRY(allow_big_smem(tc_gemm_kernel<32>));
@@ -1383,6 +1438,21 @@ struct Launcher {
         if (status != OXG4_OK) return;
         prof_end(kind, e0, e1);
         ++kernels;
+    }
+
+    // projection of many rows on SM pairs: returns the number of partial outputs in `out`; with w1 the gated activation goes
+    // to out_bf16 instead
+    int pair(const char* kind, oxg4_cache* c, int rows, const void* w, const void* w1, const uint16_t* x, int N, int K, float* out,
+             uint16_t* out_bf16, int ld, int act, int seg_rows = 0) {
+        if (status != OXG4_OK) return 1;
+        const PairPlan plan = pair_plan(rows, N, K, w1 != nullptr, seg_rows, c->part_rows, m->num_sms);
+        cudaEvent_t e0, e1;
+        prof_begin(e0, e1);
+        status = pair_gemm_launch(plan, w, w1, x, rows, N, K, seg_rows, out, out_bf16, ld, act, c->tc_err, m->stream, m->use_pdl && !m->profiling);
+        if (status != OXG4_OK) return 1;
+        prof_end(kind, e0, e1);
+        ++kernels;
+        return plan.S;
     }
 
     // profiling steps bracket every launch (collectives included) with a pair of events on the model's stream
@@ -1565,6 +1635,11 @@ struct RowSet {
     const int32_t* run_row0 = nullptr;
     const int32_t* run_n = nullptr;
     std::vector<int> run_len;            // host copy of run_n
+    // a chunk's rows in slices of at most kPrefillRows: a slice appends its K/V and attends before the next one appends
+    struct Slice {
+        int row0, rows, grp0[2], grps[2];    // its groups per layer kind; their first rows count from row0
+    };
+    std::vector<Slice> slices;
     int max_visible = 1;                 // bound on the visible positions of any row (launch geometry only)
 };
 
@@ -1587,9 +1662,10 @@ struct TraceCtx {
 };
 
 // q/k norm + RoPE + v norm + KV append + attention of layer l for the rows of `rs` (decode.rs:99-157,
-// 176-325). qkv: [qkv_splits, R, qkv_n] projection output; the result goes to c->attn_out (+ BF16 copy).
-static void launch_attention(Launcher& ln, oxg4_cache* c, const RowSet& rs, int l, const float* qkv, int qkv_splits,
-                             uint16_t* out_bf16, bool many_rows) {
+// 176-325). qkv: [qkv_splits, split_rows, qkv_n] projection output; the result goes to `out` (+ BF16 copy).
+// split_rows: rows between two partials of qkv; out: [R, qw].
+static void launch_attention(Launcher& ln, oxg4_cache* c, const RowSet& rs, int l, const float* qkv, int qkv_splits, int split_rows,
+                             float* out, uint16_t* out_bf16, bool many_rows) {
     oxg4_model* m = c->m;
     const LayerPlan& p = m->layers[l];
     const int D = p.D, R = rs.R, kind = p.sliding ? 0 : 1;
@@ -1605,7 +1681,7 @@ static void launch_attention(Launcher& ln, oxg4_cache* c, const RowSet& rs, int 
         // norms, RoPE and the K/V append of every row first (a chunk's later tokens are visible to none of its earlier ones
         // only through the causal mask, so all rows may be in the cache before attention starts)
         QkvPostArgs q{};
-        q.qkv = qkv; q.qkv_n = p.qkv_n; q.splits = qkv_splits; q.R = R; q.Nq = m->Nq; q.Nkv = p.Nkv;
+        q.qkv = qkv; q.qkv_n = p.qkv_n; q.splits = qkv_splits; q.split_rows = split_rows; q.R = R; q.Nq = m->Nq; q.Nkv = p.Nkv;
         q.q_norm = p.q_norm; q.k_norm = p.k_norm; q.inv_freq = p.inv_freq; q.rotary_half = p.rotary_dim / 2;
         q.eps = m->cfg.rms_norm_eps;
         q.row_pos = rs.pos; q.row_seq = rs.seq; q.row_tok = rs.tok;
@@ -1630,7 +1706,7 @@ static void launch_attention(Launcher& ln, oxg4_cache* c, const RowSet& rs, int 
         a.part = c->am_part;
         a.pre_out = c->am_pre;
         a.err = c->tc_err;
-        a.out = c->attn_out;
+        a.out = out;
         a.out_bf16 = out_bf16;
         AttnMmaFn fn;
         AttnMergeFn merge;
@@ -1645,6 +1721,7 @@ static void launch_attention(Launcher& ln, oxg4_cache* c, const RowSet& rs, int 
     AttnArgs a{};
     a.qkv = qkv;
     a.qkv_splits = qkv_splits;
+    a.split_rows = split_rows;
     a.out_bf16 = out_bf16;
     a.qkv_n = p.qkv_n;
     a.B = R;
@@ -1669,7 +1746,7 @@ static void launch_attention(Launcher& ln, oxg4_cache* c, const RowSet& rs, int 
     a.min_split = c->min_split;
     a.part = c->attn_part;
     a.ticket = c->attn_ticket;
-    a.out = c->attn_out;
+    a.out = out;
     if ((m->far_prefetch & 2) && !rs.chunk) {
         // the attention kernel of a one-sequence step moves almost no bytes: HBM is idle, so it pulls the up
         // projection's weights (or as much as the cap allows) into L2 for the kernel after next
@@ -1690,6 +1767,30 @@ static void launch_attention(Launcher& ln, oxg4_cache* c, const RowSet& rs, int 
     ln.cluster_x = cl ? a.n_splits : 0;
     ln.go("attn", fn, dim3(a.n_splits, p.Nkv, R), dim3(aw * 32), smem, a);
     ln.cluster_x = 0;
+}
+
+// launch_attention for all rows of a pass: a prompt chunk goes slice by slice
+static void attend_rows(Launcher& ln, oxg4_cache* c, const RowSet& rs, int l, const float* qkv, int qkv_splits, uint16_t* out_bf16,
+                        bool many_rows) {
+    const LayerPlan& p = c->m->layers[l];
+    if (rs.slices.size() <= 1) {
+        launch_attention(ln, c, rs, l, qkv, qkv_splits, rs.R, c->attn_out, out_bf16, many_rows);
+        return;
+    }
+    for (const RowSet::Slice& sl : rs.slices) {
+        RowSet s = rs;
+        s.R = sl.rows;
+        s.tok = rs.tok + sl.row0;
+        s.pos = rs.pos + sl.row0;
+        s.seq = rs.seq + sl.row0;
+        for (int k = 0; k < 2; ++k) {
+            s.grp_row0[k] = rs.grp_row0[k] + sl.grp0[k];
+            s.grp_n[k] = rs.grp_n[k] + sl.grp0[k];
+            s.NG[k] = sl.grps[k];
+        }
+        launch_attention(ln, c, s, l, qkv + (size_t)sl.row0 * p.qkv_n, qkv_splits, rs.R, c->attn_out + (size_t)sl.row0 * p.qw,
+                         out_bf16 ? out_bf16 + (size_t)sl.row0 * p.qw : nullptr, many_rows);
+    }
 }
 
 // Per-layer embeddings (Gemma4-E; ple.rs). Once per pass: the packed per-layer inputs of every row.
@@ -1751,11 +1852,13 @@ static Pending run_layers(oxg4_cache* c, Launcher& ln, const RowSet& rs, bool us
     oxg4_model* m = c->m;
     if (m->layered) return run_layered(c, ln, rs, use_tc, tr);
     const int R = rs.R, L = m->cfg.num_hidden_layers, H = m->H;
-    const int s_gu = rs.chunk ? c->ps_gu : c->s_gu, s_down = rs.chunk ? c->ps_down : c->s_down;
+    const int s_gu = rs.chunk ? c->ps_gu : c->s_gu;
+    int s_down = rs.chunk ? c->ps_down : c->s_down;
+    const bool wide = rs.chunk && c->wide && R > kWideRows;
     if (m->P > 0) ple_prepare(c, ln, rs);
     for (int l = 0; l < L; ++l) {
         const LayerPlan& p = m->layers[l];
-        const int s_qkv = rs.chunk ? c->lps_qkv[l] : c->ls_qkv[l], s_o = rs.chunk ? c->lps_o[l] : c->ls_o[l];
+        int s_qkv = rs.chunk ? c->lps_qkv[l] : c->ls_qkv[l], s_o = rs.chunk ? c->lps_o[l] : c->ls_o[l];
         if (use_tc) {
             // ---- many rows: tcgen05 projections fed by TMA, per-row kernels around them ----
             const int nqkv = p.qkv_n, qw = p.qw;
@@ -1791,13 +1894,15 @@ static Pending run_layers(oxg4_cache* c, Launcher& ln, const RowSet& rs, bool us
                 f.h_in = tr->inject_dev + (size_t)l * R * H;
                 ln.go("norm", rows_norm_kernel<uint16_t>, dim3(R), dim3(kRowsThreads), 0, f);
             }
-            ln.tc("qkv", c, R, p.wqkv, nullptr, c->x_h, nqkv, H, s_qkv, c->qkv_part, nqkv, 0);
-            launch_attention(ln, c, rs, l, c->qkv_part, s_qkv, c->x_a, true);
+            if (wide) s_qkv = ln.pair("qkv", c, R, p.wqkv, nullptr, c->x_h, nqkv, H, c->qkv_part, nullptr, nqkv, 0);
+            else ln.tc("qkv", c, R, p.wqkv, nullptr, c->x_h, nqkv, H, s_qkv, c->qkv_part, nqkv, 0);
+            attend_rows(ln, c, rs, l, c->qkv_part, s_qkv, c->x_a, true);
             // row-split projection under tensor parallelism: without K-splits the kernel writes the rank's partial
             // sum straight into the buffer that is all-reduced (one launch less); with the peer-memory exchange
             // the summation kernel is what pushes it to the peers
             const bool direct = m->tp > 1 && !peer && s_o == 1;
-            ln.tc("o", c, R, p.wo, nullptr, c->x_a, H, qw, s_o, direct ? c->o_raw : c->o_part, H, 0);
+            if (wide) s_o = ln.pair("o", c, R, p.wo, nullptr, c->x_a, H, qw, c->o_part, nullptr, H, 0);
+            else ln.tc("o", c, R, p.wo, nullptr, c->x_a, H, qw, s_o, direct ? c->o_raw : c->o_part, H, 0);
             const size_t bh = (size_t)R * H;
             const dim3 sum_grid((unsigned)((bh / 4 + kRowsThreads - 1) / kRowsThreads));
             PeerExchange none{};
@@ -1822,6 +1927,11 @@ static Pending run_layers(oxg4_cache* c, Launcher& ln, const RowSet& rs, bool us
             n2.eps = m->cfg.rms_norm_eps;
             n2.x = c->x_h;
             ln.go("norm", rows_norm_kernel<uint16_t>, dim3(R), dim3(kRowsThreads), 0, n2);
+            if (wide) {
+                ln.pair("gateup", c, R, p.wgate, p.wup, c->x_h, m->I, H, nullptr, c->x_i, m->I, (int)ACT_GELU_TANH);
+                s_down = ln.pair("down", c, R, p.wdown, nullptr, c->x_i, H, m->I, c->down_part, nullptr, H, 0);
+                continue;
+            }
             ln.tc("gateup", c, R, p.wgate, p.wup, c->x_h, m->I, H, s_gu, c->gu_part, 2 * m->I, 0);
             ln.go("geglu", geglu_rows_kernel, dim3((m->I / 4 + kRowsThreads - 1) / kRowsThreads, R), dim3(kRowsThreads), 0, R,
                   m->I, (const float*)c->gu_part, s_gu, c->x_i, (int)ACT_GELU_TANH);
@@ -1880,7 +1990,7 @@ static Pending run_layers(oxg4_cache* c, Launcher& ln, const RowSet& rs, bool us
                 launch_gemv(ln, "qkv", c, R, a, p.p_qkv, PRO_NORM, EPI_STORE);
             }
         }
-        launch_attention(ln, c, rs, l, c->qkv_raw, 1, nullptr, false);
+        attend_rows(ln, c, rs, l, c->qkv_raw, 1, nullptr, false);
         {   // O projection (decode.rs:159)
             GemvArgs a{};
             a.W0 = p.wo;
@@ -2566,7 +2676,7 @@ extern "C" int32_t oxg4_smoke_decoder_attention(oxg4_model* m, uint32_t token, i
     const LayerPlan& p = m->layers[layer];
     Launcher ln{m};
     smoke_qkv(c, ln, layer);
-    launch_attention(ln, c, smoke_rows(c), layer, c->qkv_raw, 1, nullptr, false);
+    launch_attention(ln, c, smoke_rows(c), layer, c->qkv_raw, 1, 1, c->attn_out, nullptr, false);
     {
         GemvArgs a{};
         a.W0 = p.wo;
@@ -2603,7 +2713,7 @@ extern "C" int32_t oxg4_smoke_cached_attention(oxg4_model* m, oxg4_cache* c, uin
     TRY(smoke_stage(c, token));
     Launcher ln{m};
     smoke_qkv(c, ln, layer);
-    launch_attention(ln, c, smoke_rows(c), layer, c->qkv_raw, 1, nullptr, false);
+    launch_attention(ln, c, smoke_rows(c), layer, c->qkv_raw, 1, 1, c->attn_out, nullptr, false);
     TRY(smoke_finish(c, ln, c->attn_out, attended, (size_t)m->layers[layer].qw));
     c->pos_host[0] += 1;
     CK(cudaMemcpyAsync(c->pos, c->pos_host.data(), sizeof(int32_t), cudaMemcpyHostToDevice, m->stream));
@@ -2634,7 +2744,7 @@ extern "C" int32_t oxg4_profile_count(const oxg4_model* m, const char* kind) {
 }
 
 // Feeds lens[b] (possibly zero) further tokens of every sequence, which continues at its current position. The tokens of
-// all sequences go through the layers in chunks of up to kPrefillRows, each chunk one pass with matrix-shaped projections
+// all sequences go through the layers in chunks of up to chunk_rows, each chunk one pass with matrix-shaped projections
 // (tcgen05 for BF16 weights) and causal / sliding paged attention over the chunk; a chunk may hold the tail of one
 // sequence and the head of the next. `want` (null: none) marks the tokens whose logits are wanted; they are written to
 // `logits` in token order.
@@ -2657,12 +2767,7 @@ static int32_t ingest(oxg4_model* m, oxg4_cache* c, const uint32_t* tokens, cons
     // tokens per attention group, per layer kind (0 sliding, 1 global): 8 / (query heads per KV head)
     int tg[2] = {1, 1};
     for (auto& lp : m->layers) tg[lp.sliding ? 0 : 1] = std::max(1, kAmRows / lp.G);
-    int32_t* h_pos = c->h_pf_meta;
-    int32_t* h_seq = h_pos + kPrefillRows;
-    int32_t* h_g0[2] = {h_seq + kPrefillRows, h_seq + kPrefillRows + 2 * kAmMaxGroups};
-    int32_t* h_gn[2] = {h_g0[0] + kAmMaxGroups, h_g0[1] + kAmMaxGroups};
-    int32_t* h_run0 = h_seq + kPrefillRows + 4 * kAmMaxGroups;
-    int32_t* h_runn = h_run0 + kPrefillRows;
+    const ChunkMeta hm{c->h_pf_meta, c->chunk_rows}, dm{c->pf_meta, c->chunk_rows};
     // wanted rows wait in last_x / last_h + last_raw until B of them (or all) are there: one LM head pass over B rows
     int held = 0;
     int64_t delivered = 0;
@@ -2685,27 +2790,37 @@ static int32_t ingest(oxg4_model* m, oxg4_cache* c, const uint32_t* tokens, cons
     };
     int b = 0, p = 0;                                          // next token to place: sequence b, position p
     while (b < B) {
-        int R = 0, NG[2] = {0, 0};
+        int R = 0, NG[2] = {0, 0}, run_seq = -1;
         std::vector<int> wanted;                               // rows whose logits are asked for
         RowSet rs;
-        while (b < B && R < kPrefillRows) {
+        while (b < B && R < c->chunk_rows) {
             if (lens[b] == 0) { ++b; continue; }
-            const int take = std::min(kPrefillRows - R, lens[b] - p);
+            if (R % kPrefillRows == 0) rs.slices.push_back({R, 0, {NG[0], NG[1]}, {0, 0}});
+            RowSet::Slice& sl = rs.slices.back();
+            const int take = std::min(kPrefillRows - sl.rows, lens[b] - p);
             for (int i = 0; i < take; ++i) {
-                c->h_pf_tok[R + i] = tokens[off[b] + p + i];
-                h_pos[R + i] = c->pos_host[b] + p + i;
+                hm.tok()[R + i] = tokens[off[b] + p + i];
+                hm.pos()[R + i] = c->pos_host[b] + p + i;
                 if (want && want[off[b] + p + i]) wanted.push_back(R + i);
-                h_seq[R + i] = b;
+                hm.seq()[R + i] = b;
             }
             for (int k = 0; k < 2; ++k)
                 for (int i = 0; i < take; i += tg[k]) {
-                    h_g0[k][NG[k]] = R + i;
-                    h_gn[k][NG[k]] = std::min(tg[k], take - i);
+                    hm.grp_row0(k)[NG[k]] = sl.rows + i;
+                    hm.grp_n(k)[NG[k]] = std::min(tg[k], take - i);
                     ++NG[k];
+                    ++sl.grps[k];
                 }
-            h_run0[rs.run_len.size()] = R;
-            h_runn[rs.run_len.size()] = take;
-            rs.run_len.push_back(take);
+            if (run_seq == b) {                                // the same run goes on in the next slice
+                hm.run_n()[rs.run_len.size() - 1] += take;
+                rs.run_len.back() += take;
+            } else {
+                hm.run_row0()[rs.run_len.size()] = R;
+                hm.run_n()[rs.run_len.size()] = take;
+                rs.run_len.push_back(take);
+                run_seq = b;
+            }
+            sl.rows += take;
             R += take;
             p += take;
             rs.max_visible = std::max(rs.max_visible, c->pos_host[b] + p);
@@ -2713,28 +2828,20 @@ static int32_t ingest(oxg4_model* m, oxg4_cache* c, const uint32_t* tokens, cons
         }
         if (R == 0) break;
         cudaStream_t st = m->stream;
-        CK(cudaMemcpyAsync(c->pf_tok, c->h_pf_tok, sizeof(uint32_t) * R, cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(c->pf_pos, h_pos, sizeof(int32_t) * R, cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(c->pf_seq, h_seq, sizeof(int32_t) * R, cudaMemcpyHostToDevice, st));
-        for (int k = 0; k < 2; ++k) {
-            CK(cudaMemcpyAsync(c->pf_grp_row0[k], h_g0[k], sizeof(int32_t) * NG[k], cudaMemcpyHostToDevice, st));
-            CK(cudaMemcpyAsync(c->pf_grp_n[k], h_gn[k], sizeof(int32_t) * NG[k], cudaMemcpyHostToDevice, st));
-        }
-        CK(cudaMemcpyAsync(c->pf_run_row0, h_run0, sizeof(int32_t) * rs.run_len.size(), cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(c->pf_run_n, h_runn, sizeof(int32_t) * rs.run_len.size(), cudaMemcpyHostToDevice, st));
+        CK(cudaMemcpyAsync(c->pf_meta, c->h_pf_meta, sizeof(int32_t) * ChunkMeta::kArrays * c->chunk_rows, cudaMemcpyHostToDevice, st));
         const bool prof = getenv("GEMMA4_PROFILE") != nullptr && getenv("OXG4_PROFILE_PREFILL") != nullptr;
         m->profiling = prof || m->profile_ingest;           // events around every launch of the chunk (a measurement aid, like the reference's GEMMA4_PROFILE)
         Launcher ln{m};
         rs.R = R;
-        rs.run_row0 = c->pf_run_row0;
-        rs.run_n = c->pf_run_n;
-        rs.tok = c->pf_tok;
-        rs.pos = c->pf_pos;
-        rs.seq = c->pf_seq;
+        rs.run_row0 = dm.run_row0();
+        rs.run_n = dm.run_n();
+        rs.tok = dm.tok();
+        rs.pos = dm.pos();
+        rs.seq = dm.seq();
         rs.chunk = true;
         for (int k = 0; k < 2; ++k) {
-            rs.grp_row0[k] = c->pf_grp_row0[k];
-            rs.grp_n[k] = c->pf_grp_n[k];
+            rs.grp_row0[k] = dm.grp_row0(k);
+            rs.grp_n[k] = dm.grp_n(k);
             rs.NG[k] = NG[k];
         }
         const Pending pd = run_layers(c, ln, rs, use_tc, false, false, nullptr);
@@ -3157,6 +3264,51 @@ extern "C" int32_t oxg4_debug_tc_gemm(const uint16_t* w_host, const uint16_t* x_
     cudaEventDestroy(e1);
     cudaFree(w); cudaFree(x); cudaFree(o); cudaFree(e);
     return s;
+}
+
+// SM-pair projection, stand-alone entry of its parity tests: out[M, N] = x[M, K] . w[N, K]^T, or with w1 the BF16 value of
+// gelu(x . w^T) * (x . w1^T); seg_rows > 0: rows of w from s * seg_rows on multiply rows s * M .. of x.
+extern "C" int32_t oxg4_debug_pair_gemm(const uint16_t* w_host, const uint16_t* w1_host, const uint16_t* x_host, int32_t N, int32_t K,
+                                        int32_t M, int32_t seg_rows, float* out_host, int32_t* slots_or_null) {
+    if (!w_host || !x_host || !out_host) return fail(OXG4_INVALID_ARGUMENT, "null argument");
+    if (M < 1 || M > kChunkRows || N < 1 || K < 8 || K % 8 != 0 || seg_rows < 0 || seg_rows % 128 != 0 || (w1_host && seg_rows > 0))
+        return fail(OXG4_INVALID_SHAPE, "SM-pair projection: 1..%d rows and K %% 8 == 0 required", kChunkRows);
+    TRY(allow_big_smem(pair_gemm_kernel<PG_STORE>));
+    TRY(allow_big_smem(pair_gemm_kernel<PG_GLU>));
+    cudaDeviceProp prop;
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaGetDeviceProperties(&prop, dev));
+    const size_t segs = seg_rows > 0 ? (N + seg_rows - 1) / seg_rows : 1, wb = (size_t)N * K * 2, xb = segs * M * K * 2;
+    const PairPlan plan = pair_plan(M, N, K, w1_host != nullptr, seg_rows, 2048, prop.multiProcessorCount);
+    const size_t ob = w1_host ? (size_t)M * N * 2 : (size_t)plan.S * M * N * 4;
+    char* d = nullptr;
+    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    CK(cudaMalloc(&d, 2 * up(wb) + up(xb) + up(ob) + 256));
+    char *w = d, *w1 = w + up(wb), *x = w1 + up(wb), *o = x + up(xb), *e = o + up(ob);
+    std::vector<uint8_t> host(ob);
+    int err = 0;
+    int32_t s = OXG4_OK;
+    if (cudaMemcpy(w, w_host, wb, cudaMemcpyHostToDevice) != cudaSuccess || cudaMemcpy(x, x_host, xb, cudaMemcpyHostToDevice) != cudaSuccess ||
+        (w1_host && cudaMemcpy(w1, w1_host, wb, cudaMemcpyHostToDevice) != cudaSuccess) || cudaMemset(o, 0xff, ob) != cudaSuccess ||
+        cudaMemset(e, 0, 4) != cudaSuccess)
+        s = fail(OXG4_CUDA, "Gemma 4 CUDA error: copy failed");
+    if (s == OXG4_OK)
+        s = pair_gemm_launch(plan, w, w1_host ? w1 : nullptr, x, M, N, K, seg_rows, (float*)o, (uint16_t*)o, N, (int)ACT_GELU_TANH, (int*)e, 0, false);
+    if (s == OXG4_OK && (cudaMemcpy(host.data(), o, ob, cudaMemcpyDeviceToHost) != cudaSuccess || cudaMemcpy(&err, e, 4, cudaMemcpyDeviceToHost) != cudaSuccess))
+        s = fail(OXG4_CUDA, "Gemma 4 CUDA error: SM-pair projection failed: %s", cudaGetErrorString(cudaGetLastError()));
+    cudaFree(d);
+    TRY(s);
+    if (err) return fail(OXG4_TIMEOUT, "SM-pair projection: a bounded barrier wait ran out (code %d)", err);
+    for (size_t i = 0; i < (size_t)M * N; ++i) {
+        float t = 0.0f;
+        if (w1_host) t = host_bf16_to_f32(((const uint16_t*)host.data())[i]);
+        else
+            for (int sp = 0; sp < plan.S; ++sp) t += ((const float*)host.data())[(size_t)sp * M * N + i];
+        out_host[i] = t;
+    }
+    if (slots_or_null) *slots_or_null = plan.S;
+    return OXG4_OK;
 }
 
 #include "layered.inl"
