@@ -481,6 +481,8 @@ struct QkvPostArgs {
     int pages_per_seq, page_tokens;
     const int32_t* cap;
     uint16_t* q_hl;              // [R][Nq][2][D] or null
+    uint16_t *kc, *vc;           // [Nkv][kv_rows][D] BF16: the keys and values go here and not to the pools (prompt_attn.cuh), or null
+    int kv_rows;
     int write_kv;                // 0: a KV-shared layer (its source layer has appended K/V; the projection holds q only)
 };
 
@@ -585,6 +587,13 @@ __global__ void __launch_bounds__(128) qkv_post_kernel(const QkvPostArgs a) {
         return;
     }
     const int kvh = (task - a.Nq) % a.Nkv;
+    if (a.kc != nullptr) {
+        uint32_t bits[EPT];
+#pragma unroll
+        for (int e = 0; e < EPT; ++e) bits[e] = f32_to_bf16_bits(o[e]);
+        st_u16_vec<EPT>((is_v ? a.vc : a.kc) + ((size_t)kvh * a.kv_rows + row) * D + lane * EPT, bits);
+        return;
+    }
     const int seq = a.row_seq ? a.row_seq[row] : row;
     const int slot = pos % a.cap[seq];
     const size_t off = (((size_t)a.page_table[(size_t)seq * a.pages_per_seq + slot / a.page_tokens] * a.Nkv + kvh) *

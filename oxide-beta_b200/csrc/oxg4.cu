@@ -30,6 +30,7 @@
 #include "layered_ops.cuh"
 #include "latent_mma.cuh"
 #include "head_mma.cuh"
+#include "prompt_attn.cuh"
 #include "tp.h"
 
 using namespace oxg4;
@@ -767,6 +768,9 @@ struct oxg4_cache {
     unsigned long long* ts_buf = nullptr;     // [kMaxTimeline][4] optional device timeline
     // rows a pass over the layers may carry: the batch for a decode step, up to chunk_rows prompt tokens for a chunk
     int rows_cap = 0, chunk_rows = 0;
+    bool prompt_attn = false;                 // chunks attend through prompt_attn_kernel
+    uint16_t *pa_k = nullptr, *pa_v = nullptr;   // keys and values of a chunk, [Nkv][chunk_rows][D]
+    float* pa_part = nullptr;                 // partials of kPaPartRows rows
     bool wide = false;                        // prompt chunks may use the SM-pair projections (csrc/pair_gemm.cuh)
     size_t part_rows = 0;                     // rows of partial outputs that qkv_part, o_part and down_part hold
     // prompt chunks: per-row metadata (token, position, sequence), the attention groups per layer kind (sliding, global) and
@@ -836,7 +840,12 @@ constexpr int kChunkRows = 2048;              // most prompt tokens one pass ove
 // 2.42, 4.49 and 1.51.
 constexpr int kWideRows = 96;
 
-// The metadata block of a prompt chunk: nine arrays of `cap` 32-bit entries.
+// Chunks of fewer rows than kPaMinRows do not fill the 128-row tiles of prompt_attn_kernel; they stay with the kernel that
+// deals the positions to all warps of the GPU.
+constexpr int kPaMinRows = 64;
+constexpr int kPaPartRows = 1024;             // rows times splits
+
+// The metadata block of a prompt chunk: arrays of `cap` 32-bit entries.
 struct ChunkMeta {
     int32_t* base;
     int cap;
@@ -848,7 +857,11 @@ struct ChunkMeta {
     int32_t* grp_n(int kind) const { return at(5 + kind); }
     int32_t* run_row0() const { return at(7); }
     int32_t* run_n() const { return at(8); }
-    static constexpr int kArrays = 9;
+    int32_t* row_end() const { return at(9); }                           // position behind the sequence's last token of the chunk
+    int32_t* tile_row0(int kind) const { return at(10 + kind); }         // row tiles of prompt_attn_kernel
+    int32_t* tile_n(int kind) const { return at(12 + kind); }
+    int32_t* tile_run0(int kind) const { return at(14 + kind); }
+    static constexpr int kArrays = 16;
 };
 
 static int32_t tc_gemm_setup();
@@ -948,6 +961,7 @@ static int32_t cache_build(oxg4_cache* c) {
     c->tc_ok = m->es == 2 && m->P == 0 && (m->layered || getenv("OXG4_DISABLE_TCGEN05") == nullptr);
     // a KV-shared layer attends after its source layer has appended a whole pass, so a pass may not outgrow the ring's spare rows
     c->wide = c->tc_ok && !m->layered && m->tp == 1 && m->cfg.num_kv_shared_layers == 0;
+    c->prompt_attn = c->wide && c->kv_dtype == OXG4_BF16 && getenv("OXG4_DISABLE_MMA_ATTN") == nullptr;
     int64_t all_tokens = 0;
     for (int b = 0; b < B; ++b) all_tokens += c->max_seq[b];
     c->chunk_rows = c->wide ? (int)std::max<int64_t>(kPrefillRows, std::min<int64_t>(kChunkRows, (all_tokens + 255) / 256 * 256)) : kPrefillRows;
@@ -1003,10 +1017,19 @@ static int32_t cache_build(oxg4_cache* c) {
         TRY(attn_mma_setup());
         int kvh_max = 1;
         for (auto& p : m->layers) kvh_max = std::max(kvh_max, p.Nkv);
-        TRY(dalloc(c, &c->q_hl, (size_t)A * 2 * m->qw_max));
+        TRY(dalloc(c, &c->q_hl, (size_t)(c->prompt_attn ? R : A) * 2 * m->qw_max));
         const int warps = m->num_sms * 4;                       // upper bound of the consumer warps of a launch
         TRY(dalloc(c, &c->am_part, ((size_t)std::min(A, kAmMaxGroups) * kvh_max + warps) * kAmRows * (m->Dmax + 2)));
         TRY(dalloc(c, &c->am_pre, (size_t)kAmMaxGroups + 1));
+    }
+    if (c->prompt_attn) {
+        if (!c->mma_attn) TRY(dalloc(c, &c->q_hl, (size_t)R * 2 * m->qw_max));
+        TRY(dalloc(c, &c->pa_k, (size_t)c->chunk_rows * m->kvw_max));
+        TRY(dalloc(c, &c->pa_v, (size_t)c->chunk_rows * m->kvw_max));
+        TRY(dalloc(c, &c->pa_part, (size_t)kPaPartRows * (m->qw_max + 2 * m->Nq)));
+        TRY(allow_big_smem(prompt_attn_kernel<64>));
+        TRY(allow_big_smem(prompt_attn_kernel<128>));
+        TRY(allow_big_smem(prompt_attn_kernel<256>));
     }
     c->use_tc = c->tc_ok && B >= (m->layered ? 2 : 8) && B <= kPrefillRows;       // up to 256 sequences: row blocks of 128 / 256 (UMMA N)
     c->ls_qkv.assign(L, 1);
@@ -1640,6 +1663,11 @@ struct RowSet {
         int row0, rows, grp0[2], grps[2];    // its groups per layer kind; their first rows count from row0
     };
     std::vector<Slice> slices;
+    // row tiles of prompt_attn_kernel per layer kind, and the rows' ends
+    const int32_t *tile_row0[2] = {nullptr, nullptr}, *tile_n[2] = {nullptr, nullptr}, *tile_run0[2] = {nullptr, nullptr};
+    int tiles[2] = {0, 0};
+    int longest[2] = {1, 1};             // most positions that the rows of a tile see together
+    const int32_t* row_end = nullptr;
     int max_visible = 1;                 // bound on the visible positions of any row (launch geometry only)
 };
 
@@ -1769,6 +1797,56 @@ static void launch_attention(Launcher& ln, oxg4_cache* c, const RowSet& rs, int 
     ln.cluster_x = 0;
 }
 
+// Attention of a prompt chunk on its own keys and values and those in the cache (csrc/prompt_attn.cuh); the rows that stay in
+// the cache are appended behind it.
+static void prompt_attention(Launcher& ln, oxg4_cache* c, const RowSet& rs, int l, const float* qkv, int qkv_splits, uint16_t* out) {
+    oxg4_model* m = c->m;
+    const LayerPlan& p = m->layers[l];
+    const int R = rs.R, kind = p.sliding ? 0 : 1, D = p.D;
+    const int32_t* page_table = p.sliding ? c->pt_slide : c->pt_full;
+    const int pps = p.sliding ? c->pps_slide : c->pps_full;
+    const int32_t* cap = p.sliding ? c->cap_slide : c->cap_full;
+    QkvPostArgs q{};
+    q.qkv = qkv; q.qkv_n = p.qkv_n; q.splits = qkv_splits; q.split_rows = R; q.R = R; q.Nq = m->Nq; q.Nkv = p.Nkv;
+    q.q_norm = p.q_norm; q.k_norm = p.k_norm; q.inv_freq = p.inv_freq; q.rotary_half = p.rotary_dim / 2;
+    q.eps = m->cfg.rms_norm_eps;
+    q.row_pos = rs.pos; q.row_seq = rs.seq; q.row_tok = rs.tok;
+    q.q_hl = c->q_hl;
+    q.write_kv = 1;
+    q.kc = c->pa_k; q.vc = c->pa_v; q.kv_rows = c->chunk_rows;
+    ln.go("qkv_post", D == 64 ? qkv_post_kernel<uint16_t, 64> : D == 128 ? qkv_post_kernel<uint16_t, 128> : qkv_post_kernel<uint16_t, 256>,
+          dim3((R * (m->Nq + 2 * p.Nkv) + 3) / 4), dim3(128), 0, q);
+    PromptAttnArgs a{};
+    a.q_hl = c->q_hl; a.kc = c->pa_k; a.vc = c->pa_v; a.kv_rows = c->chunk_rows;
+    a.Nq = m->Nq; a.Nkv = p.Nkv;
+    while ((1 << a.lg_group) < p.G) ++a.lg_group;
+    a.tile_row0 = rs.tile_row0[kind]; a.tile_n = rs.tile_n[kind]; a.tile_run0 = rs.tile_run0[kind];
+    a.row_pos = rs.pos; a.row_seq = rs.seq;
+    a.kpool = (const uint16_t*)c->kpool[l]; a.vpool = (const uint16_t*)c->vpool[l];
+    a.page_table = page_table; a.pages_per_seq = pps; a.page_tokens = c->PT; a.cap = cap;
+    a.window = p.sliding ? m->cfg.sliding_window : 0x7fffffff;
+    // few tiles (a portion of one prompt): their positions are split until the CTAs fill the GPU, at least two tiles each
+    const int units = rs.tiles[kind] * p.Nkv;
+    a.splits = std::max(1, std::min({m->num_sms / std::max(1, units), kPaPartRows / R, (rs.longest[kind] + 2 * kPaTile - 1) / (2 * kPaTile)}));
+    a.part = c->pa_part;
+    a.R = R;
+    a.out = out;
+    const dim3 grid((unsigned)(units * a.splits));
+    if (D == 64) ln.go("attn", prompt_attn_kernel<64>, grid, dim3(kPaThreads), prompt_attn_smem<64>(), a);
+    else if (D == 128) ln.go("attn", prompt_attn_kernel<128>, grid, dim3(kPaThreads), prompt_attn_smem<128>(), a);
+    else ln.go("attn", prompt_attn_kernel<256>, grid, dim3(kPaThreads), prompt_attn_smem<256>(), a);
+    if (a.splits > 1)
+        ln.go("attn_merge", D == 64 ? prompt_merge_kernel<64> : D == 128 ? prompt_merge_kernel<128> : prompt_merge_kernel<256>,
+              dim3((R * m->Nq + 3) / 4), dim3(128), 0, a);
+    KvAppendArgs k{};
+    k.kc = c->pa_k; k.vc = c->pa_v; k.kv_rows = c->chunk_rows; k.R = R; k.Nkv = p.Nkv;
+    k.row_pos = rs.pos; k.row_seq = rs.seq; k.row_end = rs.row_end;
+    k.kpool = (uint16_t*)c->kpool[l]; k.vpool = (uint16_t*)c->vpool[l];
+    k.page_table = page_table; k.pages_per_seq = pps; k.page_tokens = c->PT; k.cap = cap;
+    ln.go("kv_append", D == 64 ? kv_append_kernel<64> : D == 128 ? kv_append_kernel<128> : kv_append_kernel<256>,
+          dim3((R * p.Nkv + 3) / 4), dim3(128), 0, k);
+}
+
 // launch_attention for all rows of a pass: a prompt chunk goes slice by slice
 static void attend_rows(Launcher& ln, oxg4_cache* c, const RowSet& rs, int l, const float* qkv, int qkv_splits, uint16_t* out_bf16,
                         bool many_rows) {
@@ -1896,7 +1974,8 @@ static Pending run_layers(oxg4_cache* c, Launcher& ln, const RowSet& rs, bool us
             }
             if (wide) s_qkv = ln.pair("qkv", c, R, p.wqkv, nullptr, c->x_h, nqkv, H, c->qkv_part, nullptr, nqkv, 0);
             else ln.tc("qkv", c, R, p.wqkv, nullptr, c->x_h, nqkv, H, s_qkv, c->qkv_part, nqkv, 0);
-            attend_rows(ln, c, rs, l, c->qkv_part, s_qkv, c->x_a, true);
+            if (rs.tiles[0] + rs.tiles[1] > 0) prompt_attention(ln, c, rs, l, c->qkv_part, s_qkv, c->x_a);
+            else attend_rows(ln, c, rs, l, c->qkv_part, s_qkv, c->x_a, true);
             // row-split projection under tensor parallelism: without K-splits the kernel writes the rank's partial
             // sum straight into the buffer that is all-reduced (one launch less); with the peer-memory exchange
             // the summation kernel is what pushes it to the peers
@@ -2827,6 +2906,37 @@ static int32_t ingest(oxg4_model* m, oxg4_cache* c, const uint32_t* tokens, cons
             if (p == lens[b]) { ++b; p = 0; }
         }
         if (R == 0) break;
+        if (c->prompt_attn && R >= kPaMinRows) {
+            struct Tile { int row0, n, run0, seen; };
+            std::vector<Tile> tiles;
+            for (int k = 0; k < 2; ++k) {
+                const int per = kPaRows / kAmRows * tg[k], window = k == 0 ? m->cfg.sliding_window : 0x7fffffff;
+                tiles.clear();
+                for (size_t r = 0; r < rs.run_len.size(); ++r) {
+                    const int run0 = hm.run_row0()[r], n = rs.run_len[r], pos0 = hm.pos()[run0];
+                    for (int i = 0; i < n; i += per) {
+                        const int t = std::min(per, n - i), end = pos0 + i + t;
+                        tiles.push_back({run0 + i, t, run0, end - std::max(0, pos0 + i + 1 - window)});
+                    }
+                }
+                std::stable_sort(tiles.begin(), tiles.end(), [](const Tile& x, const Tile& y) { return x.seen > y.seen; });
+                for (size_t t = 0; t < tiles.size(); ++t) {
+                    hm.tile_row0(k)[t] = tiles[t].row0;
+                    hm.tile_n(k)[t] = tiles[t].n;
+                    hm.tile_run0(k)[t] = tiles[t].run0;
+                }
+                rs.tiles[k] = (int)tiles.size();
+                rs.longest[k] = tiles[0].seen;
+                rs.tile_row0[k] = dm.tile_row0(k);
+                rs.tile_n[k] = dm.tile_n(k);
+                rs.tile_run0[k] = dm.tile_run0(k);
+            }
+            for (size_t r = 0; r < rs.run_len.size(); ++r) {
+                const int run0 = hm.run_row0()[r], end = hm.pos()[run0] + rs.run_len[r];
+                for (int i = 0; i < rs.run_len[r]; ++i) hm.row_end()[run0 + i] = end;
+            }
+            rs.row_end = dm.row_end();
+        }
         cudaStream_t st = m->stream;
         CK(cudaMemcpyAsync(c->pf_meta, c->h_pf_meta, sizeof(int32_t) * ChunkMeta::kArrays * c->chunk_rows, cudaMemcpyHostToDevice, st));
         const bool prof = getenv("GEMMA4_PROFILE") != nullptr && getenv("OXG4_PROFILE_PREFILL") != nullptr;

@@ -410,7 +410,7 @@ class Gemma4CudaState:
         return out, s, ms.value
 
     PROFILE_KINDS = ["qkv", "shift", "decay", "recur", "recjoin", "outnorm", "latent", "uq", "latsplit", "uk", "latq", "latmerge", "uv",
-                     "latout", "qkv_post", "attn", "attn_merge", "o", "gateup", "down", "lmhead", "norm", "geglu", "sum",
+                     "latout", "qkv_post", "attn", "attn_merge", "kv_append", "o", "gateup", "down", "lmhead", "norm", "geglu", "sum",
                      "topk1", "topk2", "tp_pick", "allreduce", "allgather", "step_begin", "step_end"]
 
     def profile_step(self, tokens, table: Gemma4CudaCacheTable, totals: bool = False) -> dict:
