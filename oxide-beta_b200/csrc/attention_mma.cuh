@@ -366,13 +366,16 @@ inline size_t attn_mma_smem_bytes() {
 // One CTA per unit (group, kv head): adds the unit's partials in warp order and writes the normalised
 // output rows. The partial slots of a unit are (unit + w) for the consumer warps w whose tile range
 // meets the unit's.
+// A thread has one output value of a decode step (up to 512 threads) and loads eight partials at a time.
+constexpr int kAmMergeThreads = 512;
 template <int D, int G>
-__global__ void __launch_bounds__(128) attn_merge_kernel(const AttnMmaArgs a) {
+__global__ void __launch_bounds__(kAmMergeThreads) attn_merge_kernel(const AttnMmaArgs a) {
     constexpr int CH = 64;                                     // partials handled per round
     __shared__ float s_m[kAmRows][CH], s_e[kAmRows][CH], s_l[kAmRows][CH], s_L[kAmRows], s_M[kAmRows];
+    const int u = blockIdx.x, g = u / a.Nkv, kvh = u % a.Nkv;
+    const int nrows = a.grp_n[g] * G, row0 = a.grp_row0[g];    // there before the step
     pdl_wait();
     pdl_launch();
-    const int u = blockIdx.x, g = u / a.Nkv, kvh = u % a.Nkv;
     // tile prefix of the groups as the attention kernel computed it (one round of loads instead of a CTA-wide scan)
     const int pre_g = __ldcg(a.pre_out + g), pre_g1 = __ldcg(a.pre_out + g + 1), pre_all = __ldcg(a.pre_out + a.NG);
     const int nt = pre_g1 - pre_g;
@@ -380,7 +383,6 @@ __global__ void __launch_bounds__(128) attn_merge_kernel(const AttnMmaArgs a) {
     const int T = pre_all * a.Nkv, W = a.total_warps;
     const int ub = pre_g * a.Nkv + kvh * nt;
     const int w0 = am_warp_of(T, W, ub), w1 = am_warp_of(T, W, ub + nt - 1);
-    const int nrows = a.grp_n[g] * G, row0 = a.grp_row0[g];
     const int tid = threadIdx.x;
     const float* base = a.part + (size_t)(u + w0) * a.part_rows * (D + 2);
     const size_t slot = (size_t)a.part_rows * (D + 2);
@@ -410,7 +412,16 @@ __global__ void __launch_bounds__(128) attn_merge_kernel(const AttnMmaArgs a) {
         for (int idx = tid; idx < nrows * D; idx += blockDim.x) {
             const int r = idx / D, d = idx % D;
             float acc = 0.0f;
-            for (int w = 0; w < np; ++w) acc += s_e[r][w] * base[(size_t)w * slot + (size_t)r * (D + 2) + d];
+            const float* p = base + (size_t)r * (D + 2) + d;
+            for (int w = 0; w < np; w += 8) {
+                float v[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    if (w + q < np) v[q] = __ldcg(p + (size_t)(w + q) * slot);
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    if (w + q < np) acc += s_e[r][w + q] * v[q];
+            }
             const size_t oi = (size_t)(row0 + r / G) * a.Nq * D + (size_t)(kvh * G + r % G) * D + d;
             const float ov = acc / s_L[r];
             a.out[oi] = ov;
@@ -518,55 +529,88 @@ template <int EPT> DEVINL void st_u16_vec(uint16_t* p, const uint32_t (&bits)[EP
     else *reinterpret_cast<uint32_t*>(p) = w[0];
 }
 
-template <typename KT, int D>
+// FEW: no more rows than SMs, where latency is all that counts
+template <typename KT, int D, bool FEW>
 __global__ void __launch_bounds__(128) qkv_post_kernel(const QkvPostArgs a) {
-    constexpr int EPT = D / 32;
-    pdl_wait();
-    pdl_launch();
+    constexpr int EPT = D / 32, half = D / 2;
     const int lane = threadIdx.x & 31;
     const int first_task = a.q_hl ? 0 : a.Nq;
     const int last_task = a.write_kv ? a.Nq + 2 * a.Nkv : a.Nq;      // tasks: q heads, then k heads, then v heads
     const int per_row = last_task - first_task;
     const int job = blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (per_row <= 0 || job >= a.R * per_row) return;
-    const int row = job / per_row, task = first_task + job % per_row;
-    if (a.row_tok != nullptr && a.row_tok[row] == kInactiveToken) return;
-    const int pos = a.row_pos[row];
+    const int row = per_row > 0 ? job / per_row : 0, task = per_row > 0 ? first_task + job % per_row : 0;
+    const bool mine = per_row > 0 && job < a.R * per_row;
+    // Everything but the projection was there before the step (or before the chunk's row data were copied): norm weights, the
+    // position with its rotation (FEW) and the place in the cache are looked up ahead of the dependency wait.
+    const bool is_v = task >= a.Nq + a.Nkv;
+    const int kvh = task < a.Nq ? 0 : (task - a.Nq) % a.Nkv;
+    bool active = false;
+    float w[EPT], fr[EPT], cs[FEW ? EPT : 1], sn[FEW ? EPT : 1];
+    size_t off = 0;
+    int pos = 0;
+    auto look_up = [&]() {
+        ld_f32_vec<EPT>((task < a.Nq ? a.q_norm : a.k_norm) + lane * EPT, w);
+        ld_f32_vec<EPT>(a.inv_freq + (lane * EPT) % half, fr);               // a lane's elements lie in one half
+    };
+    if (mine) {
+        active = a.row_tok == nullptr || a.row_tok[row] != kInactiveToken;
+        pos = a.row_pos[row];
+        if (FEW && !is_v) {
+            look_up();
+#pragma unroll
+            for (int e = 0; e < EPT; ++e)
+                if ((lane * EPT + e) % half < a.rotary_half) sincosf((float)pos * fr[e], &sn[FEW ? e : 0], &cs[FEW ? e : 0]);
+        }
+        if (task >= a.Nq && a.kc == nullptr && active) {
+            const int seq = a.row_seq ? a.row_seq[row] : row;
+            const int slot = pos % a.cap[seq];
+            off = (((size_t)a.page_table[(size_t)seq * a.pages_per_seq + slot / a.page_tokens] * a.Nkv + kvh) * a.page_tokens +
+                   slot % a.page_tokens) * (size_t)D + lane * EPT;
+        }
+    }
+    pdl_wait();
+    pdl_launch();
+    if (!active) return;
     const int col = task * D;                                  // q heads, then k heads, then v heads
     float t[EPT];
 #pragma unroll
     for (int e = 0; e < EPT; ++e) t[e] = 0.0f;
-    for (int sp = 0; sp < a.splits; ++sp) {                    // K-split partials, in split order
-        float v[EPT];
-        ld_f32_vec<EPT>(a.qkv + ((size_t)sp * a.split_rows + row) * a.qkv_n + col + lane * EPT, v);
+    const float* src = a.qkv + (size_t)row * a.qkv_n + col + lane * EPT;
+    const size_t split_stride = (size_t)a.split_rows * a.qkv_n;
+    constexpr int NF = FEW ? 4 : 1;
+    for (int s0 = 0; s0 < a.splits; s0 += NF) {                // K-split partials, in split order, NF loads in flight
+        float v[NF][EPT];
 #pragma unroll
-        for (int e = 0; e < EPT; ++e) t[e] += v[e];
+        for (int q = 0; q < NF; ++q)
+            if (s0 + q < a.splits) ld_f32_vec<EPT>(src + (size_t)(s0 + q) * split_stride, v[q]);
+#pragma unroll
+        for (int q = 0; q < NF; ++q)
+            if (s0 + q < a.splits) {
+#pragma unroll
+                for (int e = 0; e < EPT; ++e) t[e] += v[q][e];
+            }
     }
     float ss = 0.0f;
 #pragma unroll
     for (int e = 0; e < EPT; ++e) ss += t[e] * t[e];
     ss = warp_sum(ss);
     const float r = 1.0f / sqrtf(ss / (float)D + a.eps);
-    const bool is_v = task >= a.Nq + a.Nkv;
     float o[EPT];
     if (!is_v) {
-        constexpr int half = D / 2;
-        float w[EPT], fr[EPT];
-        ld_f32_vec<EPT>((task < a.Nq ? a.q_norm : a.k_norm) + lane * EPT, w);
-        ld_f32_vec<EPT>(a.inv_freq + (lane * EPT) % half, fr);               // a lane's elements lie in one half
+        if constexpr (!FEW) look_up();
 #pragma unroll
         for (int e = 0; e < EPT; ++e) t[e] = t[e] * r * w[e];
 #pragma unroll
         for (int e = 0; e < EPT; ++e) {
             const int d = lane * EPT + e;
-            const int fi = d % half;
             const float partner = __shfl_xor_sync(0xffffffffu, t[e], 16);      // element d +- D/2 lives 16 lanes away
             float v = t[e];
-            if (fi < a.rotary_half) {
-                float sn, cs;
-                sincosf((float)pos * fr[e], &sn, &cs);
+            if (d % half < a.rotary_half) {
+                float s1, c1;
+                if constexpr (FEW) { s1 = sn[e]; c1 = cs[e]; }
+                else sincosf((float)pos * fr[e], &s1, &c1);
                 const float rotated = d < half ? -partner : partner;
-                v = v * cs + rotated * sn;
+                v = v * c1 + rotated * s1;
             }
             o[e] = v;
         }
@@ -586,7 +630,6 @@ __global__ void __launch_bounds__(128) qkv_post_kernel(const QkvPostArgs a) {
         st_u16_vec<EPT>(dst + D, lo);
         return;
     }
-    const int kvh = (task - a.Nq) % a.Nkv;
     if (a.kc != nullptr) {
         uint32_t bits[EPT];
 #pragma unroll
@@ -594,10 +637,6 @@ __global__ void __launch_bounds__(128) qkv_post_kernel(const QkvPostArgs a) {
         st_u16_vec<EPT>((is_v ? a.vc : a.kc) + ((size_t)kvh * a.kv_rows + row) * D + lane * EPT, bits);
         return;
     }
-    const int seq = a.row_seq ? a.row_seq[row] : row;
-    const int slot = pos % a.cap[seq];
-    const size_t off = (((size_t)a.page_table[(size_t)seq * a.pages_per_seq + slot / a.page_tokens] * a.Nkv + kvh) *
-                            a.page_tokens + slot % a.page_tokens) * (size_t)D + lane * EPT;
     KT* pool = (KT*)(is_v ? a.vpool : a.kpool);
     if constexpr (sizeof(KT) == 2) {
         uint32_t bits[EPT];

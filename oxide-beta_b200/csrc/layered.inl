@@ -705,8 +705,8 @@ struct LayeredPass {
             n.tokens = rs.tok;
             n.embed_scale = 1.0f;
         }
-        if (m->es == 2) ln.go("norm", rows_norm_kernel<uint16_t>, dim3(R), dim3(kRowsThreads), 0, n);
-        else ln.go("norm", rows_norm_kernel<float>, dim3(R), dim3(kRowsThreads), 0, n);
+        if (m->es == 2) launch_rows_norm<uint16_t>(ln, R, n);
+        else launch_rows_norm<float>(ln, R, n);
         advance();
     }
     // out = x . W^T for all rows; x holds the projection's operand type

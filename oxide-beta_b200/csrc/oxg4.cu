@@ -1640,6 +1640,12 @@ static int32_t attn_mma_setup() {
     return OXG4_OK;
 }
 
+template <typename XT>
+static void launch_rows_norm(Launcher& ln, int rows, const RowsNormArgs& n) {
+    if (rows <= ln.m->num_sms) ln.go("norm", rows_norm_kernel<XT, kFewRowsThreads>, dim3(rows), dim3(kFewRowsThreads), 0, n);
+    else ln.go("norm", rows_norm_kernel<XT, kRowsThreads>, dim3(rows), dim3(kRowsThreads), 0, n);
+}
+
 // The rows one pass over the layers carries: the sequences of a decode step, or up to kPrefillRows prompt
 // tokens (a chunk), each with its token id, absolute position and, for a chunk, the sequence it belongs to.
 struct RowSet {
@@ -1689,6 +1695,16 @@ struct TraceCtx {
     float* trace_dev;          // [L+1][B][H] receives every layer's input and the final hidden state
 };
 
+typedef void (*QkvPostFn)(const QkvPostArgs);
+template <typename KT, bool FEW>
+static QkvPostFn pick_qkv_post(int D) {
+    return D == 64 ? qkv_post_kernel<KT, 64, FEW> : D == 128 ? qkv_post_kernel<KT, 128, FEW> : qkv_post_kernel<KT, 256, FEW>;
+}
+static QkvPostFn pick_qkv_post(int kv_dtype, int D, bool few) {
+    if (kv_dtype == OXG4_BF16) return few ? pick_qkv_post<uint16_t, true>(D) : pick_qkv_post<uint16_t, false>(D);
+    return few ? pick_qkv_post<float, true>(D) : pick_qkv_post<float, false>(D);
+}
+
 // q/k norm + RoPE + v norm + KV append + attention of layer l for the rows of `rs` (decode.rs:99-157,
 // 176-325). qkv: [qkv_splits, split_rows, qkv_n] projection output; the result goes to `out` (+ BF16 copy).
 // split_rows: rows between two partials of qkv; out: [R, qw].
@@ -1718,10 +1734,7 @@ static void launch_attention(Launcher& ln, oxg4_cache* c, const RowSet& rs, int 
         q.q_hl = use_mma ? c->q_hl : nullptr;
         q.write_kv = p.shared ? 0 : 1;
         const int per_row = (use_mma ? m->Nq : 0) + (p.shared ? 0 : 2 * p.Nkv);
-        void (*fn)(const QkvPostArgs) = nullptr;
-        if (c->kv_dtype == OXG4_BF16) fn = D == 64 ? qkv_post_kernel<uint16_t, 64> : D == 128 ? qkv_post_kernel<uint16_t, 128> : qkv_post_kernel<uint16_t, 256>;
-        else fn = D == 64 ? qkv_post_kernel<float, 64> : D == 128 ? qkv_post_kernel<float, 128> : qkv_post_kernel<float, 256>;
-        ln.go("qkv_post", fn, dim3((R * per_row + 3) / 4), dim3(128), 0, q);
+        ln.go("qkv_post", pick_qkv_post(c->kv_dtype, D, R <= m->num_sms), dim3((R * per_row + 3) / 4), dim3(128), 0, q);
     }
     if (use_mma) {
         AttnMmaArgs a{};
@@ -1743,7 +1756,7 @@ static void launch_attention(Launcher& ln, oxg4_cache* c, const RowSet& rs, int 
         pick_attn_mma(D, p.G, &fn, &merge, &smem, &ncw);
         a.total_warps = m->num_sms * ncw;
         ln.go("attn", fn, dim3(m->num_sms), dim3((ncw + 1) * 32), smem, c->kmap[l], c->vmap[l], a);
-        ln.go("attn_merge", merge, dim3(rs.NG[kind] * p.Nkv), dim3(128), 0, a);
+        ln.go("attn_merge", merge, dim3(rs.NG[kind] * p.Nkv), dim3(std::min(kAmMergeThreads, a.part_rows * D)), 0, a);
         return;
     }
     AttnArgs a{};
@@ -1814,8 +1827,7 @@ static void prompt_attention(Launcher& ln, oxg4_cache* c, const RowSet& rs, int 
     q.q_hl = c->q_hl;
     q.write_kv = 1;
     q.kc = c->pa_k; q.vc = c->pa_v; q.kv_rows = c->chunk_rows;
-    ln.go("qkv_post", D == 64 ? qkv_post_kernel<uint16_t, 64> : D == 128 ? qkv_post_kernel<uint16_t, 128> : qkv_post_kernel<uint16_t, 256>,
-          dim3((R * (m->Nq + 2 * p.Nkv) + 3) / 4), dim3(128), 0, q);
+    ln.go("qkv_post", pick_qkv_post(OXG4_BF16, D, R <= m->num_sms), dim3((R * (m->Nq + 2 * p.Nkv) + 3) / 4), dim3(128), 0, q);
     PromptAttnArgs a{};
     a.q_hl = c->q_hl; a.kc = c->pa_k; a.vc = c->pa_v; a.kv_rows = c->chunk_rows;
     a.Nq = m->Nq; a.Nkv = p.Nkv;
@@ -1964,13 +1976,13 @@ static Pending run_layers(oxg4_cache* c, Launcher& ln, const RowSet& rs, bool us
                 n.w_post = m->layers[l - 1].post_ff_ln;
                 n.scalar = m->layers[l - 1].layer_scalar;
             }
-            ln.go("norm", rows_norm_kernel<uint16_t>, dim3(R), dim3(kRowsThreads), 0, n);
+            launch_rows_norm<uint16_t>(ln, R, n);
             copy_trace_tc();
             if (tr && tr->inject_dev) {
                 RowsNormArgs f = n;                      // layer-wise teacher forcing: forced input, nothing pending
                 f.embed = nullptr; f.raw = nullptr; f.w_post = nullptr; f.scalar = 1.0f;
                 f.h_in = tr->inject_dev + (size_t)l * R * H;
-                ln.go("norm", rows_norm_kernel<uint16_t>, dim3(R), dim3(kRowsThreads), 0, f);
+                launch_rows_norm<uint16_t>(ln, R, f);
             }
             if (wide) s_qkv = ln.pair("qkv", c, R, p.wqkv, nullptr, c->x_h, nqkv, H, c->qkv_part, nullptr, nqkv, 0);
             else ln.tc("qkv", c, R, p.wqkv, nullptr, c->x_h, nqkv, H, s_qkv, c->qkv_part, nqkv, 0);
@@ -2005,7 +2017,7 @@ static Pending run_layers(oxg4_cache* c, Launcher& ln, const RowSet& rs, bool us
             n2.w_norm = p.pre_ff_ln;
             n2.eps = m->cfg.rms_norm_eps;
             n2.x = c->x_h;
-            ln.go("norm", rows_norm_kernel<uint16_t>, dim3(R), dim3(kRowsThreads), 0, n2);
+            launch_rows_norm<uint16_t>(ln, R, n2);
             if (wide) {
                 ln.pair("gateup", c, R, p.wgate, p.wup, c->x_h, m->I, H, nullptr, c->x_i, m->I, (int)ACT_GELU_TANH);
                 s_down = ln.pair("down", c, R, p.wdown, nullptr, c->x_i, H, m->I, c->down_part, nullptr, H, 0);
@@ -2143,7 +2155,7 @@ static void closing_norm_tc(oxg4_cache* c, Launcher& ln, int rows, const Pending
     n.w_norm = m->final_norm;
     n.eps = m->cfg.rms_norm_eps;
     n.x = c->x_h;
-    ln.go("norm", rows_norm_kernel<uint16_t>, dim3(rows), dim3(kRowsThreads), 0, n);
+    launch_rows_norm<uint16_t>(ln, rows, n);
 }
 
 // Tied LM head over B rows + arg-max / top-k (decode.rs:495-508, kernel_module.rs:1988-2075).
