@@ -7,10 +7,7 @@
 //
 // A pass takes one of three forms:
 //   one row (a decode step of one sequence)  gemv.cuh with norms, token shift and output norms in the prologues
-//   BF16 weights, many rows                  tc_gemm.cuh, prompt passes of more than kWideRows rows pair_gemm.cuh, row kernels around
-//                                            them; only the recurrences go slice by slice (up to 256 rows). Prompts in ms, passes
-//                                            of 256 rows / of up to 2048: Pabovik, width 2560, 12 layers, 1 x 3001 tokens 48.5 / 20.4,
-//                                            32 ragged ones of up to 150 37.0 / 13.9; Nozurax, width 4096, 1 x 3000 36.2 / 25.7
+//   BF16 weights, many rows                  tc_gemm.cuh, row kernels around it
 //   f32 weights, many rows                   gemv.cuh in passes of up to four rows, the same row kernels
 //
 // Residual rows, weight rows and weight columns are zero-padded to multiples of 8, so that every size of a model is
@@ -406,11 +403,7 @@ static int layered_splits(const oxg4_model* m, const Proj& p, int R, bool chunk)
 
 static int32_t latent_mma_setup(const MixPlan& x);
 static int32_t head_attn_setup(const MixPlan& x);
-// most splits of the visible positions in a prompt chunk: longer chunks fill the GPU with their rows
-static int latent_chunk_splits(int R) { return R <= kPrefillRows ? 4 : R <= 2 * kPrefillRows ? 2 : 1; }
-// rows of partial outputs that the buffer of an SM-pair projection with n output columns holds: two sets of a chunk's rows,
-// one where its many columns fill the GPU by themselves
-static size_t layered_pair_rows(const oxg4_cache* c, int n) { return n > 16384 ? (size_t)c->chunk_rows : c->part_rows; }
+constexpr int kLatentChunkSplits = 4;     // most splits of the visible positions in a prompt chunk
 
 static int32_t layered_cache_build(oxg4_cache* c, int pages_full) {
     oxg4_model* m = c->m;
@@ -422,8 +415,7 @@ static int32_t layered_cache_build(oxg4_cache* c, int pages_full) {
     auto floats = [&](const Proj& p) {       // of a projection's output, K-split partials included
         const size_t n = (size_t)p.N * (p.w1 ? 2 : 1);
         if (!tc) return (size_t)R * n;
-        const size_t streamed = std::max((size_t)layered_splits(m, p, B, false) * B, (size_t)layered_splits(m, p, kPrefillRows, true) * kPrefillRows);
-        return n * std::max(streamed, c->wide && !p.w1 ? layered_pair_rows(c, p.N) : 0);
+        return n * std::max((size_t)layered_splits(m, p, B, false) * B, (size_t)layered_splits(m, p, kPrefillRows, true) * kPrefillRows);
     };
     size_t in_n = 1, o_n = 1, gu_n = 1, down_n = 1, q_n = 1, uk_n = 1, uv_n = 1, dec = 1, latq = 1, rh = 1, rh_rank = 1, xo = 1, xi = 1, xq = 1,
            xu = 1, xl = 1, rot = 1, act = 1, block_n = 1;
@@ -517,14 +509,14 @@ static int32_t layered_cache_build(oxg4_cache* c, int pages_full) {
     TRY(dalloc(c, &c->uv_buf, uv_n));
     TRY(bytes_alloc(&c->x_u, (size_t)R * xu * 2));
     TRY(bytes_alloc(&c->x_l, (size_t)R * xl * 2));
-    const size_t part_rows = std::max({(size_t)B * c->lat_splits, (size_t)4 * kPrefillRows, (size_t)2 * c->chunk_rows});
+    const size_t part_rows = std::max((size_t)B * c->lat_splits, (size_t)R * kLatentChunkSplits);
     TRY(dalloc(c, &c->lat_o, part_rows * rh_rank));
     TRY(dalloc(c, &c->lat_ml, part_rows * rh * 2));
     return OXG4_OK;
 }
 
 // ---- a pass over the layers -----------------------------------------------------------------------------------
-static_assert(kRecMaxBlocks * kRecBlock == kPrefillRows, "blocks of a slice");
+static_assert(kRecMaxBlocks * kRecBlock == kPrefillRows, "blocks of a pass");
 typedef void (*RecurFn)(const RecurArgs);
 // lanes along the key channels and channels per lane for heads of `dim`
 static void recur_shape(int dim, int* ks, int* kpt) {
@@ -642,7 +634,6 @@ struct LayeredPass {
     Launcher& ln;
     const RowSet& rs;
     const bool tc;                       // BF16 projections on the tensor cores
-    const bool wide;                     // projections on SM pairs
     const bool fused;                    // one row: prologues carry the row kernels' work
     const TraceCtx* tr;
     oxg4_model* m = c->m;
@@ -712,11 +703,6 @@ struct LayeredPass {
     // out = x . W^T for all rows; x holds the projection's operand type
     SplitIn project(const char* kind, const Proj& p, const void* x, float* out) {
         const int n = p.N * (p.w1 ? 2 : 1);
-        if (wide) {
-            const int S = ln.pair(kind, c, R, p.w, nullptr, (const uint16_t*)x, p.N, p.K, out, nullptr, n, 0, p.nseg > 1 ? p.seg_rows : 0,
-                                  layered_pair_rows(c, n));
-            return SplitIn{out, S, (size_t)R * n, n};
-        }
         if (tc) {
             const int S = layered_splits(m, p, R, rs.chunk);
             ln.tc(kind, c, R, p.w, p.w1, (const uint16_t*)x, p.N, p.K, S, out, n, 0, p.nseg > 1 ? p.seg_rows / kTcTileM : 0);
@@ -869,35 +855,24 @@ struct LayeredPass {
         else fn = ret ? pick_recur<REC_RETENTION, float>(ks, kpt, step) : pick_recur<REC_LIGHTNING, float>(ks, kpt, step);
         const int vs = kRecThreads / ks * kRecCols, dp = ks * kpt, tile = step ? 1 : rec_tile(dp);
         size_t smem = sizeof(float) * ((step ? 1 : 2) * ((size_t)tile * dp * (wkv ? 3 : 2) + tile * vs + pad_to(tile, 4)) + (wkv ? dp + x.low_rank : 0));
-        const bool blocks = !step && !wkv; // blocks of the runs, joined where a run has several
-        if (blocks) {
+        int parts = (int)rs.run_len.size();
+        bool join = false;
+        if (!step && !wkv) {               // blocks of the runs, joined where a run has several
             smem = fixed_recur_smem(ks, kpt);
+            parts = 0;
+            for (int n : rs.run_len) {
+                parts += (n + kRecBlock - 1) / kRecBlock;
+                join |= n > kRecBlock;
+            }
+            a.runs = (int)rs.run_len.size();
             a.block_state = c->block_state;
             a.block_q = c->lat_q;
         }
         if (ln.status == OXG4_OK && smem > 48 * 1024) ln.status = allow_big_smem(fn);
-        // a chunk's slices follow each other: a run that goes on in the next slice starts there from the state in memory
-        const size_t n_slices = step ? 1 : rs.slices.size();
-        for (size_t i = 0; i < n_slices; ++i) {
-            const int run0 = step ? 0 : rs.slices[i].run0, n_runs = step ? (int)rs.run_len.size() : rs.slices[i].runs;
-            int parts = n_runs;
-            bool join = false;
-            a.rows.row0 = rs.run_row0 + run0;
-            a.rows.n = rs.run_n + run0;
-            if (blocks) {
-                parts = 0;
-                for (int r = run0; r < run0 + n_runs; ++r) {
-                    parts += (rs.run_len[r] + kRecBlock - 1) / kRecBlock;
-                    join |= rs.run_len[r] > kRecBlock;
-                }
-                a.runs = n_runs;
-                a.slice_row0 = rs.slices[i].row0;
-            }
-            ln.go("recur", fn, dim3(x.heads, (x.vdim + vs - 1) / vs, (unsigned)parts), dim3(kRecThreads), smem, a);
-            if (join) {
-                if (ln.status == OXG4_OK && join_smem(x.dim) > 48 * 1024) ln.status = allow_big_smem(recur_join_kernel);
-                ln.go("recjoin", recur_join_kernel, dim3(x.heads, (x.vdim + kJoinCols - 1) / kJoinCols, (unsigned)parts), dim3(kJoinThreads), join_smem(x.dim), a);
-            }
+        ln.go("recur", fn, dim3(x.heads, (x.vdim + vs - 1) / vs, (unsigned)parts), dim3(kRecThreads), smem, a);
+        if (join) {
+            if (ln.status == OXG4_OK && join_smem(x.dim) > 48 * 1024) ln.status = allow_big_smem(recur_join_kernel);
+            ln.go("recjoin", recur_join_kernel, dim3(x.heads, (x.vdim + kJoinCols - 1) / kJoinCols, (unsigned)parts), dim3(kJoinThreads), join_smem(x.dim), a);
         }
         if (ret) output(x, one(c->attn_out, x.owp), x.vdim, x.vdim, nullptr, in, ACT_SILU);
         else output(x, one(c->attn_out, x.owp), x.vdim, wkv ? x.dim : x.ow, x.out_norm, in, wkv ? ACT_SILU : ACT_SIGMOID);
@@ -944,7 +919,7 @@ struct LayeredPass {
         int mma_tiles = 0;
         if (mma) {
             for (int n : rs.run_len) mma_tiles += (n * x.heads + tile_rows - 1) / tile_rows;
-            const int most = rs.chunk ? latent_chunk_splits(R) : c->lat_splits, visible_tiles = (rs.max_visible + kLmTile - 1) / kLmTile;
+            const int most = rs.chunk ? kLatentChunkSplits : c->lat_splits, visible_tiles = (rs.max_visible + kLmTile - 1) / kLmTile;
             part.splits = groups * latent_splits(mma_tiles, (visible_tiles + groups - 1) / groups, std::max(1, most / groups), m->num_sms);
             ma.heads = x.heads; ma.rank = x.rank; ma.rot = x.rot;
             ma.scale = x.scale;
@@ -957,8 +932,7 @@ struct LayeredPass {
         if (mma && tc) {
             // many rows: per-head products with W_uk^T and W_uv on the tensor cores
             ln.go("latsplit", latent_split_query_kernel, dim3(R), dim3(256), 0, a, R, q, (uint16_t*)c->x_u, x.uk.K, c->lat_rot);
-            if (wide) ln.pair("uk", c, R, x.uk.w, nullptr, (const uint16_t*)c->x_u, x.uk.N, x.uk.K, c->uk_buf, nullptr, x.uk.N, 0, x.uk.seg_rows, R);
-            else ln.tc("uk", c, R, x.uk.w, nullptr, (const uint16_t*)c->x_u, x.uk.N, x.uk.K, 1, c->uk_buf, x.uk.N, 0, x.uk.seg_rows / kTcTileM);
+            ln.tc("uk", c, R, x.uk.w, nullptr, (const uint16_t*)c->x_u, x.uk.N, x.uk.K, 1, c->uk_buf, x.uk.N, 0, x.uk.seg_rows / kTcTileM);
             ma.q_abs = c->uk_buf; ma.abs_row = x.uk.N; ma.abs_head = x.uk.seg_rows;
             ma.q_rot = c->lat_rot; ma.rot_row = (size_t)x.heads * x.rot; ma.rot_head = x.rot;
             ln.go("attn", mma, dim3(mma_tiles, part.splits / groups), dim3(kLmThreads * groups), mma_smem, ma);
@@ -1011,7 +985,7 @@ struct LayeredPass {
                   (uint16_t*)c->x_u, x.kd);
             int units = 0;
             for (int n : rs.run_len) units += (n * group + tile_rows - 1) / tile_rows;
-            const int most = rs.chunk ? latent_chunk_splits(R) : c->lat_splits;
+            const int most = rs.chunk ? kLatentChunkSplits : c->lat_splits;
             part.splits = latent_splits(units * x.kv_heads, (rs.max_visible + kHmTile - 1) / kHmTile, most, 2 * m->num_sms);
             HeadMmaArgs h{};
             h.q = (const uint16_t*)c->x_u;
@@ -1066,12 +1040,6 @@ struct LayeredPass {
             return;
         }
         close_rows(x.norm2, c->mix_x, nullptr);
-        if (wide) {
-            ln.pair("gateup", c, R, x.gateup.w, x.gateup.w1, (const uint16_t*)c->mix_x, x.gateup.N, x.gateup.K, nullptr, (uint16_t*)c->mix_y,
-                    x.ffp, m->ff_act);
-            pend(project("down", x.down, c->mix_y, c->down_part), x.norm2b);
-            return;
-        }
         const SplitIn gu = project("gateup", x.gateup, c->mix_x, c->gu_part);
         ln.go("geglu", geglu_rows_kernel, dim3((x.ffp / 4 + kRowsThreads - 1) / kRowsThreads, R), dim3(kRowsThreads), 0, R, x.ffp,
               (const float*)c->gu_part, gu.splits, (uint16_t*)c->mix_y, m->ff_act);
@@ -1083,7 +1051,7 @@ struct LayeredPass {
 
 static Pending run_layered(oxg4_cache* c, Launcher& ln, const RowSet& rs, bool use_tc, const TraceCtx* tr) {
     oxg4_model* m = c->m;
-    LayeredPass p{c, ln, rs, use_tc, use_tc && rs.chunk && c->wide && rs.R > kWideRows, !use_tc && rs.R == 1 && !rs.chunk, tr};
+    LayeredPass p{c, ln, rs, use_tc, !use_tc && rs.R == 1 && !rs.chunk, tr};
     for (int l = 0; l < m->cfg.num_hidden_layers && ln.status == OXG4_OK; ++l) {
         const MixPlan& x = m->layers[l].mix;
         const SplitIn in = p.input(x, l);

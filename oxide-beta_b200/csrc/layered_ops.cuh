@@ -157,13 +157,13 @@ wkv_decay_kernel(int R, int N, int rank, SplitIn low, int col, const WT* w2, con
 // Prompts with fixed decays (LIGHTNING, RETENTION) go through fixed_recur_kernel: a run is cut into blocks of kRecBlock tokens
 // that are walked side by side, every block but the first from a zero state, and recur_join_kernel adds what the state at a
 // block's start contributes: o_t += decay^(t + 1) S_start^T q_t for the block's t-th token, S_start = sum of the earlier
-// blocks' end states times the decay in between. End states lie in slots of their own, 2 * (row of the slice / kRecBlock), plus one
+// blocks' end states times the decay in between. End states lie in slots of their own, 2 * (first row / kRecBlock), plus one
 // for a block that is not full: full blocks begin kRecBlock rows apart, and a last, shorter block follows a full one.
 enum { REC_LIGHTNING = 0, REC_WKV = 1, REC_RETENTION = 2 };
 constexpr int kRecThreads = 128;
 constexpr int kRecCols = 2;              // value columns per thread
 constexpr int kRecBlock = 64;            // tokens of a block
-constexpr int kRecMaxBlocks = 4;         // blocks of the longest run (a slice of a pass has at most 256 rows)
+constexpr int kRecMaxBlocks = 4;         // blocks of the longest run (a pass carries at most 256 rows)
 __host__ __device__ constexpr int rec_tile(int dp) { return dp <= 128 ? 16 : dp <= 256 ? 8 : 4; }   // tokens staged at a time
 
 struct RecurArgs {
@@ -183,7 +183,6 @@ struct RecurArgs {
     float* block_state;                  // fixed_recur_kernel: [slots][heads][vdim][dim]
     float* block_q;                      //   [R, heads * dim] activated queries for recur_join_kernel
     int runs;
-    int slice_row0;                      // first row of the launch's slice
     RunRows rows;
     float* out;                          // [R, ld_out]
     int ld_out;
@@ -245,7 +244,7 @@ DEVINL bool find_block(const RecurArgs& a, int t, RecBlock& b) {
     b.n = min(kRecBlock, a.rows.n[s_run] - b.first);
     b.split = a.rows.n[s_run] > kRecBlock;
     b.last = b.first + b.n == a.rows.n[s_run];
-    b.slot = 2 * (size_t)((b.row0 - a.slice_row0) / kRecBlock) + (b.n < kRecBlock ? 1 : 0);
+    b.slot = 2 * (size_t)(b.row0 / kRecBlock) + (b.n < kRecBlock ? 1 : 0);
     return true;
 }
 
@@ -712,7 +711,7 @@ __global__ void __launch_bounds__(kJoinThreads) recur_join_kernel(const RecurArg
     __syncthreads();
     // the earlier blocks of the run are full and lie one behind the other
     const size_t all = (size_t)a.heads * a.vdim * dim, here = ((size_t)hd * a.vdim + v0) * dim;
-    const float* e0 = a.block_state + 2 * (size_t)((b.row0 - b.first - a.slice_row0) / kRecBlock) * all + here;
+    const float* e0 = a.block_state + 2 * (size_t)((b.row0 - b.first) / kRecBlock) * all + here;
     const float* mine = a.block_state + b.slot * all + here;
     float* st = a.state + seq * all + here;
     const int earlier = b.first / kRecBlock;

@@ -960,8 +960,8 @@ static int32_t cache_build(oxg4_cache* c) {
     // are tiny and have no tcgen05 variant)
     c->tc_ok = m->es == 2 && m->P == 0 && (m->layered || getenv("OXG4_DISABLE_TCGEN05") == nullptr);
     // a KV-shared layer attends after its source layer has appended a whole pass, so a pass may not outgrow the ring's spare rows
-    c->wide = c->tc_ok && m->tp == 1 && m->cfg.num_kv_shared_layers == 0;
-    c->prompt_attn = c->wide && !m->layered && c->kv_dtype == OXG4_BF16 && getenv("OXG4_DISABLE_MMA_ATTN") == nullptr;
+    c->wide = c->tc_ok && !m->layered && m->tp == 1 && m->cfg.num_kv_shared_layers == 0;
+    c->prompt_attn = c->wide && c->kv_dtype == OXG4_BF16 && getenv("OXG4_DISABLE_MMA_ATTN") == nullptr;
     int64_t all_tokens = 0;
     for (int b = 0; b < B; ++b) all_tokens += c->max_seq[b];
     c->chunk_rows = c->wide ? (int)std::max<int64_t>(kPrefillRows, std::min<int64_t>(kChunkRows, (all_tokens + 255) / 256 * 256)) : kPrefillRows;
@@ -1047,12 +1047,9 @@ static int32_t cache_build(oxg4_cache* c) {
         TRY(dalloc(c, &c->ple_raw, (size_t)R * H));
     }
     if (m->layered) TRY(layered_cache_build(c, pages_full));
-    if (c->tc_ok) TRY(tc_gemm_setup());
-    if (c->wide) {
-        TRY(allow_big_smem(pair_gemm_kernel<PG_STORE>));
-        TRY(allow_big_smem(pair_gemm_kernel<PG_GLU>));
-    }
+    if (c->tc_ok && m->layered) TRY(tc_gemm_setup());
     if (c->tc_ok && !m->layered) {
+        TRY(tc_gemm_setup());
         const int sms = m->num_sms;
         auto tiles = [](int n) { return (n + kTcTileM - 1) / kTcTileM; };
         auto kbs = [](int k) { return (k + kTcTileK - 1) / kTcTileK; };
@@ -1062,6 +1059,10 @@ static int32_t cache_build(oxg4_cache* c) {
         const int chunk_tc = c->wide ? kWideRows : kPrefillRows;
         auto rows_splits = [&](int sd, int sp) { return (size_t)std::max(sd * B, sp * chunk_tc); };
         auto part_rows = [&](int sd, int sp) { return std::max(rows_splits(sd, sp), c->wide ? c->part_rows : 0); };
+        if (c->wide) {
+            TRY(allow_big_smem(pair_gemm_kernel<PG_STORE>));
+            TRY(allow_big_smem(pair_gemm_kernel<PG_GLU>));
+        }
         for (int l = 0; l < L; ++l) {
             const LayerPlan& p = m->layers[l];
             c->ls_qkv[l] = tc_pick_splits(tiles(p.qkv_n), kbs(H), sms, Bd, p.qkv_n, H);
@@ -1463,11 +1464,11 @@ struct Launcher {
     }
 
     // projection of many rows on SM pairs: returns the number of partial outputs in `out`; with w1 the gated activation goes
-    // to out_bf16 instead. max_rows: rows of partial outputs that `out` holds (0: part_rows of the cache table)
+    // to out_bf16 instead
     int pair(const char* kind, oxg4_cache* c, int rows, const void* w, const void* w1, const uint16_t* x, int N, int K, float* out,
-             uint16_t* out_bf16, int ld, int act, int seg_rows = 0, size_t max_rows = 0) {
+             uint16_t* out_bf16, int ld, int act, int seg_rows = 0) {
         if (status != OXG4_OK) return 1;
-        const PairPlan plan = pair_plan(rows, N, K, w1 != nullptr, seg_rows, max_rows ? max_rows : c->part_rows, m->num_sms);
+        const PairPlan plan = pair_plan(rows, N, K, w1 != nullptr, seg_rows, c->part_rows, m->num_sms);
         cudaEvent_t e0, e1;
         prof_begin(e0, e1);
         status = pair_gemm_launch(plan, w, w1, x, rows, N, K, seg_rows, out, out_bf16, ld, act, c->tc_err, m->stream, m->use_pdl && !m->profiling);
@@ -1666,7 +1667,6 @@ struct RowSet {
     // a chunk's rows in slices of at most kPrefillRows: a slice appends its K/V and attends before the next one appends
     struct Slice {
         int row0, rows, grp0[2], grps[2];    // its groups per layer kind; their first rows count from row0
-        int run0, runs;                      // layered models: its runs
     };
     std::vector<Slice> slices;
     // row tiles of prompt_attn_kernel per layer kind, and the rows' ends
@@ -2886,7 +2886,7 @@ static int32_t ingest(oxg4_model* m, oxg4_cache* c, const uint32_t* tokens, cons
         RowSet rs;
         while (b < B && R < c->chunk_rows) {
             if (lens[b] == 0) { ++b; continue; }
-            if (R % kPrefillRows == 0) rs.slices.push_back({R, 0, {NG[0], NG[1]}, {0, 0}, (int)rs.run_len.size(), 0});
+            if (R % kPrefillRows == 0) rs.slices.push_back({R, 0, {NG[0], NG[1]}, {0, 0}});
             RowSet::Slice& sl = rs.slices.back();
             const int take = std::min(kPrefillRows - sl.rows, lens[b] - p);
             for (int i = 0; i < take; ++i) {
@@ -2902,14 +2902,13 @@ static int32_t ingest(oxg4_model* m, oxg4_cache* c, const uint32_t* tokens, cons
                     ++NG[k];
                     ++sl.grps[k];
                 }
-            if (run_seq == b && (!m->layered || sl.rows > 0)) {     // the same run goes on in the next slice
+            if (run_seq == b) {                                // the same run goes on in the next slice
                 hm.run_n()[rs.run_len.size() - 1] += take;
                 rs.run_len.back() += take;
             } else {
                 hm.run_row0()[rs.run_len.size()] = R;
                 hm.run_n()[rs.run_len.size()] = take;
                 rs.run_len.push_back(take);
-                ++sl.runs;
                 run_seq = b;
             }
             sl.rows += take;
