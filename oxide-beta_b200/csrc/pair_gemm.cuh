@@ -270,6 +270,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 const bool vec = (a.ld & 7) == 0;
                 for (int c0 = part * 32; c0 < a.bn; c0 += 64) {
                     uint32_t v[2][16];
+                    __syncwarp();                              // rows past M skip the stores: all lanes meet before the aligned loads
                     tmem_ld16(v[0], taddr + (uint32_t)c0);
                     tmem_ld16(v[1], taddr + (uint32_t)c0 + 16);
                     tmem_ld_wait();
@@ -300,6 +301,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 const bool vec = (a.ld & 15) == 0;
                 for (int c0 = part * 16; c0 < cols; c0 += 32) {
                     uint32_t g[16], up[16], o[8];
+                    __syncwarp();
                     tmem_ld16(g, taddr + (uint32_t)c0);
                     tmem_ld16(up, taddr + (uint32_t)(cols + c0));
                     tmem_ld_wait();
