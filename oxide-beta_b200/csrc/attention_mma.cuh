@@ -228,7 +228,8 @@ attn_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
         const uint32_t q_off = (uint32_t)((((lm_i & 1) * 8 + lm_r) * QS + (lm_i >> 1) * 8) * 2);
         int t = begin, it = 0;
         const int end = begin + len;
-        while (t < end && !failed) {
+        bool lost = false;                                      // the same in all lanes of the warp: ldmatrix and mma are .aligned
+        while (t < end && !lost) {
             int g, kvh, lt, nt;
             am_locate(pre, a.NG, a.Nkv, t, g, kvh, lt, nt);
             const int seg_end = min(end, t + (nt - lt));
@@ -263,9 +264,9 @@ attn_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
 
             for (; t < seg_end; ++t, ++lt, ++it) {
                 const int s = it % NST;
-                if (!mbar_wait(&full[warp][s], (it / NST) & 1)) {
-                    failed = 1;
-                    if (lane == 0) atomicExch(a.err, 12);
+                if (!mbar_wait_warp(&full[warp][s], (it / NST) & 1)) {
+                    lost = true;
+                    if (lane == 0) { failed = 1; atomicExch(a.err, 12); }
                     break;
                 }
                 const uint32_t kb = smem_u32(stages + ((size_t)warp * NST + s) * STAGE);
@@ -337,7 +338,8 @@ attn_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&empty[warp][s]);       // the stage may be refilled
             }
-            if (failed) break;
+            lost |= __any_sync(0xffffffffu, failed) != 0;
+            if (lost) break;
             // ---- this warp's partial of the unit: slot (unit + warp), rows < nrows ----
             l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
             l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
@@ -350,7 +352,7 @@ attn_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
             }
         }
         // after a failed wait: let this warp's copies in flight land (bounded) before the CTA's memory goes away
-        if (failed) {
+        if (lost) {
             __syncwarp();
             if (lane == 0)
                 for (int w_it = it; w_it < issued[warp]; ++w_it) mbar_wait(&full[warp][w_it % NST], (w_it / NST) & 1);

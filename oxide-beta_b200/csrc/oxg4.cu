@@ -3268,13 +3268,14 @@ extern "C" int32_t oxg4_debug_wait_timeout(oxg4_model* m, oxg4_cache* c, int32_t
     if (spin_limit == 0 || spin_limit > 1000000u) return fail(OXG4_INVALID_ARGUMENT, "spin_limit must be 1..1000000");
     TRY(bind_device(m));
     // the flag that is waited on is the (zero) attention ticket array: nothing writes it during the probe
-    wait_probe_kernel<<<1, 32, 0, m->stream>>>(kind, spin_limit, c->attn_ticket, c->tc_err);
+    wait_probe_kernel<<<1, 64, 0, m->stream>>>(kind, spin_limit, c->attn_ticket, c->tc_err);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(m->stream));
     int err = 0;
     CK(cudaMemcpy(&err, c->tc_err, sizeof err, cudaMemcpyDeviceToHost));
     if (err) {
         CK(cudaMemset(c->tc_err, 0, sizeof err));
+        if (err == 23) return fail(OXG4_CUDA, "mbarrier wait: the lanes of a warp got different answers");
         return fail(OXG4_TIMEOUT, "%s: a bounded wait ran out (code %d)", err == 21 ? "mbarrier wait" : "peer flag wait", err);
     }
     return OXG4_OK;

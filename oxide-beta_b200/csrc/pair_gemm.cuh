@@ -162,11 +162,13 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
+        __syncwarp();                                          // lane 0 comes from the barriers
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)), "r"(512));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    __syncwarp();
     cluster_sync_all();                                        // both CTAs' barriers exist before anyone signals them
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_base;
@@ -259,7 +261,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         PairWalk w = start;
         for (; w.next(); ++tile_i) {
             const uint32_t ab = tile_i & 1, use = tile_i >> 1;
-            if (!mbar_wait(&acc_full[ab], use & 1)) { if (lane == 0) { failed = 1; atomicExch(a.err, 4); } break; }
+            if (!mbar_wait_warp(&acc_full[ab], use & 1)) { if (lane == 0) { failed = 1; atomicExch(a.err, 4); } break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int n0 = w.tile / tiles_m * cols;
             const int row = w.tile % tiles_m * kPgTileM + (int)rank * 128 + quad * 32 + lane;
@@ -330,6 +332,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     // ---- teardown: always reached, also after a failed wait ----
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    __syncwarp();
     cluster_sync_all();
     if (warp == 0) {
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));

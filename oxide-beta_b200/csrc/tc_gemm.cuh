@@ -73,6 +73,11 @@ DEVINL bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t limit = kTcSpinLi
     }
     return false;
 }
+// The same for a whole warp, which goes on together with one answer: false when the budget of any lane ran out. A lane that went its
+// own way would leave the others at an .aligned instruction or a full-mask barrier that never sees it.
+DEVINL bool mbar_wait_warp(uint64_t* bar, uint32_t parity, uint32_t limit = kTcSpinLimit) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit));
+}
 
 DEVINL void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile(
@@ -135,6 +140,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
+        __syncwarp();                                          // lane 0 comes from the barriers
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)), "r"(TM_COLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
@@ -248,7 +254,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         uint32_t tile_i = 0;
         for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, ++tile_i) {
             const uint32_t ab = tile_i & 1, use = tile_i >> 1;
-            if (!mbar_wait(&acc_full[ab], use & 1)) { if (lane == 0) atomicExch(a.err, 4); break; }
+            if (!mbar_wait_warp(&acc_full[ab], use & 1)) { if (lane == 0) { failed = 1; atomicExch(a.err, 4); } break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int tg = t / (a.S * a.TB), sp = (t / a.TB) % a.S, b0 = (t % a.TB) * BN;
             const bool second = tg >= tiles_per_mat;
@@ -258,6 +264,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             for (int c0 = 0; c0 < BN; c0 += 16) {
                 uint32_t v[16];
                 const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) + ab * ACC_COLS + (uint32_t)c0;
+                __syncwarp();                                  // rows past N skip the stores: all lanes meet before the aligned load
                 asm volatile(
                     "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
@@ -279,6 +286,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) {
+        __syncwarp();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TM_COLS));
     }
 }
