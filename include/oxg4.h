@@ -372,11 +372,10 @@ int32_t oxg4_debug_tc_gemm(const uint16_t* w_host, const uint16_t* x_host, int32
                            float* out_host, float* ms);
 
 /* The same for the SM-pair projection of prompt passes (csrc/pair_gemm.cuh): out[M, N] = x[M, K] . W[N, K]^T, or with w1 the
- * BF16 value of gelu(x . W^T) * (x . W1^T) widened to f32. seg_rows > 0 (a multiple of 128, without w1): rows of W from
- * s * seg_rows on multiply rows s * M .. of x. 1 <= M <= 2048, K a multiple of 8. slots (may be NULL) receives the number of
+ * BF16 value of gelu(x . W^T) * (x . W1^T) widened to f32. 1 <= M <= 2048, K a multiple of 8. slots (may be NULL) receives the number of
  * partial outputs. */
 int32_t oxg4_debug_pair_gemm(const uint16_t* w_host, const uint16_t* w1_host, const uint16_t* x_host, int32_t N, int32_t K,
-                             int32_t M, int32_t seg_rows, float* out_host, int32_t* slots);
+                             int32_t M, float* out_host, int32_t* slots);
 
 /* Diagnostics (no counterpart in the reference): when the environment variable OXG4_TIMELINE is
  * set before oxg4_model_create, every kernel of a step stamps the GPU's nanosecond timer at entry,

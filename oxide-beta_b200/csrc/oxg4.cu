@@ -1354,18 +1354,16 @@ static int32_t tc_gemm_launch(const void* w_dev, const void* w1_dev, const void*
 
 // Projection of many rows on SM pairs by `plan` (csrc/pair_gemm.cuh): partials out[plan.S, M, ld], or with w1 (gate and up)
 // out_bf16[M, ld] = bf16(act(gate) * up)
-static int32_t pair_gemm_launch(const PairPlan& plan, const void* w, const void* w1, const void* x, int M, int N, int K, int seg_rows,
-                                float* out, uint16_t* out_bf16, int ld, int act, int* err, cudaStream_t st, bool pdl) {
+static int32_t pair_gemm_launch(const PairPlan& plan, const void* w, const void* w1, const void* x, int M, int N, int K, float* out,
+                                uint16_t* out_bf16, int ld, int act, int* err, cudaStream_t st, bool pdl) {
     if (M < 1 || K % 8 != 0) return fail(OXG4_INVALID_SHAPE, "tcgen05 projection: at least one row and K %% 8 == 0 required");
-    const int n_segs = seg_rows > 0 ? (N + seg_rows - 1) / seg_rows : 1;
     CUtensorMap mx, mw, mw1;
-    TRY(encode_bf16_2d(&mx, x, (uint64_t)M * n_segs, (uint64_t)K, 128));
+    TRY(encode_bf16_2d(&mx, x, (uint64_t)M, (uint64_t)K, 128));
     TRY(encode_bf16_2d(&mw, w, (uint64_t)N, (uint64_t)K, (uint32_t)plan.bn / 2));
     TRY(encode_bf16_2d(&mw1, w1 ? w1 : w, (uint64_t)N, (uint64_t)K, (uint32_t)plan.bn / 2));
     PairGemmArgs a{};
     a.M = M; a.N = N; a.K = K;
     a.bn = plan.bn; a.cut = plan.cut; a.S = plan.S;
-    a.seg_rows = seg_rows;
     a.out = out; a.out_bf16 = out_bf16; a.ld = ld; a.act = act;
     a.err = err;
     cudaLaunchConfig_t cfg = {};
@@ -1466,12 +1464,12 @@ struct Launcher {
     // projection of many rows on SM pairs: returns the number of partial outputs in `out`; with w1 the gated activation goes
     // to out_bf16 instead
     int pair(const char* kind, oxg4_cache* c, int rows, const void* w, const void* w1, const uint16_t* x, int N, int K, float* out,
-             uint16_t* out_bf16, int ld, int act, int seg_rows = 0) {
+             uint16_t* out_bf16, int ld, int act) {
         if (status != OXG4_OK) return 1;
-        const PairPlan plan = pair_plan(rows, N, K, w1 != nullptr, seg_rows, c->part_rows, m->num_sms);
+        const PairPlan plan = pair_plan(rows, N, K, w1 != nullptr, c->part_rows, m->num_sms);
         cudaEvent_t e0, e1;
         prof_begin(e0, e1);
-        status = pair_gemm_launch(plan, w, w1, x, rows, N, K, seg_rows, out, out_bf16, ld, act, c->tc_err, m->stream, m->use_pdl && !m->profiling);
+        status = pair_gemm_launch(plan, w, w1, x, rows, N, K, out, out_bf16, ld, act, c->tc_err, m->stream, m->use_pdl && !m->profiling);
         if (status != OXG4_OK) return 1;
         prof_end(kind, e0, e1);
         ++kernels;
@@ -3390,11 +3388,11 @@ extern "C" int32_t oxg4_debug_tc_gemm(const uint16_t* w_host, const uint16_t* x_
 }
 
 // SM-pair projection, stand-alone entry of its parity tests: out[M, N] = x[M, K] . w[N, K]^T, or with w1 the BF16 value of
-// gelu(x . w^T) * (x . w1^T); seg_rows > 0: rows of w from s * seg_rows on multiply rows s * M .. of x.
+// gelu(x . w^T) * (x . w1^T).
 extern "C" int32_t oxg4_debug_pair_gemm(const uint16_t* w_host, const uint16_t* w1_host, const uint16_t* x_host, int32_t N, int32_t K,
-                                        int32_t M, int32_t seg_rows, float* out_host, int32_t* slots_or_null) {
+                                        int32_t M, float* out_host, int32_t* slots_or_null) {
     if (!w_host || !x_host || !out_host) return fail(OXG4_INVALID_ARGUMENT, "null argument");
-    if (M < 1 || M > kChunkRows || N < 1 || K < 8 || K % 8 != 0 || seg_rows < 0 || seg_rows % 128 != 0 || (w1_host && seg_rows > 0))
+    if (M < 1 || M > kChunkRows || N < 1 || K < 8 || K % 8 != 0)
         return fail(OXG4_INVALID_SHAPE, "SM-pair projection: 1..%d rows and K %% 8 == 0 required", kChunkRows);
     TRY(allow_big_smem(pair_gemm_kernel<PG_STORE>));
     TRY(allow_big_smem(pair_gemm_kernel<PG_GLU>));
@@ -3402,8 +3400,8 @@ extern "C" int32_t oxg4_debug_pair_gemm(const uint16_t* w_host, const uint16_t* 
     int dev = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaGetDeviceProperties(&prop, dev));
-    const size_t segs = seg_rows > 0 ? (N + seg_rows - 1) / seg_rows : 1, wb = (size_t)N * K * 2, xb = segs * M * K * 2;
-    const PairPlan plan = pair_plan(M, N, K, w1_host != nullptr, seg_rows, 2048, prop.multiProcessorCount);
+    const size_t wb = (size_t)N * K * 2, xb = (size_t)M * K * 2;
+    const PairPlan plan = pair_plan(M, N, K, w1_host != nullptr, 2048, prop.multiProcessorCount);
     const size_t ob = w1_host ? (size_t)M * N * 2 : (size_t)plan.S * M * N * 4;
     char* d = nullptr;
     auto up = [](size_t b) { return (b + 255) / 256 * 256; };
@@ -3417,7 +3415,7 @@ extern "C" int32_t oxg4_debug_pair_gemm(const uint16_t* w_host, const uint16_t* 
         cudaMemset(e, 0, 4) != cudaSuccess)
         s = fail(OXG4_CUDA, "Gemma 4 CUDA error: copy failed");
     if (s == OXG4_OK)
-        s = pair_gemm_launch(plan, w, w1_host ? w1 : nullptr, x, M, N, K, seg_rows, (float*)o, (uint16_t*)o, N, (int)ACT_GELU_TANH, (int*)e, 0, false);
+        s = pair_gemm_launch(plan, w, w1_host ? w1 : nullptr, x, M, N, K, (float*)o, (uint16_t*)o, N, (int)ACT_GELU_TANH, (int*)e, 0, false);
     if (s == OXG4_OK && (cudaMemcpy(host.data(), o, ob, cudaMemcpyDeviceToHost) != cudaSuccess || cudaMemcpy(&err, e, 4, cudaMemcpyDeviceToHost) != cudaSuccess))
         s = fail(OXG4_CUDA, "Gemma 4 CUDA error: SM-pair projection failed: %s", cudaGetErrorString(cudaGetLastError()));
     cudaFree(d);

@@ -50,7 +50,6 @@ struct PairGemmArgs {
     int bn;                  // weight rows of a tile, both halves together: a multiple of 32, at most 256
     int cut;                 // 1: k-blocks dealt as ranges (PG_STORE only), 0: whole tiles in turn
     int S;                   // most pieces of a tile (1 unless cut)
-    int seg_rows;            // > 0: weight rows [s * seg_rows, (s + 1) * seg_rows) multiply activation rows s * M ..; a multiple of bn
     float* out;              // PG_STORE: [S, M, ld]
     uint16_t* out_bf16;      // PG_GLU: [M, ld]
     int ld;
@@ -182,7 +181,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             if (!w.next()) return false;
             const int n0 = w.tile / tiles_m * cols;
             kb = w.kb0;
-            xrow = w.tile % tiles_m * kPgTileM + (int)rank * 128 + (a.seg_rows > 0 ? n0 / a.seg_rows * a.M : 0);
+            xrow = w.tile % tiles_m * kPgTileM + (int)rank * 128;
             wrow = EPI == PG_GLU ? n0 : n0 + (int)rank * (a.bn / 2);
             return true;
         };
@@ -359,12 +358,11 @@ inline int pair_pieces(int n_tiles, int KB, int pairs) {
 // 256-wide tile and hardly less for a narrower one (0.37 us at 128: the refill of shared memory and not the tensor cores
 // sets the pace), about 3 us to start and drain; every slot of partial outputs is written and read once (~4.5 TB/s).
 // max_rows: rows of `ld` floats that the output buffer holds (slots * M must fit). glu: gate and up in one launch.
-inline PairPlan pair_plan(int M, int N, int K, bool glu, int seg_rows, size_t max_rows, int num_sms) {
+inline PairPlan pair_plan(int M, int N, int K, bool glu, size_t max_rows, int num_sms) {
     const int P = num_sms / 2, KB = (K + kTcTileK - 1) / kTcTileK, tiles_m = (M + kPgTileM - 1) / kPgTileM;
     PairPlan best;
     double best_us = 1e30;
     for (int bn : {256, 224, 192, 160, 128}) {
-        if (seg_rows > 0 && seg_rows % bn != 0) continue;
         const int cols = glu ? bn / 2 : bn, T = tiles_m * ((N + cols - 1) / cols);
         const double kb_us = bn == 128 ? 0.37 : bn == 160 ? 0.41 : 0.42;
         auto consider = [&](int pairs, int cut) {

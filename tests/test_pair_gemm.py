@@ -1,5 +1,5 @@
 """GPU parity test of the SM-pair projection (tcgen05, cta_group::2) against a float64 matmul of the same BF16 values: whole
-tiles and tiles cut over several pairs, ragged rows, columns and depths, gate and up in one launch, segments of weight rows."""
+tiles and tiles cut over several pairs, ragged rows, columns and depths, gate and up in one launch."""
 import ctypes as C
 
 import numpy as np
@@ -15,11 +15,11 @@ def bf16(rng, shape, std):
     return bits, syn.bf16_bits_to_f32(bits).reshape(shape).astype(np.float64)
 
 
-def launch(w, w1, x, M, seg_rows=0):
+def launch(w, w1, x, M):
     N, K = w.shape
     out, slots = np.zeros((M, N), dtype=np.float32), C.c_int32(0)
     p = lambda a: None if a is None else a.ctypes.data_as(C.c_void_p)  # noqa: E731
-    pkg._native.check(pkg._native.lib().oxg4_debug_pair_gemm(p(w), p(w1), p(x), N, K, M, seg_rows, p(out), C.byref(slots)))
+    pkg._native.check(pkg._native.lib().oxg4_debug_pair_gemm(p(w), p(w1), p(x), N, K, M, p(out), C.byref(slots)))
     return out, slots.value
 
 
@@ -46,13 +46,3 @@ def test_gate_and_up(N, K, M):
     ref = 0.5 * g * (1.0 + np.tanh(0.7978845608 * (g + 0.044715 * g ** 3))) * (xd @ wd1.T)
     # one rounding to BF16 (2^-9) on top of f32 arithmetic; near zero the f32 sums' absolute error
     assert (np.abs(out - ref) <= 2.0 ** -8 * np.abs(ref) + 1e-4 * np.abs(ref).max()).all()
-
-
-@pytest.mark.parametrize("N,K,M,seg", [(640, 64, 100, 128), (1280, 512, 300, 256), (1000, 136, 513, 384)])
-def test_segments(N, K, M, seg):
-    rng = np.random.default_rng(N + K + M)
-    n = -(-N // seg)
-    (w, wd), (x, xd) = bf16(rng, (N, K), 0.05), bf16(rng, (n * M, K), 1.0)
-    out, _ = launch(w, None, x, M, seg)
-    ref = np.concatenate([xd[s * M:(s + 1) * M] @ wd[s * seg:(s + 1) * seg].T for s in range(n)], axis=1)
-    assert np.abs(out - ref).max() <= 2e-5 * max(1.0, np.abs(ref).max())
