@@ -317,11 +317,14 @@ int32_t oxg4_smoke_cached_attention(oxg4_model* model, oxg4_cache* cache, uint32
 /* Failure-path test hooks (no counterpart in the reference, whose errors are Result values and whose
  * capture always ends, crates/oxide-torch-cuda/src/cuda_graph.rs:84-97). Neither faults or hangs a GPU.
  * oxg4_debug_wait_timeout runs one of the library's bounded device-side waits (kind 1: mbarrier phase,
- * kind 2: tensor-parallel peer flag) on something nobody signals, with a polling budget of `spin_limit`:
- * the kernel returns, the status word is raised and the call returns OXG4_TIMEOUT; later calls work.
+ * kind 2: tensor-parallel peer flag) on something nobody signals, with a limit of `spin_limit` microseconds (kind 1) or
+ * polls (kind 2): the kernel returns, the status word is raised and the call returns OXG4_TIMEOUT; later calls work.
+ * oxg4_debug_set_status sets the status word of the table's tensor-core kernels as a failed wait would: the launches of the next
+ * call return without output, the call reports OXG4_TIMEOUT and clears the word.
  * oxg4_debug_fail_alloc_after makes the n-th device allocation of the next oxg4_cache_create report
  * OXG4_OOM (0 switches it off); the failed create must release everything it had allocated. */
 int32_t oxg4_debug_wait_timeout(oxg4_model* model, oxg4_cache* cache, int32_t kind, uint32_t spin_limit);
+int32_t oxg4_debug_set_status(oxg4_model* model, oxg4_cache* cache, int32_t code);
 void oxg4_debug_fail_alloc_after(int32_t n);
 
 /* Measurement aid (no counterpart in the reference): marks lens[b] positions of every sequence of an EMPTY cache
@@ -372,10 +375,12 @@ int32_t oxg4_debug_tc_gemm(const uint16_t* w_host, const uint16_t* x_host, int32
                            float* out_host, float* ms);
 
 /* The same for the SM-pair projection of prompt passes (csrc/pair_gemm.cuh): out[M, N] = x[M, K] . W[N, K]^T, or with w1 the
- * BF16 value of gelu(x . W^T) * (x . W1^T) widened to f32. 1 <= M <= 2048, K a multiple of 8. slots (may be NULL) receives the number of
+ * BF16 value of gelu(x . W^T) * (x . W1^T) widened to f32. status: the kernel's status word
+ * ahead of the launch; non-zero, the launch returns without output and the call reports OXG4_TIMEOUT, out being the untouched buffer (NaN).
+ * 1 <= M <= 2048, K a multiple of 8. slots (may be NULL) receives the number of
  * partial outputs. */
 int32_t oxg4_debug_pair_gemm(const uint16_t* w_host, const uint16_t* w1_host, const uint16_t* x_host, int32_t N, int32_t K,
-                             int32_t M, float* out_host, int32_t* slots);
+                             int32_t M, int32_t status, float* out_host, int32_t* slots);
 
 /* Diagnostics (no counterpart in the reference): when the environment variable OXG4_TIMELINE is
  * set before oxg4_model_create, every kernel of a step stamps the GPU's nanosecond timer at entry,

@@ -121,6 +121,7 @@ SYMBOLS = {
     "oxg4_profile_extend": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "oxg4_profile_ms": (C.c_float, [C.c_void_p, C.c_char_p]),
     "oxg4_profile_count": (C.c_int32, [C.c_void_p, C.c_char_p]),
+    "oxg4_debug_set_status": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_int32]),
     "oxg4_debug_wait_timeout": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_int32, C.c_uint32]),
     "oxg4_debug_fail_alloc_after": (None, [C.c_int32]),
     "oxg4_smoke_embedding_logits": (C.c_int32, [C.c_void_p, C.c_uint32, C.c_void_p]),
@@ -133,8 +134,8 @@ SYMBOLS = {
     "oxg4_decode_trace": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "oxg4_debug_tc_gemm": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_void_p,
                                        C.POINTER(C.c_float)]),
-    "oxg4_debug_pair_gemm": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_void_p,
-                                         C.POINTER(C.c_int32)]),
+    "oxg4_debug_pair_gemm": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_int32,
+                                         C.c_void_p, C.POINTER(C.c_int32)]),
     "oxg4_debug_timeline": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_int32]),
     "oxg4_generate": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_int64, C.POINTER(GenerationConfigC), C.c_int32,
                                   TOKEN_CALLBACK, C.c_void_p, C.c_void_p, C.POINTER(C.c_int64)]),

@@ -164,12 +164,12 @@ attn_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
     if (tid == 0) {
         for (int w = 0; w < NCW; ++w)
             for (int s = 0; s < NST; ++s) { mbar_init(&full[w][s], 1); mbar_init(&empty[w][s], 1); }
-        failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (tid < NCW) issued[tid] = 0;
     pdl_wait();
     pdl_launch();
+    // a launch behind a failed one returns at once; the thread that looks has no group to count unless there are many
+    if (tid == (int)blockDim.x - 1) failed = *(const volatile int*)a.err != 0;
     am_prefix(a, pre);                                         // contains the CTA-wide barriers
     const int T = pre[a.NG] * a.Nkv;
     const int W = (int)gridDim.x * NCW;
@@ -195,9 +195,8 @@ attn_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
                 const int32_t* pt = a.page_table + (size_t)seq * a.pages_per_seq;
                 for (; t < seg_end; ++t, ++lt, ++it) {
                     const int s = it % NST;
-                    if (it >= NST && !mbar_wait(&empty[lane][s], ((it / NST) & 1) ^ 1)) {
-                        failed = 1;
-                        atomicExch(a.err, 11);
+                    if (it >= NST && !mbar_wait(&empty[lane][s], ((it / NST) & 1) ^ 1, &failed)) {
+                        wait_failed(a.err, 11, &failed);
                         break;
                     }
                     const int slot = ((t0 + lt) * kAmTile) % cap;
@@ -228,7 +227,7 @@ attn_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
         const uint32_t q_off = (uint32_t)((((lm_i & 1) * 8 + lm_r) * QS + (lm_i >> 1) * 8) * 2);
         int t = begin, it = 0;
         const int end = begin + len;
-        bool lost = false;                                      // the same in all lanes of the warp: ldmatrix and mma are .aligned
+        bool lost = __any_sync(0xffffffffu, failed) != 0;       // the same in all lanes of the warp: ldmatrix and mma are .aligned
         while (t < end && !lost) {
             int g, kvh, lt, nt;
             am_locate(pre, a.NG, a.Nkv, t, g, kvh, lt, nt);
@@ -264,9 +263,9 @@ attn_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
 
             for (; t < seg_end; ++t, ++lt, ++it) {
                 const int s = it % NST;
-                if (!mbar_wait_warp(&full[warp][s], (it / NST) & 1)) {
+                if (!mbar_wait_warp(&full[warp][s], (it / NST) & 1, &failed)) {
                     lost = true;
-                    if (lane == 0) { failed = 1; atomicExch(a.err, 12); }
+                    if (lane == 0) wait_failed(a.err, 12, &failed);
                     break;
                 }
                 const uint32_t kb = smem_u32(stages + ((size_t)warp * NST + s) * STAGE);
@@ -351,13 +350,10 @@ attn_mma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
                 if ((lane & 3) == 0) { dst[D] = m_run; dst[D + 1] = l_run; }
             }
         }
-        // after a failed wait: let this warp's copies in flight land (bounded) before the CTA's memory goes away
-        if (lost) {
-            __syncwarp();
-            if (lane == 0)
-                for (int w_it = it; w_it < issued[warp]; ++w_it) mbar_wait(&full[warp][w_it % NST], (w_it / NST) & 1);
-        }
     }
+    // after a failed wait: let the copies in flight land (bounded) before the CTA's memory goes away
+    __syncthreads();
+    if (failed && tid < NCW) ring_drain(full[tid], empty[tid], NST, (uint32_t)issued[tid], 0u);
 }
 
 template <int D>

@@ -3279,6 +3279,15 @@ extern "C" int32_t oxg4_debug_wait_timeout(oxg4_model* m, oxg4_cache* c, int32_t
     return OXG4_OK;
 }
 
+// The status word of the tensor-core kernels as a failed wait would leave it (csrc/tc_gemm.cuh), ahead of a call.
+extern "C" int32_t oxg4_debug_set_status(oxg4_model* m, oxg4_cache* c, int32_t code) {
+    if (!m || !c || c->m != m) return fail(OXG4_INVALID_ARGUMENT, "null or mismatched handle");
+    TRY(bind_device(m));
+    CK(cudaStreamSynchronize(m->stream));
+    CK(cudaMemcpy(c->tc_err, &code, sizeof code, cudaMemcpyHostToDevice));
+    return OXG4_OK;
+}
+
 // ------------------------------------------------------------------------------------------------
 // top-k without any allocation
 // ------------------------------------------------------------------------------------------------
@@ -3388,9 +3397,10 @@ extern "C" int32_t oxg4_debug_tc_gemm(const uint16_t* w_host, const uint16_t* x_
 }
 
 // SM-pair projection, stand-alone entry of its parity tests: out[M, N] = x[M, K] . w[N, K]^T, or with w1 the BF16 value of
-// gelu(x . w^T) * (x . w1^T).
+// gelu(x . w^T) * (x . w1^T). status: the kernel's status word ahead of the launch; where it is set out receives the output buffer as
+// the launch left it (every byte of it 0xff before).
 extern "C" int32_t oxg4_debug_pair_gemm(const uint16_t* w_host, const uint16_t* w1_host, const uint16_t* x_host, int32_t N, int32_t K,
-                                        int32_t M, float* out_host, int32_t* slots_or_null) {
+                                        int32_t M, int32_t status, float* out_host, int32_t* slots_or_null) {
     if (!w_host || !x_host || !out_host) return fail(OXG4_INVALID_ARGUMENT, "null argument");
     if (M < 1 || M > kChunkRows || N < 1 || K < 8 || K % 8 != 0)
         return fail(OXG4_INVALID_SHAPE, "SM-pair projection: 1..%d rows and K %% 8 == 0 required", kChunkRows);
@@ -3408,11 +3418,11 @@ extern "C" int32_t oxg4_debug_pair_gemm(const uint16_t* w_host, const uint16_t* 
     CK(cudaMalloc(&d, 2 * up(wb) + up(xb) + up(ob) + 256));
     char *w = d, *w1 = w + up(wb), *x = w1 + up(wb), *o = x + up(xb), *e = o + up(ob);
     std::vector<uint8_t> host(ob);
-    int err = 0;
+    int err = status;
     int32_t s = OXG4_OK;
     if (cudaMemcpy(w, w_host, wb, cudaMemcpyHostToDevice) != cudaSuccess || cudaMemcpy(x, x_host, xb, cudaMemcpyHostToDevice) != cudaSuccess ||
         (w1_host && cudaMemcpy(w1, w1_host, wb, cudaMemcpyHostToDevice) != cudaSuccess) || cudaMemset(o, 0xff, ob) != cudaSuccess ||
-        cudaMemset(e, 0, 4) != cudaSuccess)
+        cudaMemcpy(e, &err, 4, cudaMemcpyHostToDevice) != cudaSuccess)
         s = fail(OXG4_CUDA, "Gemma 4 CUDA error: copy failed");
     if (s == OXG4_OK)
         s = pair_gemm_launch(plan, w, w1_host ? w1 : nullptr, x, M, N, K, (float*)o, (uint16_t*)o, N, (int)ACT_GELU_TANH, (int*)e, 0, false);
@@ -3420,7 +3430,6 @@ extern "C" int32_t oxg4_debug_pair_gemm(const uint16_t* w_host, const uint16_t* 
         s = fail(OXG4_CUDA, "Gemma 4 CUDA error: SM-pair projection failed: %s", cudaGetErrorString(cudaGetLastError()));
     cudaFree(d);
     TRY(s);
-    if (err) return fail(OXG4_TIMEOUT, "SM-pair projection: a bounded barrier wait ran out (code %d)", err);
     for (size_t i = 0; i < (size_t)M * N; ++i) {
         float t = 0.0f;
         if (w1_host) t = host_bf16_to_f32(((const uint16_t*)host.data())[i]);
@@ -3429,6 +3438,7 @@ extern "C" int32_t oxg4_debug_pair_gemm(const uint16_t* w_host, const uint16_t* 
         out_host[i] = t;
     }
     if (slots_or_null) *slots_or_null = plan.S;
+    if (err) return fail(OXG4_TIMEOUT, "SM-pair projection: a bounded barrier wait ran out (code %d)", err);
     return OXG4_OK;
 }
 

@@ -20,8 +20,11 @@
 // HBM once and the activations, a few MB, stay in L2), or all k-blocks of all tiles are dealt to the pairs as equal
 // contiguous ranges (few tiles: whole ones would leave pairs idle in the last round). A tile that is cut gives one partial
 // output per piece, slot = number of the piece inside the tile; the consumers add S slots in order, and the pair with a
-// tile's last piece clears the slots that the tile does not use. Every wait is bounded; after a failed one the pair stops issuing, waits (bounded) for its own
-// copies, meets at the closing cluster barrier, frees its TMEM and returns with `*err` set. No multicast loads.
+// tile's last piece clears the slots that the tile does not use. No multicast loads.
+//
+// Failures are those of tc_gemm.cuh (bounded waits, `*err`, launches that find it set), for both CTAs together: a CTA that stops
+// tells its partner, both meet at a cluster barrier, then CTA 0 waits (bounded) for all copies of the pair in flight, both for the
+// MMAs' commits, and they meet again before their shared memory and TMEM go away.
 //
 // Measured (B200, back-to-back launches): gate/up of the ~4B widths, 2048 rows, 163 us = 1.31 PFLOP/s of 1.40 sustained by
 // cuBLAS (weight-streaming kernel, eight blocks of 256 rows: 8 x 64 us + 8 x 15 us for the activation kernel); ~27B widths
@@ -68,6 +71,38 @@ DEVINL void cluster_sync_all() {
 // the pair's CTA 0 keeps the barriers that both CTAs' copies and epilogues signal: the CTA's own shared address with the
 // rank bit of the cluster window cleared
 constexpr uint32_t kPairLeadMask = 0xFEFFFFFFu;
+// the same shared variable in the other CTA of the pair
+DEVINL uint32_t partner_addr(const volatile void* p) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32((const void*)p)), "r"(cluster_rank() ^ 1u));
+    return a;
+}
+DEVINL uint32_t ld_partner(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(partner_addr(p)) : "memory");
+    return v;
+}
+DEVINL void pair_stop(volatile int* stop) {
+    *stop = 1;
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(partner_addr(stop)), "r"(1) : "memory");
+}
+DEVINL void pair_failed(int* err, int code, volatile int* stop) {
+    atomicCAS(err, 0, code);
+    pair_stop(stop);
+}
+// Between the two closing cluster barriers of a failed pair, one thread per CTA. CTA 0's barriers count both CTAs' bytes, which may have
+// stopped at different stages: `mine` / `theirs` stages filled, `half` bytes each.
+DEVINL void pair_drain(uint64_t* full, uint64_t* empty, uint64_t* acc_full, uint32_t rank, uint32_t mine, uint32_t theirs, uint32_t half,
+                       uint32_t committed, uint32_t accs) {
+    if (rank == 0) {
+        for (uint32_t i = mine; i < theirs; ++i) mbar_expect_tx(&full[i % kPgStages], half);
+        for (uint32_t i = theirs; i < mine; ++i)                // bytes that the partner did not send
+            asm volatile("mbarrier.complete_tx.relaxed.cluster.shared::cta.b64 [%0], %1;"
+                         ::"r"(smem_u32(&full[i % kPgStages])), "r"(half) : "memory");
+    }
+    ring_drain(full, empty, kPgStages, rank == 0 ? max(mine, theirs) : 0u, committed);
+    if (accs > 0) mbar_wait(&acc_full[(accs - 1) & 1], ((accs - 1) >> 1) & 1);
+}
 
 DEVINL void tma_load_2d_pair(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile(
@@ -145,6 +180,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     __shared__ __align__(8) uint64_t full[kPgStages], empty[kPgStages], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_base;
     __shared__ volatile int failed;
+    __shared__ uint32_t issued, committed, accs;               // ring stages filled, stages and accumulators whose MMAs were committed
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t rank = cluster_rank();
@@ -158,6 +194,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         for (int s = 0; s < kPgStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 16); }
         failed = 0;
+        committed = accs = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -205,7 +242,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         uint32_t it = (uint32_t)n_pre;
         for (; more && !failed; ++it) {
             const int s = it % kPgStages;
-            if (!mbar_wait(&empty[s], ((it / kPgStages) & 1) ^ 1)) { failed = 1; atomicExch(a.err, 1); break; }
+            if (!mbar_wait(&empty[s], ((it / kPgStages) & 1) ^ 1, &failed)) { pair_failed(a.err, 1, &failed); break; }
             if (rank == 0) mbar_expect_tx(&full[s], 2 * (kPgHalf + half_bytes));
             tma_load_2d_pair(tiles + (size_t)s * kPgStage, &map_x, kb * kTcTileK, xrow, &full[s]);
             tma_load_2d_pair(tiles + (size_t)s * kPgStage + kPgHalf, wm, kb * kTcTileK, wrow, &full[s]);
@@ -214,7 +251,8 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         // every stage has been read, so every copy has landed and every commit has been signalled, before the CTA ends
         const uint32_t tail = min(it, (uint32_t)kPgStages);
         for (uint32_t i = it - tail; i < it; ++i)
-            if (!mbar_wait(&empty[i % kPgStages], (i / kPgStages) & 1)) { failed = 1; atomicExch(a.err, 5); break; }
+            if (!mbar_wait(&empty[i % kPgStages], (i / kPgStages) & 1, &failed)) { pair_failed(a.err, 5, &failed); break; }
+        issued = it;
     } else {
         pdl_wait();
         pdl_launch();
@@ -226,13 +264,13 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         PairWalk w = start;
         for (; !failed && w.next(); ++tile_i) {
             const uint32_t ab = tile_i & 1, use = tile_i >> 1;
-            if (use > 0 && !mbar_wait(&acc_empty[ab], (use - 1) & 1)) { failed = 1; atomicExch(a.err, 2); break; }
+            if (use > 0 && !mbar_wait(&acc_empty[ab], (use - 1) & 1, &failed)) { pair_failed(a.err, 2, &failed); break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t acc = tmem + ab * 256;
             const int nk = w.kb1 - w.kb0;
             for (int j = 0; j < nk; ++j, ++it) {
                 const int s = it % kPgStages;
-                if (!mbar_wait(&full[s], (it / kPgStages) & 1)) { failed = 1; atomicExch(a.err, 3); break; }
+                if (!mbar_wait(&full[s], (it / kPgStages) & 1, &failed)) { pair_failed(a.err, 3, &failed); break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned char* sa = tiles + (size_t)s * kPgStage;
                 const uint64_t da = umma_smem_desc(sa), db = umma_smem_desc(sa + kPgHalf);
@@ -247,8 +285,10 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 }
                 mma_commit_pair(&empty[s]);
             }
+            committed = it;
             if (failed) break;
             mma_commit_pair(&acc_full[ab]);
+            accs = tile_i + 1;
         }
     }
     __syncwarp();
@@ -258,9 +298,11 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         const int quad = warp & 3, part = (warp - 2) >> 2;
         uint32_t tile_i = 0;
         PairWalk w = start;
-        for (; w.next(); ++tile_i) {
+        const bool dead = failed_before(a.err);
+        if (dead && lane == 0) pair_stop(&failed);
+        for (; !dead && w.next(); ++tile_i) {
             const uint32_t ab = tile_i & 1, use = tile_i >> 1;
-            if (!mbar_wait_warp(&acc_full[ab], use & 1)) { if (lane == 0) { failed = 1; atomicExch(a.err, 4); } break; }
+            if (!mbar_wait_warp(&acc_full[ab], use & 1, &failed)) { if (lane == 0) pair_failed(a.err, 4, &failed); break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int n0 = w.tile / tiles_m * cols;
             const int row = w.tile % tiles_m * kPgTileM + (int)rank * 128 + quad * 32 + lane;
@@ -333,6 +375,14 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     __syncthreads();
     __syncwarp();
     cluster_sync_all();
+    if (failed) {                                              // the same in all threads of the pair: nobody sets it behind the barrier
+        if (tid == 0)
+            pair_drain(full, empty, acc_full, rank, issued, ld_partner(&issued), kPgHalf + half_bytes, rank == 0 ? committed : ld_partner(&committed),
+                       rank == 0 ? accs : ld_partner(&accs));
+        __syncthreads();
+        __syncwarp();
+        cluster_sync_all();
+    }
     if (warp == 0) {
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
     }

@@ -16,8 +16,10 @@
 //
 // A CTA walks the work units (tile, K-split, row block) u = blockIdx.x, blockIdx.x + gridDim.x, ... Rows past the end of the
 // matrix and batch rows past B are zero-filled by TMA (tensor-map bounds) and masked at the store.
-// Every mbarrier wait is bounded: when a wait runs out the kernel raises `*err`, stops issuing work,
-// still frees its TMEM columns and returns, so a protocol bug cannot hang the GPU.
+// Every mbarrier wait is bounded in time: when one runs out the kernel raises `*err`, all its other waits give up, it stops issuing
+// work, lets its copies and MMAs in flight end (bounded), frees its TMEM columns and returns, so a protocol bug cannot hang
+// the GPU. A launch that finds `*err` set returns without output: after a failure the rest of a pass takes no limit each. The
+// epilogue warps look, whose first accumulator is a tile's K loop away; the copies and MMAs need not wait for the load.
 //
 // HBM-bound: bytes per launch = N * K * 2 (+ B * K * 2 per tile from L2 for the activations).
 #pragma once
@@ -32,7 +34,7 @@ constexpr int kTcTileM = 128;        // weight rows per tile (UMMA M)
 constexpr int kTcTileK = 64;         // BF16 elements per stage row = 128 bytes = one swizzle atom row
 // shared-memory stages of the TMA ring: 6 x 24 KiB for up to 64 activation rows per block, 4 x 48 KiB for 256
 template <int BN> struct TcStages { static constexpr int value = BN <= 64 ? 6 : (BN <= 128 ? 5 : 4); };
-constexpr uint32_t kTcSpinLimit = 2u * 1000u * 1000u;   // bounded mbarrier polling
+constexpr uint64_t kWaitNs = 1000u * 1000u * 1000u;     // limit of an mbarrier wait
 
 struct TcGemmArgs {
     int N, K, B;             // rows of ONE weight matrix, columns, activation rows (cut into blocks of BN rows)
@@ -57,10 +59,18 @@ DEVINL void mbar_init(uint64_t* bar, uint32_t count) {
 DEVINL void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
-// returns false if the phase did not complete within the polling budget
-DEVINL bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t limit = kTcSpinLimit) {
+DEVINL uint64_t global_ns() {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+// One thread's bounded wait: false if the phase did not complete within the limit, or if `stop` (shared memory) was set meanwhile.
+// One loop that looks at the clock once in 1024 polls: with the polls in a loop of their own inside it, of 16 or of 1024, the producer
+// fell behind HBM (decode step of the ~4B widths, 16 sequences: 3.08 ms, 2.90 so; 2.89 with a limit in polls).
+DEVINL bool mbar_wait(uint64_t* bar, uint32_t parity, const volatile int* stop = nullptr, uint64_t limit_ns = kWaitNs) {
     const uint32_t addr = smem_u32(bar);
-    for (uint32_t i = 0; i < limit; ++i) {
+    uint64_t start = 0;
+    for (uint32_t i = 0;; ++i) {
         uint32_t done;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -70,13 +80,31 @@ DEVINL bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t limit = kTcSpinLi
             : "r"(addr), "r"(parity)
             : "memory");
         if (done) return true;
+        if ((i & 1023u) != 1023u) continue;
+        if (stop != nullptr && *stop) return false;
+        const uint64_t now = global_ns();
+        if (start == 0) start = now;
+        else if (now - start > limit_ns) return false;
     }
-    return false;
 }
-// The same for a whole warp, which goes on together with one answer: false when the budget of any lane ran out. A lane that went its
+// The same for a whole warp, which goes on together with one answer: false when any lane's wait failed. A lane that went its
 // own way would leave the others at an .aligned instruction or a full-mask barrier that never sees it.
-DEVINL bool mbar_wait_warp(uint64_t* bar, uint32_t parity, uint32_t limit = kTcSpinLimit) {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit));
+DEVINL bool mbar_wait_warp(uint64_t* bar, uint32_t parity, const volatile int* stop = nullptr, uint64_t limit_ns = kWaitNs) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, stop, limit_ns));
+}
+// After a failed wait: the first code stays, all waits of the CTA that poll `stop` give up.
+DEVINL void wait_failed(int* err, int code, volatile int* stop) {
+    atomicCAS(err, 0, code);
+    *stop = 1;
+}
+// Whole warp: an earlier launch of the pass has failed; this one shall return at once.
+DEVINL bool failed_before(const int* err) { return __any_sync(0xffffffffu, *(const volatile int*)err != 0); }
+// One thread, after the failure: waits (bounded) until `issued` copies into a ring of `stages` have landed and the MMAs up to the
+// `committed`-th commit have read them.
+DEVINL void ring_drain(uint64_t* full, uint64_t* empty, uint32_t stages, uint32_t issued, uint32_t committed) {
+    for (uint32_t i = issued > stages ? issued - stages : 0; i < issued; ++i)
+        if (!mbar_wait(&full[i % stages], (i / stages) & 1)) break;
+    if (committed > 0) mbar_wait(&empty[(committed - 1) % stages], ((committed - 1) / stages) & 1);
 }
 
 DEVINL void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
@@ -125,6 +153,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     __shared__ __align__(8) uint64_t full[kTcStages], empty[kTcStages], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_base;
     __shared__ volatile int failed;
+    __shared__ uint32_t issued, committed;                     // ring stages filled, ring stages whose MMAs have been committed
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tiles_per_mat = (a.N + kTcTileM - 1) / kTcTileM;
@@ -197,16 +226,18 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         pdl_wait();
         pdl_launch();
         for (int i = 0; i < n_pre; ++i) tma_load_2d(tiles + (size_t)i * STAGE + A_BYTES, &map_x, pre_x[i], pre_row[i], &full[i]);
-        for (uint32_t it = (uint32_t)n_pre; t < n_tiles && !failed; ++it) {
+        uint32_t it = (uint32_t)n_pre;
+        for (; t < n_tiles && !failed; ++it) {
             const int s = it % kTcStages;
             const uint32_t ph = (it / kTcStages) & 1;
-            if (!mbar_wait(&empty[s], ph ^ 1)) { failed = 1; atomicExch(a.err, 1); break; }
+            if (!mbar_wait(&empty[s], ph ^ 1, &failed)) { wait_failed(a.err, 1, &failed); break; }
             mbar_expect_tx(&full[s], A_BYTES + B_BYTES);
             const int kx = (k0 + jr) * kTcTileK;
             tma_load_2d(tiles + (size_t)s * STAGE, wmap, kx, trow, &full[s]);
             tma_load_2d(tiles + (size_t)s * STAGE + A_BYTES, &map_x, kx, xrow, &full[s]);
             advance();
         }
+        issued = it;
     } else {
         pdl_wait();
         pdl_launch();
@@ -218,14 +249,14 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         for (int t = blockIdx.x; t < n_tiles && !failed; t += gridDim.x, ++tile_i) {
             // accumulator tile_i % 2; its previous user (unit tile_i - 2) must have been drained by the epilogue
             const uint32_t ab = tile_i & 1, use = tile_i >> 1;
-            if (use > 0 && !mbar_wait(&acc_empty[ab], (use - 1) & 1)) { failed = 1; atomicExch(a.err, 2); break; }
+            if (use > 0 && !mbar_wait(&acc_empty[ab], (use - 1) & 1, &failed)) { wait_failed(a.err, 2, &failed); break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t acc = tmem + ab * ACC_COLS;
             const int nk = kb_end(t) - kb_begin(t);
             for (int j = 0; j < nk; ++j, ++it) {
                 const int s = it % kTcStages;
                 const uint32_t ph = (it / kTcStages) & 1;
-                if (!mbar_wait(&full[s], ph)) { failed = 1; atomicExch(a.err, 3); break; }
+                if (!mbar_wait(&full[s], ph, &failed)) { wait_failed(a.err, 3, &failed); break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const unsigned char* sa = tiles + (size_t)s * STAGE;
                 const uint64_t da = umma_smem_desc(sa), db = umma_smem_desc(sa + A_BYTES);
@@ -245,6 +276,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             if (failed) break;
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&acc_full[ab])) : "memory");
         }
+        committed = it;
     }
     __syncwarp();
 
@@ -252,9 +284,11 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     if (warp >= 2) {
         const int quad = warp & 3;
         uint32_t tile_i = 0;
-        for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, ++tile_i) {
+        const bool dead = failed_before(a.err);
+        if (dead && lane == 0) failed = 1;
+        for (int t = blockIdx.x; t < n_tiles && !dead; t += gridDim.x, ++tile_i) {
             const uint32_t ab = tile_i & 1, use = tile_i >> 1;
-            if (!mbar_wait_warp(&acc_full[ab], use & 1)) { if (lane == 0) { failed = 1; atomicExch(a.err, 4); } break; }
+            if (!mbar_wait_warp(&acc_full[ab], use & 1, &failed)) { if (lane == 0) wait_failed(a.err, 4, &failed); break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int tg = t / (a.S * a.TB), sp = (t / a.TB) % a.S, b0 = (t % a.TB) * BN;
             const bool second = tg >= tiles_per_mat;
@@ -285,6 +319,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     // ---- teardown: always reached, also after a failed wait ----
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (failed) {                                              // the same in all threads: nobody sets it behind the barrier
+        if (tid == 0) ring_drain(full, empty, kTcStages, issued, committed);
+        __syncthreads();
+    }
     if (warp == 0) {
         __syncwarp();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TM_COLS));

@@ -1,8 +1,12 @@
 """Bounded waits of the tensor-core pipelines (csrc/tc_gemm.cuh). No GPU fault, trap or hang: every wait here has a limit, and what is
 waited for is a flag that comes late or never."""
+import ctypes as C
+import time
+
+import numpy as np
 import pytest
 
-from util import build_pair, pkg, small_cfg
+from util import build_pair, pkg, small_cfg, syn
 
 pytestmark = pytest.mark.gpu
 
@@ -21,3 +25,45 @@ def test_lanes_of_a_warp_hear_one_answer(model):
     status = N.lib().oxg4_debug_wait_timeout(model._h, table._h, 1, 1000)
     assert N.STATUS_NAMES[status] == "TIMEOUT", N.lib().oxg4_last_error()
     assert b"mbarrier wait" in N.lib().oxg4_last_error()
+
+
+@pytest.mark.parametrize("gate_up", [False, True])
+@pytest.mark.parametrize("N,K,M", [(8, 8, 2), (520, 136, 257), (2560, 10240, 300), (4104, 320, 2000)])
+def test_pair_projection_behind_a_failure_returns_without_output(N, K, M, gate_up):
+    """One tile and many, whole and cut ones; a bounded wait that ran out in it would take a second."""
+    w, x, out = np.zeros((N, K), dtype=np.uint16), np.zeros((M, K), dtype=np.uint16), np.zeros((M, N), dtype=np.float32)
+    p = lambda a: a.ctypes.data_as(C.c_void_p)  # noqa: E731
+    fn, n = pkg._native.lib().oxg4_debug_pair_gemm, pkg._native.STATUS_NAMES
+    assert n[fn(p(w), p(w) if gate_up else None, p(x), N, K, M, 0, p(out), None)] == "OK" and (out == 0).all()
+    start = time.monotonic()
+    assert n[fn(p(w), p(w) if gate_up else None, p(x), N, K, M, 4, p(out), None)] == "TIMEOUT"
+    assert np.isnan(out).all() and time.monotonic() - start < 1.0
+    assert n[fn(p(w), p(w) if gate_up else None, p(x), N, K, M, 0, p(out), None)] == "OK" and (out == 0).all()
+
+
+def test_calls_behind_a_failure_report_it_and_the_next_ones_work(model):
+    """A prompt on SM pairs with prompt attention, a short portion on the weight-streaming projections with the paged attention, and
+    steps of eight sequences: each behind a set status word. No launch may use up a wait's limit (a second each)."""
+    N = pkg._native
+    tokens = syn.prompt_ids(500, 8 * 40, seed=3)
+    lens = [40] * 8
+
+    calls = [lambda table: model.prefill_prompt(tokens, table, lens=lens),
+             lambda table: model.extend(tokens[:16], table, lens=[2] * 8, want=[15]),
+             lambda table: model.decode_token(tokens[:8], table),
+             lambda table: model.decode_greedy(tokens[:8], table, 4)[0]]
+    new = lambda: model.new_cache_table([64] * 8, batch=8, page_tokens=16, kv_dtype=pkg.BF16)  # noqa: E731
+    table = new()
+    clean = [call(table) for call in calls]
+    for i, call in enumerate(calls):
+        table = new()
+        for earlier in calls[:i]:
+            earlier(table)
+        N.check(N.lib().oxg4_debug_set_status(model._h, table._h, 12))
+        start = time.monotonic()
+        with pytest.raises(N.Oxg4Error, match="TIMEOUT"):
+            call(table)
+        assert time.monotonic() - start < 1.0
+        table.reset()
+        for again, want in zip(calls[:i + 1], clean):
+            assert np.array_equal(again(table), want)

@@ -19,7 +19,7 @@ def launch(w, w1, x, M):
     N, K = w.shape
     out, slots = np.zeros((M, N), dtype=np.float32), C.c_int32(0)
     p = lambda a: None if a is None else a.ctypes.data_as(C.c_void_p)  # noqa: E731
-    pkg._native.check(pkg._native.lib().oxg4_debug_pair_gemm(p(w), p(w1), p(x), N, K, M, p(out), C.byref(slots)))
+    pkg._native.check(pkg._native.lib().oxg4_debug_pair_gemm(p(w), p(w1), p(x), N, K, M, 0, p(out), C.byref(slots)))
     return out, slots.value
 
 
