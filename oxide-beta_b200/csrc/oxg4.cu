@@ -975,11 +975,13 @@ static int32_t cache_build(oxg4_cache* c) {
     TRY(dalloc(c, &c->rng, B));
     TRY(dalloc(c, &c->hA, (size_t)R * H));
     TRY(dalloc(c, &c->hB, (size_t)R * H));
-    TRY(dalloc(c, &c->qkv_raw, (size_t)R * m->qkv_n_max));
+    // outputs of the small-batch kernels: the prompts of a wide table never go through these, only its steps do
+    const int S = c->wide ? B : R;
+    TRY(dalloc(c, &c->qkv_raw, (size_t)S * m->qkv_n_max));
     TRY(dalloc(c, &c->attn_out, (size_t)R * qw));
-    TRY(dalloc(c, &c->o_raw, (size_t)R * H));
-    TRY(dalloc(c, &c->gu_raw, (size_t)R * m->I));
-    TRY(dalloc(c, &c->down_raw, (size_t)R * H));
+    TRY(dalloc(c, &c->o_raw, (size_t)S * H));
+    TRY(dalloc(c, &c->gu_raw, (size_t)S * m->I));
+    TRY(dalloc(c, &c->down_raw, (size_t)S * H));
     TRY(dalloc(c, &c->logits, (size_t)B * m->V));
     TRY(dalloc(c, &c->attn_part, (size_t)A * part_floats));
     TRY(dalloc(c, &c->attn_ticket, (size_t)A * ticket_n));
