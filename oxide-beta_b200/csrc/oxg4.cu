@@ -2184,7 +2184,7 @@ static void lm_head(oxg4_cache* c, Launcher& ln, int kind, int top_k, float pena
             const int chunks = (m->Vloc + kTopkChunk - 1) / kTopkChunk;
             ln.go("topk1", topk_stage1_kernel, dim3(chunks, B), dim3(kTopkThreads), 0, (const float*)c->logits, m->V,
                   m->v0, m->Vloc, (const uint8_t*)c->seen, penalty, k, c->topk_stage);
-            ln.go("topk2", topk_stage2_kernel, dim3(1, B), dim3(kTopkThreads), topk_merge_smem(chunks * k, k),
+            ln.go("topk2", topk_stage2_kernel, dim3(1, B), dim3(kTopkThreads), topk_merge_smem(chunks * k),
                   (const Cand*)c->topk_stage, chunks * k, k, c->loc_ids, c->loc_scores);
             ln.allgather(c->loc_scores, c->tpk_scores, sizeof(float) * B * k);
             ln.allgather(c->loc_ids, c->tpk_ids, sizeof(uint32_t) * B * k);
@@ -2202,7 +2202,7 @@ static void lm_head(oxg4_cache* c, Launcher& ln, int kind, int top_k, float pena
         const int chunks = (m->V + kTopkChunk - 1) / kTopkChunk;
         ln.go("topk1", topk_stage1_kernel, dim3(chunks, B), dim3(kTopkThreads), 0, (const float*)c->logits, m->V, 0,
               m->V, (const uint8_t*)c->seen, penalty, k, c->topk_stage);
-        ln.go("topk2", topk_stage2_kernel, dim3(1, B), dim3(kTopkThreads), topk_merge_smem(chunks * k, k),
+        ln.go("topk2", topk_stage2_kernel, dim3(1, B), dim3(kTopkThreads), topk_merge_smem(chunks * k),
               (const Cand*)c->topk_stage, chunks * k, k, out_ids, out_scores);
         return;
     }
@@ -2243,7 +2243,7 @@ static void lm_head(oxg4_cache* c, Launcher& ln, int kind, int top_k, float pena
         const int chunks = (m->V + kTopkChunk - 1) / kTopkChunk;
         ln.go("topk1", topk_stage1_kernel, dim3(chunks, B), dim3(kTopkThreads), 0, (const float*)c->logits,
               m->V, 0, m->V, (const uint8_t*)c->seen, penalty, top_k, c->topk_stage);
-        ln.go("topk2", topk_stage2_kernel, dim3(1, B), dim3(kTopkThreads), topk_merge_smem(chunks * top_k, top_k),
+        ln.go("topk2", topk_stage2_kernel, dim3(1, B), dim3(kTopkThreads), topk_merge_smem(chunks * top_k),
               (const Cand*)c->topk_stage, chunks * top_k, top_k, c->topk_ids, c->topk_scores);
     }
 }
@@ -3334,7 +3334,7 @@ extern "C" int32_t oxg4_topk_noalloc(const float* logits_dev, int32_t rows, int3
     topk_stage1_kernel<<<dim3(chunks, rows), kTopkThreads, 0, st>>>(logits_dev, vocab, 0, vocab, seen_dev,
                                                                     repetition_penalty, top_k, scratch);
     CK(cudaGetLastError());
-    topk_stage2_kernel<<<dim3(1, rows), kTopkThreads, topk_merge_smem(chunks * top_k, top_k), st>>>(scratch, chunks * top_k, top_k,
+    topk_stage2_kernel<<<dim3(1, rows), kTopkThreads, topk_merge_smem(chunks * top_k), st>>>(scratch, chunks * top_k, top_k,
                                                                                         ids_dev, scores_dev);
     CK(cudaGetLastError());
     return OXG4_OK;

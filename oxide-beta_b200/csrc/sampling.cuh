@@ -166,19 +166,18 @@ DEVINL uint64_t warp_max_key(uint64_t k) {
     return ((uint64_t)hi << 32) | lo;
 }
 
-// The best top_k of `lists` sorted lists of `len` candidates each, by one warp; out(r, where) receives the place of the r-th one in
-// `c` (list * len + entry), or -1 where there are no more. `at` holds a place in each list (shared memory, lists of at most 64).
+// The best top_k of `lists` sorted lists of `len` candidates each (at most 64), by one warp; out(r, where) receives the place of the r-th
+// one in `c`, or -1 where there are no more. What is taken leaves its list, so that a list's best candidate is always its first: the
+// merge needs no memory beside the lists, and takes as many of them as shared memory holds.
 template <typename F>
-DEVINL void merge_lists(const Cand* c, int lists, int len, int top_k, uint8_t* at, F&& out) {
+DEVINL void merge_lists(Cand* c, int lists, int len, int top_k, F&& out) {
     const int lane = threadIdx.x & 31;
-    for (int l = lane; l < lists; l += 32) at[l] = 0;
     uint64_t best = 0;
-    int from = -1;
+    int from = 0;
     auto look = [&]() {                                        // the best head of the lane's lists
         best = 0;
         for (int l = lane; l < lists; l += 32) {
-            if (at[l] >= len) continue;
-            const Cand o = c[l * len + at[l]];
+            const Cand o = c[l * len];
             const uint64_t k = cand_key(o.s, o.i);
             if (k > best) { best = k; from = l; }
         }
@@ -188,12 +187,23 @@ DEVINL void merge_lists(const Cand* c, int lists, int len, int top_k, uint8_t* a
         const uint64_t m = warp_max_key(best);
         if (m == 0) {
             if (lane == 0) out(r, -1);
-        } else if (m == best) {                                // ids are unique: one lane
-            out(r, from * len + at[from]);
-            ++at[from];
-            look();
+            continue;
+        }
+        const bool mine = m == best;                           // ids are unique: one lane
+        if (mine) out(r, from * len);
+        Cand* list = c + __shfl_sync(0xffffffffu, from, __ffs(__ballot_sync(0xffffffffu, mine)) - 1) * len;
+        Cand next[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int i = lane + 32 * q;
+            if (i < len) next[q] = i + 1 < len ? list[i + 1] : Cand{-INFINITY, 0u};
         }
         __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+            if (lane + 32 * q < len) list[lane + 32 * q] = next[q];
+        __syncwarp();
+        if (mine) look();
     }
 }
 
@@ -204,7 +214,6 @@ topk_stage1_kernel(const float* logits, int ld, int col0, int n_cols, const uint
                    Cand* stage) {
     constexpr int W = kTopkThreads / 32, E = kTopkChunk / kTopkThreads;
     __shared__ Cand list[W * 64];
-    __shared__ uint8_t at[W];
     pdl_wait();
     pdl_launch();
     const int b = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -261,7 +270,7 @@ topk_stage1_kernel(const float* logits, int ld, int col0, int n_cols, const uint
     __syncthreads();
     if (warp != 0) return;
     Cand* dst = stage + ((size_t)b * gridDim.x + blockIdx.x) * top_k;
-    merge_lists(list, W, top_k, top_k, at, [&](int r, int where) { dst[r] = where < 0 ? Cand{-INFINITY, 0u} : list[where]; });
+    merge_lists(list, W, top_k, top_k, [&](int r, int where) { dst[r] = where < 0 ? Cand{-INFINITY, 0u} : list[where]; });
 }
 
 // Tensor parallelism: every rank holds the sorted top-k of its vocabulary slice; after an all-gather
@@ -271,7 +280,6 @@ __global__ void __launch_bounds__(kTopkThreads)
 tp_topk_merge_kernel(int B, int ranks, int k, const float* all_scores, const uint32_t* all_ids, uint32_t* ids,
                      float* scores) {
     __shared__ Cand all[8 * 64];
-    __shared__ uint8_t at[8];
     pdl_wait();
     pdl_launch();
     const int b = blockIdx.x, n = ranks * k;
@@ -281,26 +289,25 @@ tp_topk_merge_kernel(int B, int ranks, int k, const float* all_scores, const uin
     }
     __syncthreads();
     if (threadIdx.x >= 32) return;
-    merge_lists(all, ranks, k, k, at, [&](int r, int where) {
+    merge_lists(all, ranks, k, k, [&](int r, int where) {
         ids[(size_t)b * k + r] = where < 0 ? 0u : all[where].i;
         scores[(size_t)b * k + r] = where < 0 ? -INFINITY : all[where].s;
     });
 }
 
-// grid (1, B): merge of n / top_k sorted lists of top_k candidates; dynamic shared memory topk_merge_smem(n, top_k)
-inline size_t topk_merge_smem(int n, int top_k) { return (size_t)n * sizeof(Cand) + (size_t)(n / top_k); }
+// grid (1, B): merge of n / top_k sorted lists of top_k candidates; dynamic shared memory topk_merge_smem(n)
+inline size_t topk_merge_smem(int n) { return (size_t)n * sizeof(Cand); }
 __global__ void __launch_bounds__(kTopkThreads)
 topk_stage2_kernel(const Cand* stage, int n, int top_k, uint32_t* ids, float* scores) {
     extern __shared__ __align__(16) unsigned char sm2[];
     Cand* all = reinterpret_cast<Cand*>(sm2);
-    uint8_t* at = reinterpret_cast<uint8_t*>(all + n);
     pdl_wait();
     pdl_launch();
     const int b = blockIdx.y;
     for (int i = threadIdx.x; i < n; i += kTopkThreads) all[i] = stage[(size_t)b * n + i];
     __syncthreads();
     if (threadIdx.x >= 32) return;
-    merge_lists(all, n / top_k, top_k, top_k, at, [&](int r, int where) {
+    merge_lists(all, n / top_k, top_k, top_k, [&](int r, int where) {
         ids[(size_t)b * top_k + r] = where < 0 ? 0u : all[where].i;
         scores[(size_t)b * top_k + r] = where < 0 ? -INFINITY : all[where].s;
     });

@@ -5,7 +5,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from util import pkg
+from util import build_pair, pkg, small_cfg
 
 pytestmark = pytest.mark.gpu
 
@@ -65,3 +65,16 @@ def test_rows_with_few_candidates():
         assert ids[r].tolist() == want_ids.tolist(), r
         np.testing.assert_array_equal(scores[r], want_scores)
         np.testing.assert_array_equal(np.signbit(scores[r]), np.signbit(want_scores))
+
+
+def test_lists_fill_shared_memory():
+    """966 chunks of 2048 scores with 30 candidates each take 231840 of the 232448 bytes that a block can have: the merge may need next to
+    nothing beside the lists."""
+    k, vocab = 30, 966 * 2048 - 5
+    gpu, _ = build_pair(small_cfg(hidden=16, layers=1, heads=1, kv_heads=1, head_dim=64, inter=32, vocab=vocab, window=8), "bf16",
+                        kv_bf16=False, want_oracle=False)
+    a, b = gpu.new_cache_table(4, kv_dtype=pkg.F32), gpu.new_cache_table(4, kv_dtype=pkg.F32)
+    want_ids, want_scores = _want(gpu.decode_token(7, a), None, 1.0, k)
+    got = gpu.decode_topk(7, b, k, 1.0, False)
+    assert [i for i, _ in got] == want_ids.tolist()
+    np.testing.assert_array_equal(np.array([s for _, s in got], dtype=np.float32), want_scores)
