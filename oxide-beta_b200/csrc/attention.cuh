@@ -518,8 +518,7 @@ DEVINL void attn_cta(const AttnArgs& a, float* sm, const int s, const int kvh, c
                 sl[idx] = __ldcg(part + (size_t)sp * PS + g * (D + 2) + D + 1);
             }
             bar();
-            if (warp < G) {
-                const int g = warp;
+            for (int g = warp; g < G; g += NW) {               // a CTA of many has four warps, a group up to eight heads
                 float M = -INFINITY;
                 for (int sp = lane; sp < n_eff; sp += 32) M = fmaxf(M, sf[sp * G + g]);
                 M = warp_max(M);
