@@ -961,7 +961,8 @@ static int32_t cache_build(oxg4_cache* c) {
     c->tc_ok = m->es == 2 && m->P == 0 && (m->layered || getenv("OXG4_DISABLE_TCGEN05") == nullptr);
     // a KV-shared layer attends after its source layer has appended a whole pass, so a pass may not outgrow the ring's spare rows
     c->wide = c->tc_ok && !m->layered && m->tp == 1 && m->cfg.num_kv_shared_layers == 0;
-    c->prompt_attn = c->wide && c->kv_dtype == OXG4_BF16 && getenv("OXG4_DISABLE_MMA_ATTN") == nullptr;
+    // where steps attend with queries and softmax weights in f32 (csrc/attention.cuh), prompts do so too, and not with pairs of BF16 values
+    c->prompt_attn = c->wide && c->mma_attn;
     int64_t all_tokens = 0;
     for (int b = 0; b < B; ++b) all_tokens += c->max_seq[b];
     c->chunk_rows = c->wide ? (int)std::max<int64_t>(kPrefillRows, std::min<int64_t>(kChunkRows, (all_tokens + 255) / 256 * 256)) : kPrefillRows;
@@ -1025,7 +1026,6 @@ static int32_t cache_build(oxg4_cache* c) {
         TRY(dalloc(c, &c->am_pre, (size_t)kAmMaxGroups + 1));
     }
     if (c->prompt_attn) {
-        if (!c->mma_attn) TRY(dalloc(c, &c->q_hl, (size_t)R * 2 * m->qw_max));
         TRY(dalloc(c, &c->pa_k, (size_t)c->chunk_rows * m->kvw_max));
         TRY(dalloc(c, &c->pa_v, (size_t)c->chunk_rows * m->kvw_max));
         TRY(dalloc(c, &c->pa_part, (size_t)kPaPartRows * (m->qw_max + 2 * m->Nq)));

@@ -76,3 +76,38 @@ def test_unequal_prompts_of_one_pass():
         assert np.abs(got[i] - ref[0]).max() <= TOL_BF16
         if more[i]:
             assert np.abs(got2[fed.index(i)] - ref[-1]).max() <= TOL_BF16
+
+
+@pytest.mark.parametrize("page,mma", [(16, True), (48, True), (7, False), (24, False), (1, False)])
+def test_pages_of_odd_sizes_keep_queries_in_f32(page, mma):
+    """Pages of a multiple of 16 tokens attend on the tensor cores, with queries and softmax weights as pairs of BF16 values (2^-17),
+    steps and prompts alike. With any other page size both are held in f32, and a prompt has to go through the same kernel as a step."""
+    gpu, _ = build_pair(_cfg(64, 4, 2, 50), "bf16", kv_bf16=True, want_oracle=False)
+    table = gpu.new_cache_table(310, page_tokens=page, kv_dtype=pkg.BF16)
+    for n in (63, 64, 97, 80):
+        kinds = gpu.profile_extend(syn.prompt_ids(700, n, seed=n), table)
+        assert ("kv_append" in kinds) == (mma and n >= 64)       # prompt_attn_kernel ran
+        assert mma or "attn_merge" not in kinds                  # no tensor-core attention at all
+
+
+@pytest.mark.parametrize("head_dim,heads,kv_heads", [(64, 4, 2), (64, 4, 1), (128, 2, 1), (256, 2, 2)])
+@pytest.mark.parametrize("kind,window", [("full_attention", 9), ("sliding_attention", 70)])
+def test_attention_keeps_the_low_parts_of_queries_and_weights(head_dim, heads, kv_heads, kind, window):
+    """The same prompt with pages of 16 tokens (this kernel) and of 24 (queries and softmax weights in f32), from equal projections of a
+    one-layer model: in one pass, then a portion into the filled cache.
+
+    The kernels' sums differ by about 2^-17 of a value, one value in 2^9 rounds to the other BF16 number: of the 256 of a row none or one,
+    so that six rows in ten have no such value (of 512 with heads of 256, whose weights are sharper). Weights without their low parts are off by 2^-10, one value
+    in four rounds the other way, 2^-9 in the 2-norm; queries without theirs move scores, whose spread is sqrt(head_dim), by a
+    percent and the weights as much. Measured on such kernels, 2-norm of the median row's difference: 2.2e-3 and more, 4.4e-3
+    and more."""
+    cfg = small_cfg(hidden=256, layers=1, heads=heads, kv_heads=kv_heads, head_dim=head_dim, inter=128, vocab=700, window=window,
+                    layer_types=[kind])
+    gpu, _ = build_pair(cfg, "bf16", kv_bf16=True, norm_jitter=0.1, want_oracle=False)
+    tokens = syn.prompt_ids(700, 400, seed=head_dim)
+    out = []
+    for page in (16, 24):
+        table = gpu.new_cache_table(400, page_tokens=page, kv_dtype=pkg.BF16)
+        out.append(np.concatenate([gpu.extend(tokens[:270], table, want=list(range(270))), gpu.extend(tokens[270:], table, want=list(range(130)))]))
+    rows = np.linalg.norm(out[0] - out[1], axis=1) / np.linalg.norm(out[1], axis=1)
+    assert np.median(rows) <= 2.0 ** -10 and rows.max() <= 2.0 ** -7
