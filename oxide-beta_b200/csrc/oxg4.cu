@@ -1647,14 +1647,14 @@ static void launch_rows_norm(Launcher& ln, int rows, const RowsNormArgs& n) {
     else ln.go("norm", rows_norm_kernel<XT, kRowsThreads>, dim3(rows), dim3(kRowsThreads), 0, n);
 }
 
-// The rows one pass over the layers carries: the sequences of a decode step, or up to kPrefillRows prompt
-// tokens (a chunk), each with its token id, absolute position and, for a chunk, the sequence it belongs to.
+// The rows one pass over the layers carries: the sequences of a decode step, or up to chunk_rows prompt tokens
+// (a chunk), each with its token id, absolute position and, for a chunk, the sequence it belongs to.
 struct RowSet {
     int R = 0;
     const uint32_t* tok = nullptr;       // device [R]; kInactiveToken rows sit a decode step out
     const int32_t* pos = nullptr;        // device [R]
     const int32_t* seq = nullptr;        // device [R], or null: row r is sequence r
-    bool chunk = false;                  // prompt chunk: all K/V rows are appended before any token attends
+    bool chunk = false;                  // prompt chunk: attends through prompt_attn_kernel, or slice by slice
     // attention groups (consecutive tokens of one sequence), per layer kind (0 sliding, 1 global): a group holds
     // up to 8 / G tokens and G (query heads per KV head) may differ between the kinds
     const int32_t* grp_row0[2] = {nullptr, nullptr};
