@@ -119,6 +119,18 @@ DEVINL float gelu_mul(float x, float up) {
     return gelu * up;
 }
 
+template <typename WT> struct WTraits;
+template <> struct WTraits<float> {
+    static constexpr int EPL = 4;                     // elements per 16-byte load
+    static DEVINL float elem(const void* base, size_t idx) { return ((const float*)base)[idx]; }
+};
+template <> struct WTraits<uint16_t> {
+    static constexpr int EPL = 8;
+    static DEVINL float elem(const void* base, size_t idx) {
+        return __uint_as_float((uint32_t)((const uint16_t*)base)[idx] << 16);
+    }
+};
+
 DEVINL float sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }
 DEVINL float silu(float z) { return z / (1.0f + expf(-z)); }
 

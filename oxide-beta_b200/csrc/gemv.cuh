@@ -1,8 +1,9 @@
-// Weight-streaming projection kernel for small batches (1..4 activation rows per pass).
+// Projections of small batches: what a launch does, and the kernel for f32 weights (1..4 activation rows per pass; BF16 weights:
+// gemv_mma.cuh).
 //
 // One launch covers what the reference spreads over rms_norm[_bf16] + f32_to_bf16 + cublasGemmEx
 // (+ slice / gelu_mul / add / mul_bf16_scalar) launches — crates/oxide-torch-models/src/
-// gemma4_cuda/decode.rs:4-21,43-174 and tensor_ops.rs:61-157:
+// gemma4_cuda/decode.rs:4-21,43-174 and tensor_ops.rs:61-157 (x is rounded to BF16 where the weights are BF16):
 //   prologue  PRO_NORM : finish the previous block's residual update
 //                        h = (h_in + rmsnorm(previous projection, w_post)) * layer_scalar
 //                        (the projection itself is added where w_post is null; h = embedding row * sqrt(H)
@@ -24,25 +25,25 @@
 // Work split (EPI_STORE / EPI_GATEUP). Every CTA owns a contiguous block of output rows (for
 // EPI_GATEUP a block of (gate_i, up_i) pairs, streamed as 2*I virtual rows). The block is cut into
 // 512-byte chunks (one 16-byte load per lane) and the chunks are dealt out as equal contiguous runs
-// to the 16 warps, so all warps stream the same number of bytes whatever the matrix shape. A run
+// to the 32 warps, so all warps stream the same number of bytes whatever the matrix shape. A run
 // that ends inside a row leaves a partial sum; the pieces of a row meet in shared memory and are
 // added in a fixed order, which keeps the split-K reduction deterministic without atomics.
 //
-// The kernel is HBM-bound: bytes per launch = N * K * sizeof(weight).
+// The kernel is HBM-bound: bytes per launch = N * K * 4.
 #pragma once
 #include "common.cuh"
+#include "tc_gemm.cuh"
 
 namespace oxg4 {
 
 enum { PRO_PLAIN = 0, PRO_NORM = 1, PRO_SHIFT = 2, PRO_GNORM = 3 };
 enum { EPI_STORE = 0, EPI_GATEUP = 1, EPI_LOGITS = 2, EPI_STORE_GLU = 3 };
 
-constexpr int kGemvThreads = 512;
-constexpr int kGemvWarps = kGemvThreads / 32;
-constexpr int kSimtThreads = 1024;     // SIMT kernel: more warps, fewer registers, same bytes in flight per warp
+constexpr int kSimtThreads = 1024;
 constexpr int kSimtWarps = kSimtThreads / 32;
 constexpr int kSimtMaxJ = 6;         // PRO_NORM keeps hidden/1024 values per thread: hidden <= 6144
-constexpr int kGemvMaxJ = 11;        // PRO_NORM keeps hidden/512 values per thread: hidden <= 5632
+constexpr int kMaxHidden = 5632;       // widest residual row of a norm prologue
+constexpr int kSimtPrefetchKb = 128;   // of its own weight block a CTA pulls into L2 before the dependency wait
 
 struct GemvArgs {
     const void* W0;          // [N, K] row-major (EPI_GATEUP: gate)
@@ -50,10 +51,15 @@ struct GemvArgs {
     int N, K;                // rows (EPI_GATEUP: virtual rows = 2 * intermediate), columns
     int cpr;                 // 512-byte chunks per row
     int slots;               // most pieces a row is cut into inside one CTA
+    // gemv_mma.cuh: weight rows of a box, bytes and number of places of a warp's ring, boxes between two combines
+    int box_rows, place_bytes, places, pass_boxes;
+    int early;               // gemv_mma.cuh: the dependent launch may start before this kernel waits for its predecessor
+    int* err;                // device flag of failed waits
     int B;                   // activation rows in the step
     int bpp;                 // activation rows per pass (tensor-core kernel: grid.y = ceil(B / bpp))
     // PRO_PLAIN, PRO_GNORM
     const float* in;         // [B, K]; with input segments [nseg, B, K]
+    const uint16_t* in_x;    // gemv_mma.cuh, PRO_PLAIN: the input as BF16 in the operand's order (x_place), [B, K], instead of `in`
     // input segments: output rows [s * seg_rows, (s + 1) * seg_rows) multiply input s (nseg = 0: one input)
     int nseg, seg_rows;
     // PRO_SHIFT
@@ -81,12 +87,9 @@ struct GemvArgs {
     float embed_scale;
     float eps;
     int norm_n;              // values of a row that count for the PRO_NORM means (rows may end in zero padding); 0: K
-    // weights of later kernels to pull into L2 while this kernel runs (each CTA takes a slice)
-    const void* pf_ptr[2];
-    unsigned long long pf_bytes[2];
-    int pf_cap_kb;           // bytes of its own weight block a CTA prefetches into L2 before the dependency wait (KiB)
     unsigned long long* ts;  // optional timeline slots of this launch (4 entries) or null
     // epilogue
+    uint16_t* out_x;         // gemv_mma.cuh, GATEUP: the output as a later launch's in_x, instead of `out`
     float* out;              // STORE: [B, N]; GATEUP: [B, N/2]; STORE_GLU: [B, (glu_from + N) / 2]; LOGITS: [B, n_total] or null
     const uint8_t* seen;     // LOGITS: [B, n_total] repetition bitmap or null
     float penalty;
@@ -98,47 +101,33 @@ struct GemvArgs {
     float* best_scores;      // LOGITS: [B]
 };
 
-template <typename WT> struct WTraits;
-template <> struct WTraits<float> {
-    static constexpr int EPL = 4;                     // elements per 16-byte load
-    typedef float XT;
-    static DEVINL float elem(const void* base, size_t idx) { return ((const float*)base)[idx]; }
-    static DEVINL void store_x(XT* p, float v) { *p = v; }          // f32 mode: no rounding
-};
-template <> struct WTraits<uint16_t> {
-    static constexpr int EPL = 8;
-    typedef uint16_t XT;
-    static DEVINL float elem(const void* base, size_t idx) {
-        return __uint_as_float((uint32_t)((const uint16_t*)base)[idx] << 16);
+// acc[b] += dot(w (four weights), x (matching activations of row b))
+template <int NB>
+DEVINL void fma16(float (&acc)[NB], const uint4& w, const float* xs, int K, int k) {
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+        const float4 x = *reinterpret_cast<const float4*>(xs + (size_t)b * K + k);
+        float a = acc[b];
+        a = fmaf(__uint_as_float(w.x), x.x, a); a = fmaf(__uint_as_float(w.y), x.y, a);
+        a = fmaf(__uint_as_float(w.z), x.z, a); a = fmaf(__uint_as_float(w.w), x.w, a);
+        acc[b] = a;
     }
-    static DEVINL void store_x(XT* p, float v) { *p = (uint16_t)f32_to_bf16_bits(v); }
-};
+}
 
-// acc[b] += dot(w (16 bytes of weights), x (matching activations of row b))
-template <typename WT, int NB>
-DEVINL void fma16(float (&acc)[NB], const uint4& w, const typename WTraits<WT>::XT* xs, int K, int k) {
+DEVINL void store_x4(uint16_t* p, float4 v) {
+    *reinterpret_cast<uint2*>(p) = make_uint2(f32_to_bf16_bits(v.x) | (f32_to_bf16_bits(v.y) << 16),
+                                              f32_to_bf16_bits(v.z) | (f32_to_bf16_bits(v.w) << 16));
+}
+DEVINL void store_x4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+DEVINL float sum_sq4(float4 v) { return v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w; }
+// four values of an embedding row, BF16 or f32
+template <typename WT> DEVINL float4 embed4(const void* table, size_t at, float scale) {
     if constexpr (sizeof(WT) == 2) {
-        const float w0 = bf16lo(w.x), w1 = bf16hi(w.x), w2 = bf16lo(w.y), w3 = bf16hi(w.y);
-        const float w4 = bf16lo(w.z), w5 = bf16hi(w.z), w6 = bf16lo(w.w), w7 = bf16hi(w.w);
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            const uint4 x = *reinterpret_cast<const uint4*>(xs + (size_t)b * K + k);
-            float a = acc[b];
-            a = fmaf(w0, bf16lo(x.x), a); a = fmaf(w1, bf16hi(x.x), a);
-            a = fmaf(w2, bf16lo(x.y), a); a = fmaf(w3, bf16hi(x.y), a);
-            a = fmaf(w4, bf16lo(x.z), a); a = fmaf(w5, bf16hi(x.z), a);
-            a = fmaf(w6, bf16lo(x.w), a); a = fmaf(w7, bf16hi(x.w), a);
-            acc[b] = a;
-        }
+        const uint2 e = *reinterpret_cast<const uint2*>((const uint16_t*)table + at);
+        return make_float4(bf16lo(e.x) * scale, bf16hi(e.x) * scale, bf16lo(e.y) * scale, bf16hi(e.y) * scale);
     } else {
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            const float4 x = *reinterpret_cast<const float4*>(xs + (size_t)b * K + k);
-            float a = acc[b];
-            a = fmaf(__uint_as_float(w.x), x.x, a); a = fmaf(__uint_as_float(w.y), x.y, a);
-            a = fmaf(__uint_as_float(w.z), x.z, a); a = fmaf(__uint_as_float(w.w), x.w, a);
-            acc[b] = a;
-        }
+        const float4 e = *reinterpret_cast<const float4*>((const float*)table + at);
+        return make_float4(e.x * scale, e.y * scale, e.z * scale, e.w * scale);
     }
 }
 
@@ -149,19 +138,18 @@ DEVINL void block_range(int total, int parts, int idx, int& first, int& count) {
     count = base + (idx < rem ? 1 : 0);
 }
 
-template <typename WT, int NB, int PRO, int EPI>
+template <int NB, int PRO, int EPI>
 __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a) {
-    typedef WTraits<WT> T;
-    typedef typename T::XT XT;
-    constexpr int EPL = T::EPL;
+    typedef float WT;
+    constexpr int EPL = 4;                             // weights per 16-byte load
     constexpr int STEP = 32 * EPL;                     // elements per chunk
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int K = a.K;
     constexpr bool SEGS = (PRO == PRO_SHIFT || PRO == PRO_PLAIN) && EPI == EPI_STORE;  // may have several inputs
     constexpr bool STORES = EPI == EPI_STORE || EPI == EPI_STORE_GLU;
     const int nseg = SEGS ? max(1, a.nseg) : 1;
-    XT* xs = reinterpret_cast<XT*>(smem_raw);                                        // [nseg][NB][K]
-    float* red = reinterpret_cast<float*>(smem_raw + (size_t)nseg * NB * K * sizeof(XT));   // [NB*32]
+    float* xs = reinterpret_cast<float*>(smem_raw);                                        // [nseg][NB][K]
+    float* red = reinterpret_cast<float*>(smem_raw + (size_t)nseg * NB * K * sizeof(float));   // [NB*32]
     float* pieces = red + NB * 32;                     // [rows_cta][slots][NB] / Cand scratch
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int b0 = blockIdx.y * NB;
@@ -207,7 +195,7 @@ __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a)
         // this CTA's own block is contiguous in memory (two slabs for gate/up): bulk L2 prefetch
         if (tid < 8 && rows_cta > 0) {
             constexpr size_t PIECE = 32 * 1024;
-            const size_t cap = (size_t)a.pf_cap_kb * 1024;
+            const size_t cap = (size_t)kSimtPrefetchKb * 1024;
             if constexpr (EPI == EPI_GATEUP) {
                 const size_t slab = min((size_t)(rows_cta / 2) * row_bytes, cap / 2);
                 const char* g0 = (const char*)a.W0 + (size_t)(row_first / 2) * row_bytes;
@@ -219,22 +207,6 @@ __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a)
                 const char* s0 = (const char*)a.W0 + (size_t)row_first * row_bytes;
                 for (size_t off = (size_t)tid * PIECE; off < slab; off += 8 * PIECE)
                     prefetch_l2_bulk(s0 + off, min(PIECE, slab - off));
-            }
-        }
-    }
-    // slices of later kernels' weights: one 32 KiB bulk prefetch per thread at most
-    if (tid >= 32) {
-#pragma unroll
-        for (int which = 0; which < 2; ++which) {
-            const unsigned long long total = a.pf_bytes[which];
-            if (total) {
-                constexpr unsigned long long PIECE = 32 * 1024;
-                const unsigned long long npieces = (total + PIECE - 1) / PIECE;
-                for (unsigned long long pi = blockIdx.x + (unsigned long long)gridDim.x * (tid - 32); pi < npieces;
-                     pi += (unsigned long long)gridDim.x * (kSimtThreads - 32)) {
-                    const unsigned long long off = pi * PIECE;
-                    prefetch_l2_bulk((const char*)a.pf_ptr[which] + off, (size_t)min(PIECE, total - off));
-                }
             }
         }
     }
@@ -257,12 +229,12 @@ __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a)
         for (int sg = 0; sg < nseg; ++sg)
             for (int b = 0; b < nb; ++b)
                 for (int i = tid; i < K; i += kSimtThreads)
-                    T::store_x(xs + ((size_t)sg * NB + b) * K + i, a.in[((size_t)sg * a.B + b0 + b) * K + i]);
+                    xs[((size_t)sg * NB + b) * K + i] = a.in[((size_t)sg * a.B + b0 + b) * K + i];
     } else if constexpr (PRO == PRO_GNORM) {
         auto put = [&](int i, float v) {
             if (a.gn_w) v *= a.gn_w[i];
             if (a.gn_gate) v *= a.act == ACT_SILU ? silu(a.gn_gate[i]) : sigmoid(a.gn_gate[i]);
-            T::store_x(xs + i, v);
+            xs[i] = v;
         };
         if (a.gn_group == 0 || a.gn_group == a.gn_n) {
             float r = 1.0f;
@@ -283,11 +255,11 @@ __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a)
             }
         }
         if (a.gn_tail != nullptr) {
-            for (int i = a.gn_n + tid; i < a.gn_tail_at; i += kSimtThreads) T::store_x(xs + i, 0.0f);
+            for (int i = a.gn_n + tid; i < a.gn_tail_at; i += kSimtThreads) xs[i] = 0.0f;
             for (int i = a.gn_tail_at + tid; i < K; i += kSimtThreads)
-                T::store_x(xs + i, i < a.gn_tail_at + a.gn_tail_n ? a.gn_tail[i - a.gn_tail_at] : 0.0f);
+                xs[i] = i < a.gn_tail_at + a.gn_tail_n ? a.gn_tail[i - a.gn_tail_at] : 0.0f;
         } else {
-            for (int i = a.gn_n + tid; i < K; i += kSimtThreads) T::store_x(xs + i, 0.0f);
+            for (int i = a.gn_n + tid; i < K; i += kSimtThreads) xs[i] = 0.0f;
         }
     } else {
         const bool writer = (blockIdx.x == 0);
@@ -302,7 +274,7 @@ __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a)
 #pragma unroll
                 for (int j = 0; j < kSimtMaxJ; ++j) {
                     const int i = tid + j * kSimtThreads;
-                    hv[j] = (i < K) ? T::elem(a.embed, (size_t)tok * K + i) * a.embed_scale : 0.0f;
+                    hv[j] = (i < K) ? ((const float*)a.embed)[(size_t)tok * K + i] * a.embed_scale : 0.0f;
                 }
             } else if (a.raw == nullptr) {
                 // nothing pending: h_in already is the layer's input (layer-wise tracing)
@@ -351,13 +323,13 @@ __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a)
                     const float c = hv[j] * r2 * wnorm[j], p = first ? 0.0f : a.shift_state[i];
                     if (writer) a.x_f32[i] = c;
                     for (int sg = 0; sg < nseg; ++sg)
-                        T::store_x(xs + (size_t)sg * K + i, c + (p - c) * a.mu[(size_t)sg * K + i]);
+                        xs[(size_t)sg * K + i] = c + (p - c) * a.mu[(size_t)sg * K + i];
                 }
             } else {
 #pragma unroll
                 for (int j = 0; j < kSimtMaxJ; ++j) {
                     const int i = tid + j * kSimtThreads;
-                    if (i < K) T::store_x(xs + (size_t)b * K + i, hv[j] * r2 * wnorm[j]);
+                    if (i < K) xs[(size_t)b * K + i] = hv[j] * r2 * wnorm[j];
                 }
             }
         }
@@ -365,7 +337,7 @@ __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a)
     // rows of a partial batch chunk that do not exist read zeros
     for (int sg = 0; sg < nseg; ++sg)
         for (int b = nb; b < NB; ++b)
-            for (int i = tid; i < K; i += kSimtThreads) xs[((size_t)sg * NB + b) * K + i] = (XT)0;
+            for (int i = tid; i < K; i += kSimtThreads) xs[((size_t)sg * NB + b) * K + i] = 0.0f;
     __syncthreads();
     pdl_launch();
     stamp(a.ts, 2);
@@ -384,7 +356,7 @@ __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a)
             const int nfull = has_tail ? ncs - 1 : ncs;
             const WT* p = row_ptr(row_first + rl) + (size_t)cc * STEP + lane * EPL;
             int k = cc * STEP + lane * EPL;
-            const XT* xr = xs;                         // the input of this row's segment
+            const float* xr = xs;                         // the input of this row's segment
             if constexpr (SEGS) {
                 if (nseg > 1) xr = xs + (size_t)((row_first + rl) / a.seg_rows) * NB * K;
             }
@@ -397,7 +369,7 @@ __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a)
 #pragma unroll
                 for (int q = 0; q < 8; ++q) w[q] = ldg_stream16(p + q * STEP);
 #pragma unroll
-                for (int q = 0; q < 8; ++q) fma16<WT, NB>(acc, w[q], xr, K, k + q * STEP);
+                for (int q = 0; q < 8; ++q) fma16<NB>(acc, w[q], xr, K, k + q * STEP);
                 p += 8 * STEP;
                 k += 8 * STEP;
             }
@@ -406,15 +378,15 @@ __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a)
 #pragma unroll
                 for (int q = 0; q < 4; ++q) w[q] = ldg_stream16(p + q * STEP);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) fma16<WT, NB>(acc, w[q], xr, K, k + q * STEP);
+                for (int q = 0; q < 4; ++q) fma16<NB>(acc, w[q], xr, K, k + q * STEP);
                 p += 4 * STEP;
                 k += 4 * STEP;
                 j += 4;
             }
             if (j + 2 <= nfull) {
                 uint4 w0 = ldg_stream16(p), w1 = ldg_stream16(p + STEP);
-                fma16<WT, NB>(acc, w0, xr, K, k);
-                fma16<WT, NB>(acc, w1, xr, K, k + STEP);
+                fma16<NB>(acc, w0, xr, K, k);
+                fma16<NB>(acc, w1, xr, K, k + STEP);
                 p += 2 * STEP;
                 k += 2 * STEP;
                 j += 2;
@@ -422,7 +394,7 @@ __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a)
             for (; j < ncs; ++j) {
                 if (k < K) {
                     uint4 w0 = ldg_stream16(p);
-                    fma16<WT, NB>(acc, w0, xr, K, k);
+                    fma16<NB>(acc, w0, xr, K, k);
                 }
                 p += STEP;
                 k += STEP;
@@ -490,15 +462,15 @@ __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a)
                 }
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    fma16<WT, NB>(acc0, wa[j], xs, K, k + j * STEP);
-                    fma16<WT, NB>(acc1, wb[j], xs, K, k + j * STEP);
+                    fma16<NB>(acc0, wa[j], xs, K, k + j * STEP);
+                    fma16<NB>(acc1, wb[j], xs, K, k + j * STEP);
                 }
             }
             for (; k < K; k += STEP) {
                 uint4 wa = ldg_stream16(p0 + k);
                 uint4 wb = ldg_stream16(p1 + k);
-                fma16<WT, NB>(acc0, wa, xs, K, k);
-                fma16<WT, NB>(acc1, wb, xs, K, k);
+                fma16<NB>(acc0, wa, xs, K, k);
+                fma16<NB>(acc1, wb, xs, K, k);
             }
 #pragma unroll
             for (int b = 0; b < NB; ++b) { acc0[b] = warp_sum(acc0[b]); acc1[b] = warp_sum(acc1[b]); }

@@ -24,8 +24,8 @@ extern "C" int32_t oxg4_model_create_layered(const oxg4_layered_config* lc, int3
     if (lc->weight_dtype != OXG4_F32 && lc->weight_dtype != OXG4_BF16)
         return fail(OXG4_INVALID_ARGUMENT, "weight_dtype must be OXG4_F32 or OXG4_BF16");
     const int max_width = std::min(kSimtMaxJ * kSimtThreads, kRowsMaxJ * 4 * kRowsThreads);
-    if (lc->width > std::min(max_width, kGemvMaxJ * kGemvThreads))
-        return fail(OXG4_UNSUPPORTED, "width above %d is not supported", std::min(max_width, kGemvMaxJ * kGemvThreads));
+    if (lc->width > std::min(max_width, kMaxHidden))
+        return fail(OXG4_UNSUPPORTED, "width above %d is not supported", std::min(max_width, kMaxHidden));
     const int L = lc->num_layers;
     if (lc->block != OXG4_BLOCK_SANDWICH && lc->block != OXG4_BLOCK_PARALLEL) return fail(OXG4_INVALID_ARGUMENT, "unknown block %d", lc->block);
     if (lc->act != OXG4_ACT_GELU_TANH && lc->act != OXG4_ACT_SILU && lc->act != OXG4_ACT_RELU)
@@ -1028,12 +1028,15 @@ struct LayeredPass {
             a.W1 = x.gateup.w1;
             residual_args(a, x.norm2);
             a.act = m->ff_act;
+            uint16_t* gu_x = m->es == 2 && x.gateup.gp.N % 64 == 0 ? (uint16_t*)c->gu_part : nullptr;     // the down projection's operand
             a.out = c->gu_part;
+            a.out_x = gu_x;
             launch_gemv(ln, "gateup", c, R, a, x.gateup.gp, PRO_NORM, EPI_GATEUP);
             advance();
             GemvArgs d{};
             d.W0 = x.down.w;
             d.in = c->gu_part;
+            d.in_x = gu_x;
             d.out = c->down_part;
             launch_gemv(ln, "down", c, R, d, x.down.gp, PRO_PLAIN, EPI_STORE);
             pend(one(c->down_part, H), x.norm2b);

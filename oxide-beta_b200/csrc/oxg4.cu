@@ -77,7 +77,7 @@ struct Tensor {
 };
 
 struct GemvPlan {             // how a projection is cut into CTA row blocks and warp runs
-    int N = 0, K = 0, cpr = 0, grid = 0, slots = 1, rows_max = 0;
+    int N = 0, K = 0, cpr = 0, grid = 0, slots = 1, rows_max = 0;     // cpr, slots: f32 weights
 };
 
 // A projection of a layered model: W [N, K] row-major, rows and columns zero-padded. With nseg > 1 the rows form
@@ -150,10 +150,6 @@ struct oxg4_model {
     cudaStream_t stream = nullptr;
     int num_sms = 148;
     bool use_pdl = true;
-    int far_prefetch = 0;         // bit mask: which kernels pull a LATER kernel's weights into L2 (1 qkv, 2 attention, 4 gate/up, 8 down)
-    int far_prefetch_mb = 64;     // most MiB one kernel prefetches that way
-    int pf_cap_kb = 128;          // KiB of its own weight block a CTA pulls into L2 before the dependency wait
-    int pf_cap_gu_kb = -1, pf_cap_down_kb = -1;   // overrides for the gate/up and down projections (-1: pf_cap_kb)
     bool timeline = false;        // OXG4_TIMELINE: kernels stamp the global timer into the cache's buffer     // pull later kernels' weights into L2 during latency-bound kernels
     bool finalized = false;
     std::map<std::string, Tensor> tensors;
@@ -183,7 +179,7 @@ struct oxg4_model {
     GemvPlan p_ple_ctx, p_ple_gate, p_ple_proj;
     int es = 2;               // bytes per weight element
     GemvPlan p_gateup, p_down, p_lm;
-    int p_lm_simt_grid = 1;    // the SIMT logits kernel deals row pairs to warps across the grid
+    int p_lm_simt_grid = 1;    // the f32 logits kernel deals row pairs to warps across the grid
     long long launches = 0;
     int tp = 1, tp_rank = 0;
     void* comm = nullptr;         // ncclComm_t once oxg4_model_tp_init has run
@@ -313,11 +309,6 @@ extern "C" int32_t oxg4_model_create(const oxg4_config* c, int32_t device, oxg4_
     m->tp_rank = c->tp_rank;
     m->use_pdl = getenv("OXG4_DISABLE_PDL") == nullptr;
     m->timeline = getenv("OXG4_TIMELINE") != nullptr;
-    if (const char* e = getenv("OXG4_PREFETCH_KB")) m->pf_cap_kb = std::max(0, atoi(e));
-    if (const char* e = getenv("OXG4_PREFETCH_KB_GATEUP")) m->pf_cap_gu_kb = std::max(0, atoi(e));
-    if (const char* e = getenv("OXG4_PREFETCH_KB_DOWN")) m->pf_cap_down_kb = std::max(0, atoi(e));
-    if (const char* e = getenv("OXG4_FAR_PREFETCH")) m->far_prefetch = atoi(e);
-    if (const char* e = getenv("OXG4_FAR_PREFETCH_MB")) m->far_prefetch_mb = std::max(1, atoi(e));
     if (cudaSetDevice(device) != cudaSuccess) { delete m; return fail(OXG4_CUDA, "Gemma 4 CUDA error: cudaSetDevice"); }
     cudaDeviceProp prop;
     if (cudaGetDeviceProperties(&prop, device) == cudaSuccess) m->num_sms = prop.multiProcessorCount;
@@ -467,65 +458,48 @@ static int32_t allow_big_smem(F* kernel) {
     return OXG4_OK;
 }
 
-template <typename WT, int NB>
+// SIMT projections: two successive launches share an SM, so the split of its memory must not change between them
+template <typename F>
+static int32_t shared_sm_attrs(F* kernel) {
+    TRY(allow_big_smem(kernel));
+    CK(cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    return OXG4_OK;
+}
+template <int NB>
 static int32_t set_gemv_attrs() {
-#define SETA(PRO, EPI) TRY(allow_big_smem(gemv_kernel<WT, NB, PRO, EPI>))
+#define SETA(PRO, EPI) TRY((allow_big_smem(gemv_kernel<NB, PRO, EPI>)))
     SETA(PRO_NORM, EPI_STORE);
-    SETA(PRO_PLAIN, EPI_STORE);
     SETA(PRO_NORM, EPI_GATEUP);
     SETA(PRO_NORM, EPI_LOGITS);
-    if constexpr (sizeof(WT) == 4) SETA(PRO_PLAIN, EPI_STORE_GLU);
     if constexpr (NB == 1) {
         SETA(PRO_NORM, EPI_STORE_GLU);
         SETA(PRO_SHIFT, EPI_STORE);
         SETA(PRO_GNORM, EPI_STORE);
     }
+    SETA(PRO_PLAIN, EPI_STORE);
+    SETA(PRO_PLAIN, EPI_STORE_GLU);
 #undef SETA
     return OXG4_OK;
 }
 
-template <int MB>
-static int32_t set_mma_attrs() {
-    TRY(allow_big_smem(gemv_mma_kernel<MB, PRO_NORM, EPI_STORE>));
-    TRY(allow_big_smem(gemv_mma_kernel<MB, PRO_PLAIN, EPI_STORE>));
-    TRY(allow_big_smem(gemv_mma_kernel<MB, PRO_NORM, EPI_GATEUP>));
-    TRY(allow_big_smem(gemv_mma_kernel<MB, PRO_NORM, EPI_LOGITS>));
-    return OXG4_OK;
-}
-
-template <typename KT, int D>
+template <typename KT, int D, int G>
 static int32_t set_attn_attrs() {
-    TRY(allow_big_smem(attn_decode_kernel<KT, D, 1, false>));
-    TRY(allow_big_smem(attn_decode_kernel<KT, D, 2, false>));
-    TRY(allow_big_smem(attn_decode_kernel<KT, D, 4, false>));
-    TRY(allow_big_smem(attn_decode_kernel<KT, D, 8, false>));
-    TRY(allow_big_smem(attn_decode_kernel<KT, D, 1, true>));
-    TRY(allow_big_smem(attn_decode_kernel<KT, D, 2, true>));
-    TRY(allow_big_smem(attn_decode_kernel<KT, D, 4, true>));
-    TRY(allow_big_smem(attn_decode_kernel<KT, D, 8, true>));
-    TRY(allow_big_smem(attn_decode_kernel<KT, D, 1, true, true>));
-    TRY(allow_big_smem(attn_decode_kernel<KT, D, 2, true, true>));
-    TRY(allow_big_smem(attn_decode_kernel<KT, D, 4, true, true>));
-    TRY(allow_big_smem(attn_decode_kernel<KT, D, 8, true, true>));
-    CK(cudaFuncSetAttribute(attn_decode_kernel<KT, D, 1, true, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    CK(cudaFuncSetAttribute(attn_decode_kernel<KT, D, 2, true, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    CK(cudaFuncSetAttribute(attn_decode_kernel<KT, D, 4, true, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    CK(cudaFuncSetAttribute(attn_decode_kernel<KT, D, 8, true, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    CK(cudaFuncSetAttribute(attn_decode_kernel<KT, D, 1, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    CK(cudaFuncSetAttribute(attn_decode_kernel<KT, D, 2, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    CK(cudaFuncSetAttribute(attn_decode_kernel<KT, D, 4, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    CK(cudaFuncSetAttribute(attn_decode_kernel<KT, D, 8, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    TRY((allow_big_smem(attn_rows_kernel<KT, D, G>)));
+    TRY((shared_sm_attrs(attn_step_kernel<KT, D, G>)));
+    CK(cudaFuncSetAttribute(attn_step_kernel<KT, D, G>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     return OXG4_OK;
 }
 
 static int32_t finalize_layered(oxg4_model* m);
+template <typename F>
+static bool each_mma(const F& f);
 static int32_t set_projection_attrs(oxg4_model* m) {
     if (m->es == 2) {
-        TRY((set_gemv_attrs<uint16_t, 1>()));
-        TRY((set_mma_attrs<8>()));
-        TRY((set_mma_attrs<16>()));
+        int32_t status = OXG4_OK;
+        each_mma([&](int, int, int, int, auto* k) { return (status = shared_sm_attrs(k)) != OXG4_OK; });
+        TRY(status);
     } else {
-        TRY((set_gemv_attrs<float, 1>())); TRY((set_gemv_attrs<float, 2>())); TRY((set_gemv_attrs<float, 4>()));
+        TRY((set_gemv_attrs<1>())); TRY((set_gemv_attrs<2>())); TRY((set_gemv_attrs<4>()));
     }
     return allow_big_smem(topk_stage2_kernel);
 }
@@ -659,8 +633,11 @@ extern "C" int32_t oxg4_model_finalize(oxg4_model* m) {
     m->p_lm = make_plan(m->Vloc, H, m->es, m->num_sms, 1);
     m->p_lm_simt_grid = std::min(m->num_sms, std::max(1, (m->Vloc + 2 * kSimtWarps - 1) / (2 * kSimtWarps)));
     TRY(set_projection_attrs(m));
-    TRY((set_attn_attrs<uint16_t, 64>())); TRY((set_attn_attrs<uint16_t, 128>())); TRY((set_attn_attrs<uint16_t, 256>()));
-    TRY((set_attn_attrs<float, 64>())); TRY((set_attn_attrs<float, 128>())); TRY((set_attn_attrs<float, 256>()));
+#define SA1(D, G) TRY((set_attn_attrs<uint16_t, D, G>())); TRY((set_attn_attrs<float, D, G>()));
+#define SA(D) SA1(D, 1) SA1(D, 2) SA1(D, 4) SA1(D, 8)
+    SA(64) SA(128) SA(256)
+#undef SA
+#undef SA1
     CK(cudaDeviceSynchronize());
     m->finalized = true;
     return OXG4_OK;
@@ -1400,6 +1377,7 @@ struct Launcher {
     unsigned long long* ts_base = nullptr;
     int cluster_x = 0;            // > 0: launch the next kernel with thread-block clusters of this many CTAs along x
     bool coop = false;            // launch the next kernel cooperatively (all CTAs resident at once), without PDL
+    bool early = false;           // decode step: SIMT projections let their successor start before they wait (see gemv.cuh)
     int kernels = 0;
     unsigned long long* ts() const { return (ts_base && kernels < kMaxTimeline) ? ts_base + (size_t)kernels * 4 : nullptr; }
     int32_t status = OXG4_OK;
@@ -1515,36 +1493,75 @@ struct Launcher {
     }
 };
 
-template <typename WT>
-static void (*pick_gemv(int nb, int pro, int epi))(const GemvArgs) {
-#define PICK(NB)                                                                              \
-    if (pro == PRO_NORM && epi == EPI_STORE) return gemv_kernel<WT, NB, PRO_NORM, EPI_STORE>;       \
-    if (pro == PRO_PLAIN && epi == EPI_STORE) return gemv_kernel<WT, NB, PRO_PLAIN, EPI_STORE>;     \
-    if (pro == PRO_NORM && epi == EPI_GATEUP) return gemv_kernel<WT, NB, PRO_NORM, EPI_GATEUP>;     \
-    if (pro == PRO_NORM && epi == EPI_LOGITS) return gemv_kernel<WT, NB, PRO_NORM, EPI_LOGITS>;
-    if (nb == 1) {
-        PICK(1)
-        if (pro == PRO_NORM && epi == EPI_STORE_GLU) return gemv_kernel<WT, 1, PRO_NORM, EPI_STORE_GLU>;
-        if (pro == PRO_SHIFT && epi == EPI_STORE) return gemv_kernel<WT, 1, PRO_SHIFT, EPI_STORE>;
-        if (pro == PRO_GNORM && epi == EPI_STORE) return gemv_kernel<WT, 1, PRO_GNORM, EPI_STORE>;
+template <int NB>
+static void (*pick_gemv(int pro, int epi))(const GemvArgs) {
+#define PG(PRO, EPI) \
+    if (pro == PRO && epi == EPI) return gemv_kernel<NB, PRO, EPI>;
+    PG(PRO_NORM, EPI_STORE)
+    PG(PRO_PLAIN, EPI_STORE)
+    PG(PRO_NORM, EPI_GATEUP)
+    PG(PRO_NORM, EPI_LOGITS)
+    if constexpr (NB == 1) {
+        PG(PRO_NORM, EPI_STORE_GLU)
+        PG(PRO_SHIFT, EPI_STORE)
+        PG(PRO_GNORM, EPI_STORE)
     }
-    if constexpr (sizeof(WT) == 4) {      // BF16 weights with more than one row use the tensor-core kernel
-        if (pro == PRO_PLAIN && epi == EPI_STORE_GLU)
-            return nb == 1 ? gemv_kernel<WT, 1, PRO_PLAIN, EPI_STORE_GLU> : nb == 2 ? gemv_kernel<WT, 2, PRO_PLAIN, EPI_STORE_GLU> : gemv_kernel<WT, 4, PRO_PLAIN, EPI_STORE_GLU>;
-        if (nb == 2) { PICK(2) }
-        if (nb == 4) { PICK(4) }
-    }
-#undef PICK
+    PG(PRO_PLAIN, EPI_STORE_GLU)
+#undef PG
     return nullptr;
 }
 
-template <int MB>
-static void (*pick_mma(int pro, int epi))(const GemvArgs) {
-    if (pro == PRO_NORM && epi == EPI_STORE) return gemv_mma_kernel<MB, PRO_NORM, EPI_STORE>;
-    if (pro == PRO_PLAIN && epi == EPI_STORE) return gemv_mma_kernel<MB, PRO_PLAIN, EPI_STORE>;
-    if (pro == PRO_NORM && epi == EPI_GATEUP) return gemv_mma_kernel<MB, PRO_NORM, EPI_GATEUP>;
-    if (pro == PRO_NORM && epi == EPI_LOGITS) return gemv_mma_kernel<MB, PRO_NORM, EPI_LOGITS>;
-    return nullptr;
+// Calls f(kernel) for every instance of gemv_mma_kernel until one returns true: (most rows, prologue, epilogue, wide hidden row)
+template <typename F>
+static bool each_mma(const F& f) {
+#define EM(MB, PRO, EPI, MAXJ) \
+    if (f(MB, PRO, EPI, MAXJ, gemv_mma_kernel<MB, PRO, EPI, MAXJ>)) return true;
+#define EM2(PRO, EPI) EM(8, PRO, EPI, 3) EM(8, PRO, EPI, 6)
+    EM2(PRO_NORM, EPI_STORE) EM2(PRO_NORM, EPI_GATEUP) EM2(PRO_NORM, EPI_LOGITS) EM2(PRO_NORM, EPI_STORE_GLU) EM2(PRO_SHIFT, EPI_STORE)
+    EM(8, PRO_PLAIN, EPI_STORE, 3) EM(8, PRO_GNORM, EPI_STORE, 3)
+    EM(16, PRO_NORM, EPI_STORE, 6) EM(16, PRO_NORM, EPI_GATEUP, 6) EM(16, PRO_NORM, EPI_LOGITS, 6) EM(16, PRO_PLAIN, EPI_STORE, 6)
+#undef EM2
+#undef EM
+    return false;
+}
+typedef void (*MmaFn)(const CUtensorMap, const CUtensorMap, const GemvArgs);
+static MmaFn pick_mma(int rows, int pro, int epi, bool wide) {
+    MmaFn fn = nullptr;
+    each_mma([&](int mb, int p, int e, int maxj, MmaFn k) {
+        const bool norm = pro == PRO_NORM || pro == PRO_SHIFT;
+        if (rows > mb || p != pro || e != epi || (mb == 8 && norm && wide != (maxj == 6))) return false;
+        fn = k;
+        return true;
+    });
+    return fn;
+}
+
+// Shared memory of a small-batch projection. Two launches in a row share an SM, so that the second one's weights arrive while the
+// first still runs, but no SM may get two CTAs of one launch: the launch would run on some of the SMs only (seen as gate/up and down
+// launches of the ~4B model that took 11 us longer). A launch that may find SMs empty beside others that an attention or row kernel
+// fills, that is an output projection, therefore claims more than half an SM, and the others leave room for one of these.
+constexpr size_t kShareBoth = 110 * 1024, kShareAlone = 116 * 1024, kSmemMost = 226 * 1024;
+static size_t sm_share(int pro, int epi) { return epi == EPI_STORE && (pro == PRO_PLAIN || pro == PRO_GNORM) ? kShareAlone : kShareBoth; }
+
+// How `nb` rows stream a BF16 matrix through gemv_mma_kernel; false (and the bytes it would take) if they do not fit.
+static bool gemv_mma_ring(GemvArgs* a, const GemvPlan& p, int nb, int pro, int epi, size_t* smem) {
+    const size_t share = sm_share(pro, epi);
+    const bool two = epi == EPI_GATEUP;
+    const int nx = std::max(nb, a->nseg), rows = two ? p.rows_max / 2 : p.rows_max, most = two ? kGmBoxRows / 2 : kGmBoxRows;
+    int boxes = (rows + most - 1) / most;
+    a->box_rows = (rows + boxes - 1) / boxes;
+    if (epi == EPI_STORE_GLU) a->box_rows += a->box_rows & 1;        // a gate row and its up row are in one box
+    boxes = (rows + a->box_rows - 1) / a->box_rows;
+    a->place_bytes = (two ? 2 : 1) * ((a->box_rows * 128 + 1023) & ~1023);
+    a->pass_boxes = nx <= 2 ? 4 : nx <= 4 ? 2 : 1;
+    if (epi != EPI_LOGITS && boxes * nx <= 16) a->pass_boxes = boxes;
+    const size_t pieces = (size_t)(boxes > a->pass_boxes ? 2 : 1) * a->pass_boxes * kGmBoxRows * kGmWarps * nx * 4;
+    const size_t rest = 1024 + (size_t)nx * mma_x_stride(p.K) * 2 + pieces, one = (size_t)kGmWarps * a->place_bytes;
+    const size_t limit = rest + 2 * one <= share ? share : kSmemMost;
+    a->places = rest + one <= limit ? (int)std::min<size_t>(kGmMaxSlots, (limit - rest) / one) : 0;
+    *smem = rest + one * std::max(1, a->places);
+    if (share == kShareAlone) *smem = std::max(*smem, share);
+    return nx <= 16 && (a->places >= 2 || (nb == 1 && a->places == 1));
 }
 
 static void launch_gemv(Launcher& ln, const char* kind, oxg4_cache* c, int rows, GemvArgs a, const GemvPlan& p, int pro,
@@ -1553,37 +1570,42 @@ static void launch_gemv(Launcher& ln, const char* kind, oxg4_cache* c, int rows,
     const int B = rows;
     a.N = p.N;
     a.K = p.K;
-    a.cpr = p.cpr;
-    a.slots = p.slots;
     a.B = B;
     a.eps = m->cfg.rms_norm_eps;
     a.ts = ln.ts();
-    a.pf_cap_kb = m->pf_cap_kb;
-    if (epi == EPI_GATEUP && m->pf_cap_gu_kb >= 0) a.pf_cap_kb = m->pf_cap_gu_kb;
-    if (!strcmp(kind, "down") && m->pf_cap_down_kb >= 0) a.pf_cap_kb = m->pf_cap_down_kb;
+    a.early = ln.early ? 1 : 0;
+    a.err = c->tc_err;
     a.norm_n = p.K == m->H ? m->Hn : p.K;
-    if ((pro == PRO_NORM || pro == PRO_SHIFT) && p.K > std::min(kGemvMaxJ * kGemvThreads, kSimtMaxJ * kSimtThreads)) {
+    if ((pro == PRO_NORM || pro == PRO_SHIFT) && p.K > kMaxHidden) {
         ln.status = fail(OXG4_UNSUPPORTED, "hidden size above %d is not supported",
-                         std::min(kGemvMaxJ * kGemvThreads, kSimtMaxJ * kSimtThreads));
+                         kMaxHidden);
         return;
     }
-    const size_t limit = 226 * 1024;
-    if (m->es == 2 && B > 1) {
-        // tensor-core kernel: as many activation rows per pass as shared memory allows (at most 16)
-        auto need = [&](int nb) { return (((size_t)nb * mma_x_stride(p.K) * 2 + 15) & ~(size_t)15) + 128 + (size_t)2 * mma_rows_per_pass(nb > 8 ? 16 : 8) * kGemvWarps * nb * 4; };
+    if (m->es == 2) {
+        // as many activation rows per pass as shared memory allows (at most 16)
+        size_t smem = 0;
         int bpp = std::min(B, 16);
-        while (bpp > 1 && need(bpp) > limit) --bpp;
-        if (need(bpp) > limit) {
-            ln.status = fail(OXG4_UNSUPPORTED, "projection %s needs %zu bytes of shared memory", kind, need(bpp));
-            return;
+        while (!gemv_mma_ring(&a, p, bpp, pro, epi, &smem)) {
+            if (bpp == 1) {
+                ln.status = fail(OXG4_UNSUPPORTED, "projection %s needs %zu bytes of shared memory", kind, smem);
+                return;
+            }
+            --bpp;
         }
         a.bpp = bpp;
-        auto fn = bpp <= 8 ? pick_mma<8>(pro, epi) : pick_mma<16>(pro, epi);
-        dim3 grid(p.grid, (B + bpp - 1) / bpp, 1);
-        ln.go(kind, fn, grid, dim3(kGemvThreads), need(bpp), a);
+        CUtensorMap map0, map1;
+        const uint64_t rows = epi == EPI_GATEUP ? p.N / 2 : p.N;
+        ln.status = encode_bf16_2d(&map0, a.W0, rows, (uint64_t)p.K, (uint32_t)a.box_rows);
+        if (ln.status != OXG4_OK) return;
+        ln.status = encode_bf16_2d(&map1, epi == EPI_GATEUP ? a.W1 : a.W0, rows, (uint64_t)p.K, (uint32_t)a.box_rows);
+        if (ln.status != OXG4_OK) return;
+        ln.go(kind, pick_mma(bpp, pro, epi, p.K > 3 * 4 * kGmThreads), dim3(p.grid, (B + bpp - 1) / bpp, 1), dim3(kGmThreads), smem, map0, map1, a);
         return;
     }
-    // one activation row with BF16 weights, or f32 weights: SIMT kernel
+    // f32 weights: SIMT kernel
+    a.cpr = p.cpr;
+    a.slots = p.slots;
+    const size_t limit = 226 * 1024;
     int nb = B >= 3 ? 4 : B;
     auto simt_need = [&](int n) {
         return (size_t)std::max(1, a.nseg) * n * p.K * m->es + (size_t)n * 32 * 4 +
@@ -1596,17 +1618,20 @@ static void launch_gemv(Launcher& ln, const char* kind, oxg4_cache* c, int rows,
         ln.status = fail(OXG4_UNSUPPORTED, "projection %s needs %zu bytes of shared memory", kind, smem);
         return;
     }
-    auto fn = m->es == 2 ? pick_gemv<uint16_t>(nb, pro, epi) : pick_gemv<float>(nb, pro, epi);
+    auto fn = nb == 1 ? pick_gemv<1>(pro, epi) : nb == 2 ? pick_gemv<2>(pro, epi) : pick_gemv<4>(pro, epi);
     dim3 grid(epi == EPI_LOGITS ? m->p_lm_simt_grid : p.grid, (B + nb - 1) / nb, 1);
     ln.go(kind, fn, grid, dim3(kSimtThreads), smem, a);
 }
 
+// step: attn_step_kernel (a decode step), otherwise attn_rows_kernel; floats: shared memory of attn_step_kernel
+typedef void (*AttnFn)(const AttnArgs);
 template <typename KT>
-static void (*pick_attn(int D, int G, bool cl, bool deep))(const AttnArgs) {
+static AttnFn pick_attn(int D, int G, bool step, int NW, int splits, size_t* floats) {
 #define PA1(DD, GG)                                                                       \
     if (D == DD && G == GG) {                                                             \
-        if (cl && deep) return attn_decode_kernel<KT, DD, GG, true, true>;                \
-        return cl ? attn_decode_kernel<KT, DD, GG, true> : attn_decode_kernel<KT, DD, GG, false>; \
+        *floats = attn_step_floats<DD, GG>(NW, splits);                                   \
+        if (step) return attn_step_kernel<KT, DD, GG>;                                    \
+        return attn_rows_kernel<KT, DD, GG>;                                              \
     }
 #define PA(DD) PA1(DD, 1) PA1(DD, 2) PA1(DD, 4) PA1(DD, 8)
     PA(64) PA(128) PA(256)
@@ -1788,25 +1813,22 @@ static void launch_attention(Launcher& ln, oxg4_cache* c, const RowSet& rs, int 
     a.part = c->attn_part;
     a.ticket = c->attn_ticket;
     a.out = out;
-    if ((m->far_prefetch & 2) && !rs.chunk) {
-        // the attention kernel of a one-sequence step moves almost no bytes: HBM is idle, so it pulls the up
-        // projection's weights (or as much as the cap allows) into L2 for the kernel after next
-        a.pf_ptr = p.wup;
-        a.pf_bytes = std::min<unsigned long long>((unsigned long long)m->I * m->H * m->es, (unsigned long long)m->far_prefetch_mb << 20);
-    }
     a.ts = ln.ts();
     a.ts_mid = ln.ts_base ? ln.ts_base + 4 * (size_t)(kMaxTimeline - 1 - l) : nullptr;   // extra stamps, from the end of the buffer
-    const bool cl = !kv_in_cache;                // decode: cluster merge; K/V already in the cache: ticket merge
-    // few CTAs (one sequence): 16 warps each to cut latency; many CTAs: 4 warps each so that several
-    // fit on an SM (the kernel needs ~90 registers per thread)
-    const int aw = (a.n_splits * p.Nkv * R <= m->num_sms) ? kAttnWarps : 4;
-    // more K/V rows in flight per warp when latency is all that counts (with more than two query heads
-    // per kv head the extra rows would spill registers)
-    const bool deep = cl && aw == kAttnWarps && p.G <= 2;
-    auto fn = c->kv_dtype == OXG4_BF16 ? pick_attn<uint16_t>(D, p.G, cl, deep) : pick_attn<float>(D, p.G, cl, deep);
-    const size_t smem = sizeof(float) * (size_t)(p.G * D + 2 * D + 2 * aw * p.G + aw * p.G * D + p.G * (D + 2) + D);
-    ln.cluster_x = cl ? a.n_splits : 0;
-    ln.go("attn", fn, dim3(a.n_splits, p.Nkv, R), dim3(aw * 32), smem, a);
+    const bool step = !kv_in_cache;              // the kernel appends K and V itself
+    // few CTAs: one per SM at most, as many warps as the K/V rows in flight need; many CTAs: 4 warps each so that several fit on an SM
+    const bool few = a.n_splits * p.Nkv * R <= m->num_sms;
+    int unit = p.G;                              // query heads of a unit (attn_step_kernel)
+    while (unit > 1 && 2 * a.n_splits * p.Nkv * (p.G / unit) * R <= m->num_sms) unit /= 2;
+    const int NW = few ? (step ? kAttnStepThreads / 32 : kAttnWarps) : 4;
+    a.group = p.G;
+    a.early = ln.early ? 1 : 0;
+    size_t floats = 0;
+    auto fn = c->kv_dtype == OXG4_BF16 ? pick_attn<uint16_t>(p.D, step ? unit : p.G, step, NW, a.n_splits, &floats)
+                                       : pick_attn<float>(p.D, step ? unit : p.G, step, NW, a.n_splits, &floats);
+    if (!step) floats = (size_t)p.G * D + 2 * NW * p.G + NW * p.G * D + D;
+    ln.cluster_x = step ? a.n_splits : 0;
+    ln.go("attn", fn, dim3(a.n_splits, step ? p.Nkv * (p.G / unit) : p.Nkv, R), dim3(NW * 32), sizeof(float) * floats, a);
     ln.cluster_x = 0;
 }
 
@@ -1937,7 +1959,7 @@ static void ple_layer(oxg4_cache* c, Launcher& ln, const RowSet& rs, int l) {
 // All layers for the rows of `rs`. The last layer's residual update is returned still pending.
 static Pending run_layered(oxg4_cache* c, Launcher& ln, const RowSet& rs, bool use_tc, const TraceCtx* tr);
 
-static Pending run_layers(oxg4_cache* c, Launcher& ln, const RowSet& rs, bool use_tc, bool peer, bool last_layer_prefetch,
+static Pending run_layers(oxg4_cache* c, Launcher& ln, const RowSet& rs, bool use_tc, bool peer,
                           const TraceCtx* tr) {
     oxg4_model* m = c->m;
     if (m->layered) return run_layered(c, ln, rs, use_tc, tr);
@@ -1945,6 +1967,8 @@ static Pending run_layers(oxg4_cache* c, Launcher& ln, const RowSet& rs, bool us
     const int s_gu = rs.chunk ? c->ps_gu : c->s_gu;
     int s_down = rs.chunk ? c->ps_down : c->s_down;
     const bool wide = rs.chunk && c->wide && R > kWideRows;
+    // small batches of BF16 models: the feed-forward's values leave the gate/up launch as the down projection's operand
+    uint16_t* gu_x = m->es == 2 && m->I % 32 == 0 ? (uint16_t*)c->gu_raw : nullptr;
     if (m->P > 0) ple_prepare(c, ln, rs);
     for (int l = 0; l < L; ++l) {
         const LayerPlan& p = m->layers[l];
@@ -2059,10 +2083,6 @@ static Pending run_layers(oxg4_cache* c, Launcher& ln, const RowSet& rs, bool us
                 a.scalar = m->layers[l - 1].layer_scalar;
             }
             a.out = c->qkv_raw;
-            if (m->far_prefetch & 1) {
-                a.pf_ptr[0] = p.wo;
-                a.pf_bytes[0] = (unsigned long long)p.p_o.N * p.p_o.K * m->es;
-            }
             auto copy_trace = [&]() {
                 if (tr && ln.status == OXG4_OK &&
                     cudaMemcpyAsync(tr->trace_dev + (size_t)l * R * H, c->hB, sizeof(float) * R * H,
@@ -2101,26 +2121,15 @@ static Pending run_layers(oxg4_cache* c, Launcher& ln, const RowSet& rs, bool us
             a.scalar = 1.0f;
             a.w_norm = p.pre_ff_ln;
             a.out = c->gu_raw;
-            if (m->far_prefetch & 4) {
-                a.pf_ptr[0] = p.wdown;
-                a.pf_bytes[0] = std::min<unsigned long long>((unsigned long long)m->p_down.N * m->p_down.K * m->es, (unsigned long long)m->far_prefetch_mb << 20);
-            }
+            a.out_x = gu_x;
             launch_gemv(ln, "gateup", c, R, a, m->p_gateup, PRO_NORM, EPI_GATEUP);
         }
         {   // GeGLU + down projection (decode.rs:17-18)
             GemvArgs a{};
             a.W0 = p.wdown;
             a.in = c->gu_raw;
+            a.in_x = gu_x;
             a.out = c->down_raw;
-            if (m->far_prefetch & 8) {
-                if (l + 1 < L) {
-                    a.pf_ptr[0] = m->layers[l + 1].wqkv;
-                    a.pf_bytes[0] = (unsigned long long)m->layers[l + 1].p_qkv.N * m->layers[l + 1].p_qkv.K * m->es;
-                } else if (last_layer_prefetch) {
-                    a.pf_ptr[0] = (const char*)m->embed + (size_t)m->v0 * H * m->es;
-                    a.pf_bytes[0] = std::min<unsigned long long>((unsigned long long)m->Vloc * H * m->es, 64ull << 20);
-                }
-            }
             launch_gemv(ln, "down", c, R, a, m->p_down, PRO_PLAIN, EPI_STORE);
             ln.allreduce(c->down_raw, (size_t)R * H);
         }
@@ -2253,6 +2262,7 @@ static int32_t run_step(oxg4_cache* c, int kind, int top_k, float penalty, int* 
     oxg4_model* m = c->m;
     Launcher ln{m};
     ln.ts_base = c->ts_buf;
+    ln.early = true;
     const int B = c->B;
     // Sums over peer memory only in steps whose last exchange is consumed (the closing norm before the
     // LM head): a prompt-ingestion step skips that norm, so it takes the NCCL all-reduce instead and the
@@ -2273,7 +2283,7 @@ static int32_t run_step(oxg4_cache* c, int kind, int top_k, float penalty, int* 
     rs.run_n = c->dec_grp_n;
     rs.run_len.assign(B, 1);
     rs.max_visible = *std::max_element(c->max_seq.begin(), c->max_seq.end());
-    const Pending pd = run_layers(c, ln, rs, c->use_tc, peer, kind != STEP_PREFILL, tr);
+    const Pending pd = run_layers(c, ln, rs, c->use_tc, peer, tr);
     if (kind != STEP_PREFILL) {
         if (c->use_tc) closing_norm_tc(c, ln, B, pd);
         lm_head(c, ln, kind, top_k, penalty, c->use_tc, c->x_h, pd, tr);
@@ -2966,7 +2976,7 @@ static int32_t ingest(oxg4_model* m, oxg4_cache* c, const uint32_t* tokens, cons
             rs.grp_n[k] = dm.grp_n(k);
             rs.NG[k] = NG[k];
         }
-        const Pending pd = run_layers(c, ln, rs, use_tc, false, false, nullptr);
+        const Pending pd = run_layers(c, ln, rs, use_tc, false, nullptr);
         // keep what the LM head will need of every wanted row
         if (use_tc && !wanted.empty() && ln.status == OXG4_OK) closing_norm_tc(c, ln, R, pd);
         last.w_post = pd.w_post;
