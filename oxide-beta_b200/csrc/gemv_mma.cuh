@@ -45,19 +45,6 @@ DEVINL void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2,
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// L2 policy of data that is read once per step
-DEVINL uint64_t evict_first_policy() {
-    uint64_t p;
-    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-    return p;
-}
-// one box of a 2-D BF16 matrix, 128-byte swizzle, with an L2 policy
-DEVINL void tma_load_2d_hint(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar, uint64_t policy) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;"
-        ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar)), "l"(policy)
-        : "memory");
-}
 // Sum over the `warps` warps of a team (a power of two, teams of neighbouring warps) of the CTA; every thread calls it.
 DEVINL float team_sum(float v, int warps, float* red) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

@@ -1300,6 +1300,7 @@ static int32_t tc_gemm_launch(const void* w_dev, const void* w1_dev, const void*
     a.ld = ld;
     a.col0 = col0;
     a.err = err_dev;
+    a.once = a.TB == 1;
     const int units = ((N + kTcTileM - 1) / kTcTileM) * a.n_mats * S * a.TB;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(std::min(units, num_sms));
