@@ -1,5 +1,5 @@
 // Paged attention on the tensor cores with TMA-fed K/V tiles, for steps that carry many rows: decode
-// with eight or more sequences, and chunked prompt ingestion (several tokens of a sequence share the
+// with two or more sequences, and chunked prompt ingestion (several tokens of a sequence share the
 // K/V tiles they attend to). Replaces, together with qkv_post_kernel, what the reference runs as
 // rms_norm / rope_state / rms_norm_unit / cache_write_f32_state / gqa_decode_block_state for one row
 // (crates/oxide-torch-models/src/gemma4_cuda/decode.rs:99-157; kernel_module.rs:1790-1894) and as

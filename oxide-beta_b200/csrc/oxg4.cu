@@ -774,7 +774,7 @@ struct oxg4_cache {
     float* am_part = nullptr;
     int* am_pre = nullptr;                    // tile prefix of the attention groups, attention kernel -> merge kernel
     std::vector<CUtensorMap> kmap, vmap;
-    // tcgen05 path (decode with eight or more sequences, and every prompt chunk of a BF16 model): BF16
+    // tcgen05 path (decode with two or more sequences, and every prompt chunk of a BF16 model): BF16
     // activations, K-split partial outputs, error flag
     bool use_tc = false, tc_ok = false;
     int s_gu = 1, s_down = 1;                                  // K-splits for a decode step (B rows)
@@ -1010,7 +1010,10 @@ static int32_t cache_build(oxg4_cache* c) {
         TRY(allow_big_smem(prompt_attn_kernel<128>));
         TRY(allow_big_smem(prompt_attn_kernel<256>));
     }
-    c->use_tc = c->tc_ok && B >= (m->layered ? 2 : 8) && B <= kPrefillRows;       // up to 256 sequences: row blocks of 128 / 256 (UMMA N)
+    // From two sequences on the tcgen05 path (up to 256: row blocks of 128 / 256, UMMA N). Steps at 250 positions with it / with
+    // gemv_mma.cuh, us: ~4B model, 2 sequences 2330 / 2346, 4 2354 / 2704, 7 2440 / 2800; ~1B model, 4 1084 / 1341; ~12B widths, 4 1637 / 1660;
+    // ~27B widths, 4 1437 / 1560. Tensor-parallel ranks from eight on: theirs has not been timed below
+    c->use_tc = c->tc_ok && B >= (m->tp > 1 ? 8 : 2) && B <= kPrefillRows;
     c->ls_qkv.assign(L, 1);
     c->ls_o.assign(L, 1);
     c->lps_qkv.assign(L, 1);
@@ -1743,7 +1746,11 @@ static void launch_attention(Launcher& ln, oxg4_cache* c, const RowSet& rs, int 
     const int pps = p.sliding ? c->pps_slide : c->pps_full;
     const int32_t* cap = p.sliding ? c->cap_slide : c->cap_full;
     const int window = p.sliding ? m->cfg.sliding_window : 0x7fffffff;
-    const bool use_mma = c->mma_attn && (many_rows || rs.chunk);
+    // Few units over few positions: one launch of attn_step_kernel instead of three (a step of the ~4B model, 16 sequences at 100 / 450 /
+    // 1000 positions: 2490 / 2775 / 3105 us, with three 2635 / 2810 / 3015; eight at 450: 2500 / 2650; 32 at 250, twice the units: 3190 / 2955)
+    const int vis = p.sliding ? std::min(rs.max_visible, m->cfg.sliding_window) : rs.max_visible;
+    const bool few_units = !rs.chunk && !p.shared && R * p.Nkv <= 64 && 4.0 * R * vis * p.Nkv * D <= 40e6;
+    const bool use_mma = c->mma_attn && (many_rows || rs.chunk) && !few_units;
     // K and V of the rows are in the cache before the attention kernel starts: rows of a prompt chunk (appended by
     // qkv_post_kernel), and every row of a KV-shared layer (its source layer appended them earlier in the step)
     const bool kv_in_cache = rs.chunk || p.shared;
