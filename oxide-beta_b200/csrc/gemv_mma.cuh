@@ -163,6 +163,7 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant_
     stamp(a.ts, 0);
     pdl_wait();
     stamp(a.ts, 1);
+    const int dead = *(const volatile int*)a.err;      // an earlier launch failed: this one uses none of its data (looked at behind the prologue)
 
     // ---- prologue: x[nx][K] (BF16) in shared memory ----
     if constexpr (PRO == PRO_PLAIN) {
@@ -402,7 +403,8 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant_
     best[0].i = best[MB / 8 - 1].i = 0xffffffffu;
     int slot = 0, pass = 0;
     uint32_t phase = 0;
-    bool ok = true;                                    // a failed wait: the warp goes on without data, so that it meets the others at every barrier
+    // a failed wait, here or in a launch before: the warp goes on without data, so that it meets the others at every barrier
+    bool ok = !__any_sync(0xffffffffu, dead != 0);
     for (int p0 = 0; p0 < n_boxes; p0 += PB, ++pass) {
         float* pc = pieces + (size_t)(pass & 1) * PB * kGmBoxRows * kGmWarps * nx;
         const int r0 = p0 * R, rows_here = min(PB * R, rows_cta - r0);

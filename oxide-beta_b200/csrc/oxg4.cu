@@ -2381,15 +2381,16 @@ static void advance_host(oxg4_cache* c, const uint32_t* tokens, int steps = 1) {
         if (tokens[b] != kInactiveToken) c->pos_host[b] += steps;
 }
 
-// the tcgen05 kernels raise a device flag instead of hanging when one of their bounded waits runs out
+// Kernels with bounded waits raise a device flag instead of hanging when one of them runs out: every projection of a BF16 model and
+// the attention over BF16 pages
 static int32_t check_tc(oxg4_cache* c) {
-    if (!c->tc_ok && !c->mma_attn) return OXG4_OK;
+    if (c->m->es != 2 && !c->mma_attn) return OXG4_OK;
     int err = 0;
     CK(cudaMemcpy(&err, c->tc_err, sizeof err, cudaMemcpyDeviceToHost));
     if (err) {
         cudaMemset(c->tc_err, 0, sizeof err);
         return fail(OXG4_TIMEOUT, "%s: a bounded barrier wait ran out (code %d)",
-                    err >= 10 ? "tensor-core attention" : "tcgen05 projection", err);
+                    err >= 10 ? "tensor-core attention" : err == 7 ? "small-batch projection" : "tcgen05 projection", err);
     }
     if (c->peer_ready) {
         CK(cudaMemcpy(&err, c->px_local + 4, sizeof err, cudaMemcpyDeviceToHost));
@@ -2619,6 +2620,7 @@ extern "C" int32_t oxg4_decode_trace(oxg4_model* m, oxg4_cache* c, const uint32_
     int n = 0;
     if (s == OXG4_OK) s = run_step(c, STEP_LOGITS, 1, 1.0f, &n, &tr);      // eager launches, no graph
     if (s == OXG4_OK && cudaStreamSynchronize(m->stream) != cudaSuccess) s = fail(OXG4_CUDA, "Gemma 4 CUDA error: trace step failed");
+    if (s == OXG4_OK) s = check_tc(c);
     if (s == OXG4_OK) {
         m->launches += n;
         cudaMemcpy2D(trace, sizeof(float) * m->Hn, d_trace, sizeof(float) * m->H, sizeof(float) * m->Hn, (size_t)c->B * (L + 1),
@@ -2670,7 +2672,7 @@ static int32_t smoke_finish(oxg4_cache* c, Launcher& ln, const float* dev, float
     m->launches += ln.kernels;
     CK(cudaMemcpyAsync(host, dev, sizeof(float) * n, cudaMemcpyDeviceToHost, m->stream));
     CK(cudaStreamSynchronize(m->stream));
-    return OXG4_OK;
+    return check_tc(c);
 }
 
 // input norm + fused QKV projection of `layer` on the embedding of the staged token: layer input -> c->hB, qkv -> c->qkv_raw

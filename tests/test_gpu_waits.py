@@ -67,3 +67,35 @@ def test_calls_behind_a_failure_report_it_and_the_next_ones_work(model):
         table.reset()
         for again, want in zip(calls[:i + 1], clean):
             assert np.array_equal(again(table), want)
+
+
+@pytest.mark.parametrize("kv", [pkg.F32, pkg.BF16])
+@pytest.mark.parametrize("batch,ple", [(1, False), (1, True), (3, True), (9, True)])
+def test_small_batch_projections_behind_a_failure_report_it(model, batch, ple, kv):
+    """The same for calls whose BF16 projections are all of the small-batch kind, with and without tensor-core attention beside them: one
+    sequence, and a model with per-layer embeddings with one, a few and more than eight rows."""
+    N = pkg._native
+    if ple:
+        model = build_pair(syn.e_tiny_cfg(), "bf16", kv_bf16=True, want_oracle=False)[0]
+    tokens = syn.prompt_ids(500, batch * 12, seed=4)
+    calls = [lambda table: model.prefill_prompt(tokens, table, lens=[12] * batch),
+             lambda table: model.decode_token(tokens[:batch], table),
+             lambda table: model.decode_greedy(tokens[:batch], table, 3)[0],
+             lambda table: model.decode_trace(tokens[:batch], table)[0]]
+    if batch == 1:
+        calls.append(lambda table: model.cached_attention_smoke(int(tokens[0]), 0, table))
+    new = lambda: model.new_cache_table([32] * batch, batch=batch, page_tokens=16, kv_dtype=kv)  # noqa: E731
+    table = new()
+    clean = [call(table) for call in calls]
+    for i, call in enumerate(calls):
+        table = new()
+        for earlier in calls[:i]:
+            earlier(table)
+        N.check(N.lib().oxg4_debug_set_status(model._h, table._h, 7))
+        start = time.monotonic()
+        with pytest.raises(N.Oxg4Error, match="TIMEOUT"):
+            call(table)
+        assert time.monotonic() - start < 1.0
+        table.reset()
+        for again, want in zip(calls[:i + 1], clean):
+            assert np.array_equal(again(table), want)
