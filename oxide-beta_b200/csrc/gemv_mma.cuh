@@ -1,4 +1,4 @@
-// Weight-streaming projection kernel for BF16 weights, 1..16 activation rows per pass.
+// Weight-streaming projection kernel for BF16 weights, 1..8 activation rows (more: gemv_rows.cuh).
 //
 // Prologues and epilogues are those of gemv.cuh (see there for the reference launches it replaces). The weights go through shared
 // memory and meet the activations on the tensor cores, so that a CTA can use them up several times faster than HBM delivers
@@ -29,7 +29,7 @@ constexpr int kGmWarps = 8;
 constexpr int kGmThreads = kGmWarps * 32;
 constexpr int kGmMaxSlots = 6;
 constexpr int kGmBoxRows = 32;                         // weight rows of a box, at most (with gate and up: 16 of each)
-constexpr int kGmMaxHidden = 6144;                     // norms of one row: six groups of four values per thread
+constexpr int kGmMaxRows = 8;                          // activation rows of a launch's pass
 
 // Row stride (elements) of the activations in shared memory: whole units of 32, rows 64 bytes apart modulo 128, so that the
 // eight lanes of an LDS.128 phase (two batch rows x four column groups) hit eight different 16-byte bank groups.
@@ -69,15 +69,14 @@ DEVINL void x_put4(uint16_t* row, int c, float4 v) {   // c a multiple of 4
 }
 DEVINL void x_put(uint16_t* row, int c, float v) { row[x_place(c) + (c & 1)] = (uint16_t)f32_to_bf16_bits(v); }
 
-// MB = 8: up to 8 rows of activations per pass; MB = 16: up to 16.
 // MAXJ: groups of four values of a residual row per thread in the norms of one row (hidden <= MAXJ * 1024); with 3 the norm
 // weights wait in registers too
-template <int MB, int PRO, int EPI, int MAXJ>
+template <int PRO, int EPI, int MAXJ>
 __global__ void __launch_bounds__(kGmThreads, 2)
 gemv_mma_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap map1, const GemvArgs a) {
     constexpr bool NORM = PRO == PRO_NORM || PRO == PRO_SHIFT;
     constexpr bool TWO = EPI == EPI_GATEUP;            // gate and up rows come from two matrices
-    constexpr bool SEGS = (PRO == PRO_SHIFT || PRO == PRO_PLAIN) && EPI == EPI_STORE && MB == 8;   // may have several inputs
+    constexpr bool SEGS = (PRO == PRO_SHIFT || PRO == PRO_PLAIN) && EPI == EPI_STORE;   // may have several inputs
     constexpr bool AHEAD = NORM && MAXJ <= 3;
     constexpr int GROUPS = kGmBoxRows / 8;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -119,13 +118,18 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant_
     while (cb >= ncb) { cb -= ncb; ++rb; }
     unsigned char* ring = rings + (size_t)warp * NS * SB;
     uint64_t* bar = bars[warp];
+    const bool once = gridDim.y == 1;                  // rows that take several passes read the weights again
     const uint64_t policy = evict_first_policy();
+    auto load_box = [&](unsigned char* dst, const CUtensorMap* map, int x, int y, uint64_t* b) {
+        if (once) tma_load_2d_hint(dst, map, x, y, b, policy);
+        else tma_load_2d(dst, map, x, y, b);
+    };
     const uint32_t box_bytes = (uint32_t)(R * 128 * (TWO ? 2 : 1));
     int irb = rb, icb = cb;                            // next item to request (lane 0)
     auto request = [&](int slot) {
         mbar_expect_tx(&bar[slot], box_bytes);
-        tma_load_2d_hint(ring + (size_t)slot * SB, &map0, icb * 64, row_first + irb * R, &bar[slot], policy);
-        if constexpr (TWO) tma_load_2d_hint(ring + (size_t)slot * SB + SB / 2, &map1, icb * 64, row_first + irb * R, &bar[slot], policy);
+        load_box(ring + (size_t)slot * SB, &map0, icb * 64, row_first + irb * R, &bar[slot]);
+        if constexpr (TWO) load_box(ring + (size_t)slot * SB + SB / 2, &map1, icb * 64, row_first + irb * R, &bar[slot]);
         next_item(irb, icb);
     };
     if (tid == 0) failed = 0;
@@ -397,10 +401,8 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant_
     const uint32_t frag = (uint32_t)((lane & 7) * 128);                // ldmatrix: row lane % 8, 16-byte chunk 4 * unit + lane / 8, swizzled
     const int c16 = lane >> 3, x7 = lane & 7;
     const uint16_t* xa = xs + (size_t)g8 * XS + t4 * 8;
-    const bool has_a = g8 < nx, has_b = MB == 16 && g8 + 8 < nx;
-    Cand best[MB / 8];
-    best[0].s = best[MB / 8 - 1].s = -INFINITY;
-    best[0].i = best[MB / 8 - 1].i = 0xffffffffu;
+    const bool has_a = g8 < nx;
+    Cand best{-INFINITY, 0xffffffffu};
     int slot = 0, pass = 0;
     uint32_t phase = 0;
     // a failed wait, here or in a launch before: the warp goes on without data, so that it meets the others at every barrier
@@ -419,13 +421,12 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant_
                     break;
                 }
                 const uint32_t base = smem_u32(ring + (size_t)slot * SB) + frag;
-                uint4 x[2], y[2];
+                uint4 x[2];
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {          // the row of the A operand ends with whole units: a unit past K is not read
-                    x[u] = y[u] = make_uint4(0u, 0u, 0u, 0u);
+                    x[u] = make_uint4(0u, 0u, 0u, 0u);
                     const int at = (cb * 2 + u) * 32;
                     if (has_a && at < K) x[u] = *reinterpret_cast<const uint4*>(xa + at);
-                    if (MB == 16 && has_b && at < K) y[u] = *reinterpret_cast<const uint4*>(xa + (size_t)8 * XS + at);
                 }
                 uint32_t w[2][GROUPS][4];
 #pragma unroll
@@ -439,24 +440,23 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant_
                 for (int u = 0; u < 2; ++u)
 #pragma unroll
                     for (int g = 0; g < GROUPS; ++g)
-                        if (g_of(g) < R) mma_bf16_16816(acc[g], x[u].x, y[u].x, x[u].y, y[u].y, w[u][g][0], w[u][g][1]);
+                        if (g_of(g) < R) mma_bf16_16816(acc[g], x[u].x, 0u, x[u].y, 0u, w[u][g][0], w[u][g][1]);
                 __syncwarp();                          // all lanes have read the slot (every ldmatrix has delivered)
                 if (lane == 0 && irb < n_boxes) request(slot);
 #pragma unroll
                 for (int u = 0; u < 2; ++u)
 #pragma unroll
                     for (int g = 0; g < GROUPS; ++g)
-                        if (g_of(g) < R) mma_bf16_16816(acc[g], x[u].z, y[u].z, x[u].w, y[u].w, w[u][g][2], w[u][g][3]);
+                        if (g_of(g) < R) mma_bf16_16816(acc[g], x[u].z, 0u, x[u].w, 0u, w[u][g][2], w[u][g][3]);
                 next_item(rb, cb);
                 if (++slot == NS) { slot = 0; phase ^= 1; }
             }
-            // lane (g8, t4) holds batch rows g8 and g8 + 8 of weight rows 2 * t4 and 2 * t4 + 1 of every group
+            // lane (g8, t4) holds batch row g8 of weight rows 2 * t4 and 2 * t4 + 1 of every group
 #pragma unroll
             for (int g = 0; g < GROUPS; ++g) {
                 float* q0 = pc + ((size_t)((box - p0) * kGmBoxRows + g * 8 + 2 * t4) * kGmWarps + warp) * nx;
                 float* q1 = q0 + (size_t)kGmWarps * nx;
                 if (has_a) { q0[g8] = acc[g][0]; q1[g8] = acc[g][1]; }
-                if (has_b) { q0[g8 + 8] = acc[g][2]; q1[g8 + 8] = acc[g][3]; }
             }
         }
         __syncthreads();
@@ -491,21 +491,17 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant_
                 else a.out[(size_t)(b0 + b) * n + row] = v;
             }
         } else {
-            // thread -> (row tid % RP, batch rows tid / RP and, with 16 of them, the next as many); RP a power of two
-            const int RP = PB * kGmBoxRows, BH = kGmThreads / RP, rl = tid & (RP - 1);
-#pragma unroll
-            for (int h = 0; h < MB / 8; ++h) {
-                const int b = tid / RP + BH * h;
-                if (rl < rows_here && b < nb) {
-                    const float v = total(rl, b);
-                    const int vid = a.row_offset + row_first + r0 + rl;
-                    const size_t gb = (size_t)(b0 + b) * a.n_total;
-                    if (a.out) a.out[gb + vid] = v;
-                    float sc = v;      // kernel_module.rs:2008-2016: penalty on seen tokens, NaN skipped, strict '>'
-                    if (a.seen && a.penalty > 1.0f && a.seen[gb + vid]) sc = sc >= 0.0f ? sc / a.penalty : sc * a.penalty;
-                    const Cand cnd{sc, (uint32_t)vid};
-                    if (sc == sc && sc > -INFINITY && cand_better(cnd, best[h])) best[h] = cnd;
-                }
+            // thread -> (row tid % RP, batch row tid / RP); RP a power of two, at most 256 / nb
+            const int RP = PB * kGmBoxRows, rl = tid & (RP - 1), b = tid / RP;
+            if (rl < rows_here && b < nb) {
+                const float v = total(rl, b);
+                const int vid = a.row_offset + row_first + r0 + rl;
+                const size_t gb = (size_t)(b0 + b) * a.n_total;
+                if (a.out) a.out[gb + vid] = v;
+                float sc = v;          // kernel_module.rs:2008-2016: penalty on seen tokens, NaN skipped, strict '>'
+                if (a.seen && a.penalty > 1.0f && a.seen[gb + vid]) sc = sc >= 0.0f ? sc / a.penalty : sc * a.penalty;
+                const Cand cnd{sc, (uint32_t)vid};
+                if (sc == sc && sc > -INFINITY && cand_better(cnd, best)) best = cnd;
             }
         }
     }
@@ -513,12 +509,8 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant_
     if constexpr (EPI == EPI_LOGITS) {
         __syncthreads();
         Cand* wc = reinterpret_cast<Cand*>(pieces);        // [nb][RP]
-        const int RP = PB * kGmBoxRows, BH = kGmThreads / RP;
-#pragma unroll
-        for (int h = 0; h < MB / 8; ++h) {
-            const int b = tid / RP + BH * h;
-            if (b < nb) wc[b * RP + (tid & (RP - 1))] = best[h];
-        }
+        const int RP = PB * kGmBoxRows;
+        if (tid / RP < nb) wc[tid] = best;
         __syncthreads();
         for (int b = warp; b < nb; b += kGmWarps) {
             Cand c = wc[b * RP + lane];

@@ -23,6 +23,7 @@
 #include "attention_mma.cuh"
 #include "gemv.cuh"
 #include "gemv_mma.cuh"
+#include "gemv_rows.cuh"
 #include "sampling.cuh"
 #include "batch_ops.cuh"
 #include "tc_gemm.cuh"
@@ -493,11 +494,21 @@ static int32_t set_attn_attrs() {
 static int32_t finalize_layered(oxg4_model* m);
 template <typename F>
 static bool each_mma(const F& f);
+template <int MB>
+static int32_t set_rows_attrs() {
+    TRY((allow_big_smem(gemv_rows_kernel<MB, PRO_NORM, EPI_STORE>)));
+    TRY((allow_big_smem(gemv_rows_kernel<MB, PRO_PLAIN, EPI_STORE>)));
+    TRY((allow_big_smem(gemv_rows_kernel<MB, PRO_NORM, EPI_GATEUP>)));
+    TRY((allow_big_smem(gemv_rows_kernel<MB, PRO_NORM, EPI_LOGITS>)));
+    return OXG4_OK;
+}
 static int32_t set_projection_attrs(oxg4_model* m) {
     if (m->es == 2) {
         int32_t status = OXG4_OK;
-        each_mma([&](int, int, int, int, auto* k) { return (status = shared_sm_attrs(k)) != OXG4_OK; });
+        each_mma([&](int, int, int, auto* k) { return (status = shared_sm_attrs(k)) != OXG4_OK; });
         TRY(status);
+        TRY(set_rows_attrs<8>());
+        TRY(set_rows_attrs<16>());
     } else {
         TRY((set_gemv_attrs<1>())); TRY((set_gemv_attrs<2>())); TRY((set_gemv_attrs<4>()));
     }
@@ -1515,29 +1526,38 @@ static void (*pick_gemv(int pro, int epi))(const GemvArgs) {
     return nullptr;
 }
 
-// Calls f(kernel) for every instance of gemv_mma_kernel until one returns true: (most rows, prologue, epilogue, wide hidden row)
+// Calls f(kernel) for every instance of gemv_mma_kernel until one returns true: (prologue, epilogue, groups of a hidden row)
 template <typename F>
 static bool each_mma(const F& f) {
-#define EM(MB, PRO, EPI, MAXJ) \
-    if (f(MB, PRO, EPI, MAXJ, gemv_mma_kernel<MB, PRO, EPI, MAXJ>)) return true;
-#define EM2(PRO, EPI) EM(8, PRO, EPI, 3) EM(8, PRO, EPI, 6)
+#define EM(PRO, EPI, MAXJ) \
+    if (f(PRO, EPI, MAXJ, gemv_mma_kernel<PRO, EPI, MAXJ>)) return true;
+#define EM2(PRO, EPI) EM(PRO, EPI, 3) EM(PRO, EPI, 6)
     EM2(PRO_NORM, EPI_STORE) EM2(PRO_NORM, EPI_GATEUP) EM2(PRO_NORM, EPI_LOGITS) EM2(PRO_NORM, EPI_STORE_GLU) EM2(PRO_SHIFT, EPI_STORE)
-    EM(8, PRO_PLAIN, EPI_STORE, 3) EM(8, PRO_GNORM, EPI_STORE, 3)
-    EM(16, PRO_NORM, EPI_STORE, 6) EM(16, PRO_NORM, EPI_GATEUP, 6) EM(16, PRO_NORM, EPI_LOGITS, 6) EM(16, PRO_PLAIN, EPI_STORE, 6)
+    EM(PRO_PLAIN, EPI_STORE, 3) EM(PRO_GNORM, EPI_STORE, 3)
 #undef EM2
 #undef EM
     return false;
 }
 typedef void (*MmaFn)(const CUtensorMap, const CUtensorMap, const GemvArgs);
-static MmaFn pick_mma(int rows, int pro, int epi, bool wide) {
+static MmaFn pick_mma(int pro, int epi, bool wide) {
     MmaFn fn = nullptr;
-    each_mma([&](int mb, int p, int e, int maxj, MmaFn k) {
+    each_mma([&](int p, int e, int maxj, MmaFn k) {
         const bool norm = pro == PRO_NORM || pro == PRO_SHIFT;
-        if (rows > mb || p != pro || e != epi || (mb == 8 && norm && wide != (maxj == 6))) return false;
+        if (p != pro || e != epi || (norm && wide != (maxj == 6))) return false;
         fn = k;
         return true;
     });
     return fn;
+}
+
+// The same for gemv_rows_kernel
+template <int MB>
+static void (*pick_rows(int pro, int epi))(const GemvArgs) {
+    if (pro == PRO_NORM && epi == EPI_STORE) return gemv_rows_kernel<MB, PRO_NORM, EPI_STORE>;
+    if (pro == PRO_PLAIN && epi == EPI_STORE) return gemv_rows_kernel<MB, PRO_PLAIN, EPI_STORE>;
+    if (pro == PRO_NORM && epi == EPI_GATEUP) return gemv_rows_kernel<MB, PRO_NORM, EPI_GATEUP>;
+    if (pro == PRO_NORM && epi == EPI_LOGITS) return gemv_rows_kernel<MB, PRO_NORM, EPI_LOGITS>;
+    return nullptr;
 }
 
 // Shared memory of a small-batch projection. Two launches in a row share an SM, so that the second one's weights arrive while the
@@ -1565,7 +1585,7 @@ static bool gemv_mma_ring(GemvArgs* a, const GemvPlan& p, int nb, int pro, int e
     a->places = rest + one <= limit ? (int)std::min<size_t>(kGmMaxSlots, (limit - rest) / one) : 0;
     *smem = rest + one * std::max(1, a->places);
     if (share == kShareAlone) *smem = std::max(*smem, share);
-    return nx <= 16 && (a->places >= 2 || (nb == 1 && a->places == 1));
+    return nx <= kGmMaxRows && (a->places >= 2 || (nb == 1 && a->places == 1));     // the A operand's half that is kept has eight rows
 }
 
 static void launch_gemv(Launcher& ln, const char* kind, oxg4_cache* c, int rows, GemvArgs a, const GemvPlan& p, int pro,
@@ -1585,10 +1605,23 @@ static void launch_gemv(Launcher& ln, const char* kind, oxg4_cache* c, int rows,
                          kMaxHidden);
         return;
     }
-    if (m->es == 2) {
+    if (m->es == 2 && B > kGmMaxRows) {
         // as many activation rows per pass as shared memory allows (at most 16)
-        size_t smem = 0;
+        auto need = [&](int nb) { return (((size_t)nb * mma_x_stride(p.K) * 2 + 15) & ~(size_t)15) + 128 + (size_t)2 * mma_rows_per_pass(nb > 8 ? 16 : 8) * kGrWarps * nb * 4; };
         int bpp = std::min(B, 16);
+        while (bpp > 1 && need(bpp) > kSmemMost) --bpp;
+        if (need(bpp) > kSmemMost) {
+            ln.status = fail(OXG4_UNSUPPORTED, "projection %s needs %zu bytes of shared memory", kind, need(bpp));
+            return;
+        }
+        a.bpp = bpp;
+        ln.go(kind, bpp <= 8 ? pick_rows<8>(pro, epi) : pick_rows<16>(pro, epi), dim3(p.grid, (B + bpp - 1) / bpp, 1), dim3(kGrThreads), need(bpp), a);
+        return;
+    }
+    if (m->es == 2) {
+        // as many activation rows per pass as shared memory allows
+        size_t smem = 0;
+        int bpp = B;
         while (!gemv_mma_ring(&a, p, bpp, pro, epi, &smem)) {
             if (bpp == 1) {
                 ln.status = fail(OXG4_UNSUPPORTED, "projection %s needs %zu bytes of shared memory", kind, smem);
@@ -1603,7 +1636,7 @@ static void launch_gemv(Launcher& ln, const char* kind, oxg4_cache* c, int rows,
         if (ln.status != OXG4_OK) return;
         ln.status = encode_bf16_2d(&map1, epi == EPI_GATEUP ? a.W1 : a.W0, rows, (uint64_t)p.K, (uint32_t)a.box_rows);
         if (ln.status != OXG4_OK) return;
-        ln.go(kind, pick_mma(bpp, pro, epi, p.K > 3 * 4 * kGmThreads), dim3(p.grid, (B + bpp - 1) / bpp, 1), dim3(kGmThreads), smem, map0, map1, a);
+        ln.go(kind, pick_mma(pro, epi, p.K > 3 * 4 * kGmThreads), dim3(p.grid, (B + bpp - 1) / bpp, 1), dim3(kGmThreads), smem, map0, map1, a);
         return;
     }
     // f32 weights: SIMT kernel
@@ -1976,7 +2009,7 @@ static Pending run_layers(oxg4_cache* c, Launcher& ln, const RowSet& rs, bool us
     int s_down = rs.chunk ? c->ps_down : c->s_down;
     const bool wide = rs.chunk && c->wide && R > kWideRows;
     // small batches of BF16 models: the feed-forward's values leave the gate/up launch as the down projection's operand
-    uint16_t* gu_x = m->es == 2 && m->I % 32 == 0 ? (uint16_t*)c->gu_raw : nullptr;
+    uint16_t* gu_x = m->es == 2 && R <= kGmMaxRows && m->I % 32 == 0 ? (uint16_t*)c->gu_raw : nullptr;
     if (m->P > 0) ple_prepare(c, ln, rs);
     for (int l = 0; l < L; ++l) {
         const LayerPlan& p = m->layers[l];

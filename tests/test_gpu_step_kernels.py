@@ -1,5 +1,5 @@
 """Kernels of decode steps with few sequences at the sizes where they can go wrong: projections through shared memory
-(csrc/gemv_mma.cuh) with columns and rows that fill no box, and the attention of one token (csrc/attention.cuh) with units of fewer
+(csrc/gemv_mma.cuh, csrc/gemv_rows.cuh) with columns and rows that fill no box, and the attention of one token (csrc/attention.cuh) with units of fewer
 heads than a key/value head has, positions around split and window edges."""
 import numpy as np
 import pytest
@@ -13,19 +13,27 @@ pytestmark = pytest.mark.gpu
 TOL = 4 * 2.0 ** -9
 
 
-@pytest.mark.parametrize("hidden,inter,heads,head_dim,vocab,batch", [
-    (72, 40, 1, 64, 37, 1),           # columns of a box past the end, fewer column blocks than warps
-    (264, 136, 2, 64, 301, 2),        # intermediate size no multiple of 32: activations in f32 between gate/up and down
-    (1160, 2080, 2, 128, 301, 3),     # three rows share four teams of warps
-    (2560, 4768, 8, 64, 4111, 1),     # 17 and 18 rows per CTA, 16 and 17 pairs: two boxes, the second nearly empty
-    (3072, 160, 4, 256, 5003, 1),     # norm weights in registers: the widest row
-    (3080, 160, 4, 256, 300, 1),      # one past it
-    (5632, 96, 2, 64, 300, 1),        # the widest hidden row
-    (3080, 96, 2, 64, 300, 4), (264, 96, 2, 64, 20011, 7), (2056, 10272, 2, 64, 300, 7)])
-def test_projections_of_few_rows(hidden, inter, heads, head_dim, vocab, batch):
+@pytest.mark.parametrize("hidden,inter,heads,head_dim,vocab,batch,tcgen05", [
+    (72, 40, 1, 64, 37, 1, True),           # columns of a box past the end, fewer column blocks than warps
+    (2560, 4768, 8, 64, 4111, 1, True),     # 17 and 18 rows per CTA, 16 and 17 pairs: two boxes, the second nearly empty
+    (3072, 160, 4, 256, 5003, 1, True),     # norm weights in registers: the widest row
+    (3080, 160, 4, 256, 300, 1, True),      # one past it
+    (5632, 96, 2, 64, 300, 1, True),        # the widest hidden row
+    (264, 136, 2, 64, 301, 2, True), (1160, 2080, 2, 128, 301, 3, True), (264, 96, 2, 64, 20011, 7, True), (2056, 10272, 2, 64, 300, 7, True),
+    # several rows without tcgen05, as models with per-layer embeddings and tensor-parallel ranks have them
+    (264, 136, 2, 64, 301, 2, False),       # intermediate size no multiple of 32: activations in f32 between gate/up and down
+    (1160, 2080, 2, 128, 301, 3, False),    # three rows share four teams of warps
+    (3080, 96, 2, 64, 300, 4, False), (264, 96, 2, 64, 20011, 7, False), (72, 40, 1, 64, 37, 8, False),
+    (264, 20000, 2, 64, 300, 7, False), (264, 20008, 2, 64, 300, 8, False),     # as many rows of the down projection as fit, twice
+    (264, 136, 2, 64, 301, 9, False), (1160, 2080, 2, 128, 20011, 15, False),   # csrc/gemv_rows.cuh
+    (264, 96, 2, 64, 301, 17, False),       # sixteen rows and one
+    (264, 20000, 2, 64, 300, 9, False)])    # nine rows, of the down projection five at a time
+def test_projections_of_few_rows(hidden, inter, heads, head_dim, vocab, batch, tcgen05, monkeypatch):
     cfg = small_cfg(hidden=hidden, layers=1, heads=heads, kv_heads=1 if heads != 8 else 4, head_dim=head_dim, inter=inter, vocab=vocab,
                     window=64, layer_types=["full_attention"])
     gpu, oracle = build_pair(cfg, "bf16", kv_bf16=True, norm_jitter=0.1)
+    if not tcgen05:
+        monkeypatch.setenv("OXG4_DISABLE_TCGEN05", "1")        # looked at when a table is made
     table = gpu.new_cache_table([8] * batch, batch=batch, page_tokens=16, kv_dtype=pkg.BF16)
     caches = [oracle.new_cache(8) for _ in range(batch)]
     for t in range(3):
@@ -33,6 +41,11 @@ def test_projections_of_few_rows(hidden, inter, heads, head_dim, vocab, batch):
         want = np.stack([c.decode_logits(int(x)) for c, x in zip(caches, tokens)])
         got = np.atleast_2d(gpu.decode_token(tokens, table))
         assert (np.linalg.norm(got - want, axis=1) / np.linalg.norm(want, axis=1)).max() <= TOL
+        if batch > 1 and t == 0:                               # the fused arg-max, one position on
+            best = gpu.decode_topk(tokens, table, 1, 1.0, False)[0].astype(np.int64)
+            want = np.stack([c.decode_logits(int(x)) for c, x in zip(caches, tokens)])
+            top = np.take_along_axis(want, best, 1)[:, 0]
+            assert (want.max(1) - top <= 2 * TOL * np.linalg.norm(want, axis=1)).all()
 
 
 # f32 cache: rounding of f32 sums. BF16 cache: a key's element (up to 4 after its norm) that lies between two BF16 values may round to
