@@ -4,7 +4,7 @@
 // (crates/oxide-torch-models/src/gemma4_cuda/decode.rs:82-157; device math in
 // crates/oxide-torch-cuda/src/kernel_module.rs:1133-1246,1423-1439,1510-1550,1790-1894).
 //
-// attn_step_kernel: decode steps. attn_rows_kernel: rows whose K/V are in the cache already (prompt chunks, KV-shared layers). The
+// attn_step_kernel, attn_decode_kernel: decode steps. attn_rows_kernel: rows whose K/V are in the cache already (prompt chunks, KV-shared layers). The
 // visible positions of a sequence are partitioned into up to `n_splits` contiguous ranges, a CTA each (split-KV "flash decoding" with
 // an online softmax per warp). Partial sums are added in a fixed order, so the result does not depend on scheduling. Attention
 // scale is 1.0 as in the reference (no 1/sqrt(d)).
@@ -16,6 +16,7 @@
 //
 // HBM-bound: bytes per launch = 2 * visible_positions * kv_heads * head_dim * sizeof(KV element).
 #pragma once
+#include <cooperative_groups.h>
 #include <type_traits>
 
 #include "common.cuh"
@@ -141,29 +142,62 @@ struct BarCta {
     DEVINL void operator()() const { __syncthreads(); }
 };
 
-// Rows whose keys and values are in the cache already (a prompt chunk, a KV-shared layer): one CTA's share of a launch, split `s` of
-// kv head `kvh` of row `b`. Partials go through global memory, the last CTA of a (row, kv head) to arrive merges them.
-template <typename KT, int D, int G, typename BAR>
+// Norm of one head (times w) and, with `rotate`, its rotation: channel d rotates with d + D / 2, sixteen lanes away; cs(e) and sn(e) are
+// the factors of this lane's channels (sn negated in the first half), 1 and 0 past the rotated ones. The result is rounded once. Element by
+// element, as the K/V rows of the first round occupy most registers meanwhile.
+template <typename NT, int EPT, typename C, typename S>
+DEVINL void norm_rotate(float (&t)[EPT], const float (&w)[EPT], const C& cs, const S& sn, float eps, bool rotate) {
+    NT ss = 0;
+#pragma unroll
+    for (int e = 0; e < EPT; ++e) ss += (NT)t[e] * (NT)t[e];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const NT r = (NT)1 / sqrt(ss / (NT)(32 * EPT) + (NT)eps);
+#pragma unroll
+    for (int e = 0; e < EPT; ++e) {
+        NT v = (NT)t[e] * r * (NT)w[e];
+        if (rotate) v = v * (NT)cs(e) + __shfl_xor_sync(0xffffffffu, v, 16) * (NT)sn(e);
+        t[e] = (float)v;
+    }
+}
+// With an f32 cache norm and rotation of a step's token are done in doubles: their roundings in q and k were most of the error of
+// the scores, and with it of an f32 model.
+template <typename KT> using NormT = typename std::conditional<sizeof(KT) == 4, double, float>::type;
+
+// One CTA's share of a launch: split `s` of kv head `kvh` of sequence `b`, computed by the `nthreads`
+// threads that call it (tid = threadIdx.x < nthreads). `sm` is attn_cta_floats() floats of shared memory.
+template <typename KT, int D, int G, bool CL, bool DEEP, typename BAR>
 DEVINL void attn_cta(const AttnArgs& a, float* sm, const int s, const int kvh, const int b, const int nthreads,
                      const BAR bar) {
     constexpr int EPT = D / 32;
     const int NW = nthreads >> 5;            // 16 warps when few CTAs exist (latency), 4 when many (occupancy)
     float* qs = sm;                          // [G][D]
-    float* wm = qs + G * D;                  // [NW][G]
+    float* kcur = qs + G * D;                // [D]
+    float* vcur = kcur + D;                  // [D]
+    float* wm = qs + G * D + (CL ? 2 * D : 0);   // [NW][G]
     float* wl = wm + NW * G;                 // [NW][G]
     float* wacc = wl + NW * G;               // [NW][G][D]
-    float* rope = wacc + NW * G * D;         // [D] cos (first half) and sin (second half) of pos * inv_freq
+    float* cpart = wacc + NW * G * D;        // [G][D + 2] this CTA's partial (cluster variant)
+    float* rope = cpart + (CL ? G * (D + 2) : 0);   // [D] cos (first half) and sin (second half) of pos * inv_freq
     __shared__ unsigned int s_last;
-    __shared__ float s_scale[16 * 8], s_M[8];             // merge scratch: up to 16 warps x 8 heads
+    __shared__ float s_scale[16 * 8], s_l[16 * 8], s_M[8];   // merge scratch: up to 16 warps or cluster splits x 8 heads
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int half = D / 2;
 
+    // The variant that merges through global memory (CL = false) serves the rows of a prompt chunk: K and V of
+    // every row, the current position included, are already in the cache (qkv_post_kernel appended the whole
+    // chunk first), so the CTA only norms its queries.
+    constexpr bool ext = !CL;
     // model constants for this lane's slice of a head: fetched before the dependency wait
-    float wq[EPT];
+    float w[EPT];                            // CL: of this warp's first task, see below
+    auto load_w = [&](int task) {
 #pragma unroll
-    for (int e = 0; e < EPT; ++e) wq[e] = a.q_norm[lane * EPT + e];
-    // Step state (token, position, ring capacity, page table) was there before the preceding kernel started: it may be read, and the
+        for (int e = 0; e < EPT; ++e) w[e] = task < G || ext ? a.q_norm[lane * EPT + e] : task == G ? a.k_norm[lane * EPT + e] : 1.0f;
+    };
+    load_w(warp);
+    // Step state (token, position, ring capacity, page table) and the K/V rows of earlier positions were complete before the step's
+    // first kernel (which waits before it lets its successor start), a chunk's row data before the chunk: they may be read, and the
     // rotation factors computed, ahead of the dependency wait.
     const bool active = a.tokens[b] != kInactiveToken;
     const int pos = a.pos[b];
@@ -174,9 +208,13 @@ DEVINL void attn_cta(const AttnArgs& a, float* sm, const int s, const int kvh, c
     const int n_eff = min(a.n_splits, (n + a.min_split - 1) / a.min_split);
     const bool has_work = active && s < n_eff;
     float* part = a.part + (((size_t)b * a.Nkv + kvh) * a.n_splits) * (size_t)(G * (D + 2));
+    size_t cur_off = 0;
+    // this CTA's range of positions, and the loads of its first step: K/V rows of earlier positions were
+    // written by earlier steps, so they can be in flight while the QKV projection finishes and while the
+    // prologue below runs
     const int begin = has_work ? lo + (int)(((long long)n * s) / n_eff) : 0;
     const int end = has_work ? lo + (int)(((long long)n * (s + 1)) / n_eff) : 0;
-    constexpr int PD = 2;
+    constexpr int PD = DEEP ? 4 : 2;
     typedef KRaw<KT, EPT> Raw;
     const KT* kpool = (const KT*)a.kpool;
     const KT* vpool = (const KT*)a.vpool;
@@ -186,15 +224,22 @@ DEVINL void attn_cta(const AttnArgs& a, float* sm, const int s, const int kvh, c
         return (((size_t)pt[slot / a.page_tokens] * a.Nkv + kvh) * a.page_tokens +
                 (slot % a.page_tokens)) * (size_t)D + lane * EPT;
     };
-    auto issue = [&](int p, Raw& kr, Raw& vr) {
-        if (p < end) {
+    auto issue = [&](int p, Raw& kr, Raw& vr) {            // loads only; the current token comes from shared memory
+        if (p < end && (p != pos || ext)) {
             const size_t off = row_offset(p);
             kraw_load<KT, EPT>(kpool + off, kr);
             kraw_load<KT, EPT>(vpool + off, vr);
         }
     };
     Raw kr[PD], vr[PD];
+    if (has_work && !ext) {
+#pragma unroll
+        for (int q = 0; q < PD; ++q) issue(begin + warp + q * NW, kr[q], vr[q]);
+    }
     if (has_work) {
+        const int slot_cur = pos % cap;
+        cur_off = (((size_t)pt[slot_cur / a.page_tokens] * a.Nkv + kvh) *
+                       a.page_tokens + (slot_cur % a.page_tokens)) * (size_t)D;
         // rotation factors of this position, one cosf or sinf per thread instead of 2 * D / 32 per lane
         for (int i = tid; i < D; i += nthreads) {
             const int fi = i % half;
@@ -208,17 +253,24 @@ DEVINL void attn_cta(const AttnArgs& a, float* sm, const int s, const int kvh, c
     pdl_wait();
     pdl_launch();
     stamp(a.ts, 1);
-    if (has_work) {
-        // the newest K/V rows were appended by the preceding kernel, so nothing may be read from the cache before the dependency wait
+    if (has_work && ext) {
+        // rows of a prompt chunk: the K/V rows of this very chunk were appended by the preceding kernel, so
+        // nothing may be read from the cache before the dependency wait
 #pragma unroll
         for (int q = 0; q < PD; ++q) issue(begin + warp + q * NW, kr[q], vr[q]);
     }
 
     if (has_work) {
+        const bool owner = (s == n_eff - 1);        // the range that contains `pos`
         bar();                                      // the rotation factors are in shared memory
-        // one warp per query head: norm and rotation
-        for (int task = warp; task < G; task += NW) {
-            const int col = (kvh * G + task) * D;
+        // tasks 0..G-1: query heads (norm + rope); task G: key (norm + rope + append);
+        // task G+1: value (unit norm + append). One warp per task.
+        const int n_tasks = (owner && !ext) ? G + 2 : G;
+        for (int task = warp; task < n_tasks; task += NW) {
+            int col;
+            if (task < G) col = (kvh * G + task) * D;
+            else if (task == G) col = a.Nq * D + kvh * D;
+            else col = (a.Nq + a.Nkv) * D + kvh * D;
             float t[EPT];
             float ss = 0.0f;
 #pragma unroll
@@ -229,28 +281,48 @@ DEVINL void attn_cta(const AttnArgs& a, float* sm, const int s, const int kvh, c
                 t[e] = v;
                 ss += v * v;
             }
-            ss = warp_sum(ss);
-            const float r = 1.0f / sqrtf(ss / (float)D + a.eps);
-            float* dst = qs + task * D;
+            float* dst = task < G ? qs + task * D : (task == G ? kcur : vcur);
+            if constexpr (CL) {
+                if (task != warp) load_w(task);
+                const float* f = rope + (lane & 15) * EPT;
+                norm_rotate<NormT<KT>>(t, w, [&](int e) { return f[e]; }, [&](int e) { return lane < 16 ? -f[half + e] : f[half + e]; }, a.eps, task <= G);
 #pragma unroll
-            for (int e = 0; e < EPT; ++e) dst[lane * EPT + e] = t[e] * r * wq[e];
-            __syncwarp();
-            float o[EPT];
+                for (int e = 0; e < EPT; ++e) dst[lane * EPT + e] = t[e];
+            } else {
+                ss = warp_sum(ss);
+                const float r = 1.0f / sqrtf(ss / (float)D + a.eps);
 #pragma unroll
-            for (int e = 0; e < EPT; ++e) {
-                const int d = lane * EPT + e;
-                const int fi = d % half;
-                float v = dst[d];
-                if (fi < a.rotary_half) {
-                    const float pv = dst[d < half ? d + half : d - half];
-                    const float rotated = d < half ? -pv : pv;
-                    v = v * rope[fi] + rotated * rope[half + fi];
+                for (int e = 0; e < EPT; ++e) dst[lane * EPT + e] = t[e] * r * w[e];
+                __syncwarp();
+                float o[EPT];
+#pragma unroll
+                for (int e = 0; e < EPT; ++e) {
+                    const int d = lane * EPT + e;
+                    const int fi = d % half;
+                    float v = dst[d];
+                    if (fi < a.rotary_half) {
+                        const float pv = dst[d < half ? d + half : d - half];
+                        const float rotated = d < half ? -pv : pv;
+                        v = v * rope[fi] + rotated * rope[half + fi];
+                    }
+                    o[e] = v;
                 }
-                o[e] = v;
-            }
-            __syncwarp();
+                __syncwarp();
 #pragma unroll
-            for (int e = 0; e < EPT; ++e) dst[lane * EPT + e] = o[e];
+                for (int e = 0; e < EPT; ++e) dst[lane * EPT + e] = o[e];
+            }
+            if (task >= G) {
+                // append to the cache; keep the stored (possibly BF16-rounded) value for this step
+                KT* pool = (KT*)(task == G ? a.kpool : a.vpool);
+                __syncwarp();
+#pragma unroll
+                for (int e = 0; e < EPT; ++e) {
+                    const int d = lane * EPT + e;
+                    const KT stored = kv_store_cvt<KT>(dst[d]);
+                    pool[cur_off + d] = stored;
+                    dst[d] = kv_widen<KT>(stored);
+                }
+            }
         }
         bar();
         stamp(a.ts, 2);
@@ -276,8 +348,14 @@ DEVINL void attn_cta(const AttnArgs& a, float* sm, const int s, const int kvh, c
             float sc[NP][G];
 #pragma unroll
             for (int q = 0; q < NP; ++q) {
+                const int pq = p0 + q * NW;
                 float kf[EPT];
-                kraw_cvt<KT, EPT>(kr[q], kf);              // rows past `end` were never loaded: their scores are not used
+                if (pq == pos && !ext) {
+#pragma unroll
+                    for (int e = 0; e < EPT; ++e) kf[e] = kcur[lane * EPT + e];
+                } else {
+                    kraw_cvt<KT, EPT>(kr[q], kf);          // rows past `end` were never loaded: their scores are not used
+                }
 #pragma unroll
                 for (int g = 0; g < G; ++g) {
                     float t = 0.0f;
@@ -314,9 +392,15 @@ DEVINL void attn_cta(const AttnArgs& a, float* sm, const int s, const int kvh, c
             }
 #pragma unroll
             for (int q = 0; q < NP; ++q) {
-                if (p0 + q * NW >= end) break;
+                const int pq = p0 + q * NW;
+                if (pq >= end) break;
                 float vf[EPT];
-                kraw_cvt<KT, EPT>(vr[q], vf);
+                if (pq == pos && !ext) {
+#pragma unroll
+                    for (int e = 0; e < EPT; ++e) vf[e] = vcur[lane * EPT + e];
+                } else {
+                    kraw_cvt<KT, EPT>(vr[q], vf);
+                }
 #pragma unroll
                 for (int g = 0; g < G; ++g)
 #pragma unroll
@@ -324,7 +408,7 @@ DEVINL void attn_cta(const AttnArgs& a, float* sm, const int s, const int kvh, c
             }
         };
         // PD positions per step, the next step's loads issued before this step's arithmetic: 2 * PD rows of
-        // K and of V in flight per warp
+        // K and of V in flight per warp (PD = 4 when one sequence has the whole GPU and latency is all that counts)
         for (int p = begin + warp; p < end; p += PD * NW) {
             Raw nk[PD], nv[PD];
 #pragma unroll
@@ -353,7 +437,7 @@ DEVINL void attn_cta(const AttnArgs& a, float* sm, const int s, const int kvh, c
             if (tid < G) s_M[g] = M;
         }
         bar();
-        float* my = part + (size_t)s * (G * (D + 2));
+        float* my = CL ? cpart : part + (size_t)s * (G * (D + 2));
         for (int idx = tid; idx < G * D; idx += nthreads) {
             const int g = idx / D, d = idx % D;
             float A = 0.0f, L = 0.0f;
@@ -367,6 +451,57 @@ DEVINL void attn_cta(const AttnArgs& a, float* sm, const int s, const int kvh, c
         }
     }
 
+    if constexpr (CL) {
+        // ---- cluster merge: every CTA finishes a slice of the outputs from its peers' shared memory ----
+        namespace cg = cooperative_groups;
+        cg::cluster_group cluster = cg::this_cluster();
+        stamp(a.ts_mid, 2);
+        cluster.sync();                                    // every CTA of the cluster arrives, with or without work
+        stamp(a.ts_mid, 3);
+        if (active) {
+            // (m, l) of every split -> this CTA's shared memory in one round of remote loads, then one scale
+            // factor per (split, head); the weighted sums below are independent remote loads
+            if (tid < n_eff * G) {
+                const int sp = tid / G, g = tid % G;
+                const float* ps = cluster.map_shared_rank(cpart, sp) + g * (D + 2);
+                s_scale[tid] = ps[D];
+                s_l[tid] = ps[D + 1];
+            }
+            bar();
+            if (tid < G) {
+                const int g = tid;
+                float M = -INFINITY;
+                for (int sp = 0; sp < n_eff; ++sp) M = fmaxf(M, s_scale[sp * G + g]);
+                float L = 0.0f;
+                for (int sp = 0; sp < n_eff; ++sp) {
+                    const float ms = s_scale[sp * G + g];
+                    const float e = (ms == -INFINITY) ? 0.0f : expf(ms - M);
+                    s_scale[sp * G + g] = e;
+                    L += e * s_l[sp * G + g];
+                }
+                s_M[g] = L;
+            }
+            bar();
+            const int cs = (int)gridDim.x;
+            const int per = (G * D + cs - 1) / cs;
+            const int hi = min(G * D, (s + 1) * per);
+            for (int idx = s * per + tid; idx < hi; idx += nthreads) {
+                const int g = idx / D, d = idx % D;
+                float A = 0.0f;
+                for (int sp = 0; sp < n_eff; ++sp)
+                    A += s_scale[sp * G + g] * cluster.map_shared_rank(cpart, sp)[g * (D + 2) + d];
+                {
+                    const size_t oi = (size_t)b * a.Nq * D + (size_t)(kvh * G + g) * D + d;
+                    const float ov = A / s_M[g];
+                    a.out[oi] = ov;
+                    if (a.out_bf16) a.out_bf16[oi] = (uint16_t)f32_to_bf16_bits(ov);
+                }
+            }
+        }
+        cluster.sync();                                    // no CTA leaves while a peer may still read its partial
+        stamp(a.ts, 3);
+        return;
+    }
     // ---- last CTA of this (sequence, kv head) merges the split partials in split order ----
     stamp(a.ts_mid, 0);
     __threadfence();
@@ -430,10 +565,26 @@ DEVINL void attn_cta(const AttnArgs& a, float* sm, const int s, const int kvh, c
     stamp(a.ts, 3);
 }
 
+// Decode steps of many units over many positions (attn_step_kernel takes the others). CL: the splits of one (sequence, kv head) form a
+// thread-block cluster (gridDim.x <= 16 CTAs); partials stay in shared memory and are merged through distributed shared memory after one
+// cluster barrier; the CTA that owns the current position also norms, rotates and appends its K and V.
+template <typename KT, int D, int G, bool DEEP>
+__global__ void __launch_bounds__(kAttnThreads, DEEP && D == 256) attn_decode_kernel(const AttnArgs a) {
+    extern __shared__ __align__(16) float attn_sm[];
+    attn_cta<KT, D, G, true, DEEP>(a, attn_sm, blockIdx.x, blockIdx.y, blockIdx.z, blockDim.x, BarCta{});
+}
+
+// Rows whose K/V are in the cache already (a prompt chunk, a KV-shared layer): partials go through global memory and the
+// last CTA to arrive (atomic ticket) merges them.
 template <typename KT, int D, int G>
 __global__ void __launch_bounds__(kAttnThreads) attn_rows_kernel(const AttnArgs a) {
     extern __shared__ __align__(16) float attn_sm[];
-    attn_cta<KT, D, G>(a, attn_sm, blockIdx.x, blockIdx.y, blockIdx.z, blockDim.x, BarCta{});
+    attn_cta<KT, D, G, false, false>(a, attn_sm, blockIdx.x, blockIdx.y, blockIdx.z, blockDim.x, BarCta{});
+}
+
+// Floats of shared memory of the two with NW warps per CTA
+template <bool CL> inline size_t attn_cta_floats(int D, int G, int NW) {
+    return (size_t)G * D + (CL ? 2 * D + G * (D + 2) : 0) + 2 * NW * G + (size_t)NW * G * D + D;
 }
 
 // ---- decode steps ----------------------------------------------------------------------------------------------------
@@ -580,26 +731,7 @@ __global__ void __launch_bounds__(kAttnStepThreads, 2) attn_step_kernel(const At
                 w[e] = task <= G ? (task < G ? a.q_norm : a.k_norm)[lane * EPT + e] : 1.0f;
             }
         }
-        // With an f32 cache norm and rotation are done in doubles and rounded once: their roundings in q and k were most of the error of
-        // the scores, and with it of an f32 model.
-        typedef typename std::conditional<sizeof(KT) == 4, double, float>::type NT;
-        NT ss = 0, v[EPT];
-#pragma unroll
-        for (int e = 0; e < EPT; ++e) {
-            v[e] = t[e];
-            ss += v[e] * v[e];
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        const NT r = (NT)1 / sqrt(ss / (NT)D + (NT)a.eps);
-#pragma unroll
-        for (int e = 0; e < EPT; ++e) v[e] = v[e] * r * (NT)w[e];
-        if (task <= G) {                               // channel d rotates with d + D / 2: sixteen lanes away; past rotary_half cos is 1 and sin 0
-#pragma unroll
-            for (int e = 0; e < EPT; ++e) v[e] = v[e] * (NT)cs[e] + __shfl_xor_sync(0xffffffffu, v[e], 16) * (NT)sn[e];
-        }
-#pragma unroll
-        for (int e = 0; e < EPT; ++e) t[e] = (float)v[e];
+        norm_rotate<NormT<KT>>(t, w, [&](int e) { return cs[e]; }, [&](int e) { return sn[e]; }, a.eps, task <= G);
         float* dst = (task < G ? qs + task * D : task == G ? kcur : vcur) + lane * EPT;
         if (task >= G) {
             // the stored (possibly BF16-rounded) value is what this step uses too

@@ -483,10 +483,19 @@ static int32_t set_gemv_attrs() {
     return OXG4_OK;
 }
 
+template <typename F>
+static int32_t decode_attrs(F* kernel) {
+    TRY(allow_big_smem(kernel));
+    CK(cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    return OXG4_OK;
+}
+
 template <typename KT, int D, int G>
 static int32_t set_attn_attrs() {
     TRY((allow_big_smem(attn_rows_kernel<KT, D, G>)));
     TRY((shared_sm_attrs(attn_step_kernel<KT, D, G>)));
+    TRY((decode_attrs(attn_decode_kernel<KT, D, G, false>)));
+    if constexpr (G <= 2) TRY((decode_attrs(attn_decode_kernel<KT, D, G, true>)));
     CK(cudaFuncSetAttribute(attn_step_kernel<KT, D, G>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     return OXG4_OK;
 }
@@ -1390,6 +1399,7 @@ static int32_t tc_gemm_setup() {
 struct Launcher {
     oxg4_model* m;
     unsigned long long* ts_base = nullptr;
+    int carveout = -1;            // >= 0: the next kernel prefers this percentage of an SM's memory as shared memory
     int cluster_x = 0;            // > 0: launch the next kernel with thread-block clusters of this many CTAs along x
     bool coop = false;            // launch the next kernel cooperatively (all CTAs resident at once), without PDL
     bool early = false;           // decode step: SIMT projections let their successor start before they wait (see gemv.cuh)
@@ -1411,8 +1421,13 @@ struct Launcher {
         cfg.blockDim = block;
         cfg.dynamicSmemBytes = smem;
         cfg.stream = m->stream;
-        cudaLaunchAttribute attr[2];
+        cudaLaunchAttribute attr[3];
         int na = 0;
+        if (carveout >= 0) {
+            attr[na].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+            attr[na].val.sharedMemCarveout = (unsigned)carveout;
+            ++na;
+        }
         if (coop) {
             attr[na].id = cudaLaunchAttributeCooperative;
             attr[na].val.cooperative = 1;
@@ -1660,16 +1675,22 @@ static void launch_gemv(Launcher& ln, const char* kind, oxg4_cache* c, int rows,
     ln.go(kind, fn, grid, dim3(kSimtThreads), smem, a);
 }
 
-// step: attn_step_kernel (a decode step), otherwise attn_rows_kernel; floats: shared memory of attn_step_kernel
+enum AttnKind { ATTN_ROWS, ATTN_DECODE, ATTN_DECODE_DEEP, ATTN_STEP };
 typedef void (*AttnFn)(const AttnArgs);
-template <typename KT>
-static AttnFn pick_attn(int D, int G, bool step, int NW, int splits, size_t* floats) {
-#define PA1(DD, GG)                                                                       \
-    if (D == DD && G == GG) {                                                             \
-        *floats = attn_step_floats<DD, GG>(NW, splits);                                   \
-        if (step) return attn_step_kernel<KT, DD, GG>;                                    \
-        return attn_rows_kernel<KT, DD, GG>;                                              \
+template <typename KT, int D, int G>
+static AttnFn pick_attn_kind(AttnKind kind, int NW, int splits, size_t* floats) {
+    *floats = kind == ATTN_STEP ? attn_step_floats<D, G>(NW, splits) : kind == ATTN_ROWS ? attn_cta_floats<false>(D, G, NW) : attn_cta_floats<true>(D, G, NW);
+    if (kind == ATTN_STEP) return attn_step_kernel<KT, D, G>;
+    if (kind == ATTN_ROWS) return attn_rows_kernel<KT, D, G>;
+    if constexpr (G <= 2) {
+        if (kind == ATTN_DECODE_DEEP) return attn_decode_kernel<KT, D, G, true>;
     }
+    return attn_decode_kernel<KT, D, G, false>;
+}
+template <typename KT>
+static AttnFn pick_attn(int D, int G, AttnKind kind, int NW, int splits, size_t* floats) {
+#define PA1(DD, GG) \
+    if (D == DD && G == GG) return pick_attn_kind<KT, DD, GG>(kind, NW, splits, floats);
 #define PA(DD) PA1(DD, 1) PA1(DD, 2) PA1(DD, 4) PA1(DD, 8)
     PA(64) PA(128) PA(256)
 #undef PA
@@ -1767,6 +1788,42 @@ static QkvPostFn pick_qkv_post(int kv_dtype, int D, bool few) {
     return few ? pick_qkv_post<float, true>(D) : pick_qkv_post<float, false>(D);
 }
 
+// One token per sequence: attn_step_kernel (true) or attn_decode_kernel, both with `ctas` CTAs of `splits` per (sequence, kv head). The
+// first is the quicker launch; the second has sixteen warps in a CTA of its own where the first has eight. Times of the first over the
+// second, 60 to 9000 positions, one to 128 (sequence, kv head), head sizes 64 / 128 / 256, f32 and BF16 caches:
+//   more CTAs than SMs (four warps each in both): 0.85 - 1.0; f32 caches of head size 256 0.9 - 1.0 at 200 positions, 1.05 - 1.2 at 800; eight
+//     heads per kv head, from twenty (sequence, kv head) on, 0.9 - 0.98 with head size 64, 0.93 - 1.0 with 128 up to the limits and 1.05 - 1.15
+//     beyond, 1.0 - 1.08 with 256; one or two heads and so many CTAs that its registers leave some waiting, 1.1
+//   heads dealt to more clusters: 0.3 - 1.0 at 9000 positions with eight heads or four of 256, four smaller ones up to 1.1; two 0.7 - 0.97 at
+//     2500 and up to 1.16 at 9000
+//   more than four fifths of the SMs: 0.65 - 0.97 up to 2500 positions (clusters that fill their SMs don't all find room), f32 caches of head
+//     size 256 up to 1.1 there and 1.2 at 9000
+//   fewer: eight heads 0.65 - 0.9 below 16 positions per CTA, 1.0 - 1.4 at 30 - 50; four 0.84 - 1.0 at 30 - 50, 1.1 at 100; one or two 0.83 -
+//     1.0 at 100, 1.1 - 1.2 at 300
+// `vis` is what the table has room for, as everywhere in the geometry of a step: the captured step serves all positions.
+static bool step_kernel(bool dealt, int ctas, int sms, int splits, int G, int D, int vis, int kv_dtype) {
+    const bool bf16 = kv_dtype == OXG4_BF16;
+    if (G == 8 && ctas >= 20 * splits && D > 64) return D == 128 && vis <= (bf16 ? 32 : 128) * splits;
+    if (ctas > sms) return (ctas <= 4 * sms || G >= 4) && (bf16 || D < 256 || vis <= 32 * splits);
+    if (dealt) return vis <= (G == 2 ? (bf16 ? 640 : 384) : G == 4 && D < 256 && !bf16 ? 512 : 1024) * splits;
+    const bool light = bf16 || D < 256;          // registers to spare
+    if (5 * ctas > 4 * sms) return vis <= (light && (D > 64 || G > 1) ? 640 : light || G != 4 ? 320 : 224) * splits;
+    return vis <= (G == 8 ? 16 : G == 4 ? (bf16 ? 100 : 56) : light ? 160 : 100) * splits;
+}
+
+// Units (sequence, kv head) times positions up to which a step with the tensor-core attention at hand attends in one of these launches
+// instead of its three. Times of the one over the three at half and at twice the limit: one head per kv head 0.8 / 1.1 - 1.4, two 0.8 - 0.9
+// / 1.2, four 0.8 - 0.9 / 1.3, eight 0.7 - 0.9 / 1.3 - 2.
+// Few units keep the limit further out (the three launches leave most of the GPU idle); eight heads of 256 from sixteen units on: 1.0 at
+// 200 positions, 2.5 at 2500.
+static double one_launch_most(int G, int D, int units) {
+    if (units > 64) return 0;
+    if (G == 1) return units < 8 ? 80e3 : units < 32 ? 48e3 : 55e3;
+    if (G == 2) return units < 8 ? 65e3 : units < 16 ? 45e3 : units < 32 ? 32e3 : 50e3;
+    if (G == 4) return units < 8 ? 50e3 : units < 16 ? 32e3 : 26e3;
+    return units <= 4 ? 32e3 : units < 8 ? 20e3 : units < 16 ? 12e3 : D < 256 ? 14e3 : 2.2e3;
+}
+
 // q/k norm + RoPE + v norm + KV append + attention of layer l for the rows of `rs` (decode.rs:99-157,
 // 176-325). qkv: [qkv_splits, split_rows, qkv_n] projection output; the result goes to `out` (+ BF16 copy).
 // split_rows: rows between two partials of qkv; out: [R, qw].
@@ -1779,10 +1836,8 @@ static void launch_attention(Launcher& ln, oxg4_cache* c, const RowSet& rs, int 
     const int pps = p.sliding ? c->pps_slide : c->pps_full;
     const int32_t* cap = p.sliding ? c->cap_slide : c->cap_full;
     const int window = p.sliding ? m->cfg.sliding_window : 0x7fffffff;
-    // Few units over few positions: one launch of attn_step_kernel instead of three (a step of the ~4B model, 16 sequences at 100 / 450 /
-    // 1000 positions: 2490 / 2775 / 3105 us, with three 2635 / 2810 / 3015; eight at 450: 2500 / 2650; 32 at 250, twice the units: 3190 / 2955)
     const int vis = p.sliding ? std::min(rs.max_visible, m->cfg.sliding_window) : rs.max_visible;
-    const bool few_units = !rs.chunk && !p.shared && R * p.Nkv <= 64 && 4.0 * R * vis * p.Nkv * D <= 40e6;
+    const bool few_units = !rs.chunk && !p.shared && (double)R * p.Nkv * vis <= one_launch_most(p.G, D, R * p.Nkv);
     const bool use_mma = c->mma_attn && (many_rows || rs.chunk) && !few_units;
     // K and V of the rows are in the cache before the attention kernel starts: rows of a prompt chunk (appended by
     // qkv_post_kernel), and every row of a KV-shared layer (its source layer appended them earlier in the step)
@@ -1856,21 +1911,28 @@ static void launch_attention(Launcher& ln, oxg4_cache* c, const RowSet& rs, int 
     a.out = out;
     a.ts = ln.ts();
     a.ts_mid = ln.ts_base ? ln.ts_base + 4 * (size_t)(kMaxTimeline - 1 - l) : nullptr;   // extra stamps, from the end of the buffer
-    const bool step = !kv_in_cache;              // the kernel appends K and V itself
     // few CTAs: one per SM at most, as many warps as the K/V rows in flight need; many CTAs: 4 warps each so that several fit on an SM
-    const bool few = a.n_splits * p.Nkv * R <= m->num_sms;
+    const int ctas = a.n_splits * p.Nkv * R;
+    const bool few = ctas <= m->num_sms;
     int unit = p.G;                              // query heads of a unit (attn_step_kernel)
     while (unit > 1 && 2 * a.n_splits * p.Nkv * (p.G / unit) * R <= m->num_sms) unit /= 2;
-    const int NW = few ? (step ? kAttnStepThreads / 32 : kAttnWarps) : 4;
+    const bool step = !kv_in_cache && step_kernel(unit < p.G, ctas, m->num_sms, a.n_splits, p.G, D, vis, c->kv_dtype);
+    const int NW = !few ? 4 : step ? kAttnStepThreads / 32 : kAttnWarps;
+    // attn_decode_kernel: more K/V rows in flight per warp when latency is all that counts (with more than two query heads
+    // per kv head the extra rows would spill registers)
+    const AttnKind attn_kind = kv_in_cache ? ATTN_ROWS : step ? ATTN_STEP : few && p.G <= 2 ? ATTN_DECODE_DEEP : ATTN_DECODE;
     a.group = p.G;
     a.early = ln.early ? 1 : 0;
     size_t floats = 0;
-    auto fn = c->kv_dtype == OXG4_BF16 ? pick_attn<uint16_t>(p.D, step ? unit : p.G, step, NW, a.n_splits, &floats)
-                                       : pick_attn<float>(p.D, step ? unit : p.G, step, NW, a.n_splits, &floats);
-    if (!step) floats = (size_t)p.G * D + 2 * NW * p.G + NW * p.G * D + D;
-    ln.cluster_x = step ? a.n_splits : 0;
+    auto fn = c->kv_dtype == OXG4_BF16 ? pick_attn<uint16_t>(p.D, step ? unit : p.G, attn_kind, NW, a.n_splits, &floats)
+                                       : pick_attn<float>(p.D, step ? unit : p.G, attn_kind, NW, a.n_splits, &floats);
+    ln.cluster_x = kv_in_cache ? 0 : a.n_splits;
+    // attn_decode_kernel with an SM per CTA asks for the shared memory that it needs, no more: behind a launch that left its SM the least L1
+    // there is, the instances that spill registers (f32 caches of head size 256, eight heads) took up to 1.45 times as long
+    ln.carveout = kv_in_cache || step || !few ? -1 : std::min<int>(100, (int)((sizeof(float) * floats + 3 * 1024) * 100 / (228 * 1024)) + 1);
     ln.go("attn", fn, dim3(a.n_splits, step ? p.Nkv * (p.G / unit) : p.Nkv, R), dim3(NW * 32), sizeof(float) * floats, a);
     ln.cluster_x = 0;
+    ln.carveout = -1;
 }
 
 // Attention of a prompt chunk on its own keys and values and those in the cache (csrc/prompt_attn.cuh); the rows that stay in

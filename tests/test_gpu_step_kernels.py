@@ -52,16 +52,18 @@ def test_projections_of_few_rows(hidden, inter, heads, head_dim, vocab, batch, t
 # the other one, 2^-6 away at most; with |q| up to 4 that moves a score by 2^-4, its softmax weight p by the factor exp(2^-4) and the
 # head's output by p (1 - p) 2^-4 <= 2^-6 of the values' size
 @pytest.mark.parametrize("kv", ["f32", "bf16"])
-@pytest.mark.parametrize("head_dim,heads,kv_heads,batch", [
-    (64, 1, 1, 1), (64, 8, 1, 1), (128, 4, 1, 1), (256, 2, 2, 1), (256, 8, 1, 1), (128, 16, 8, 1), (64, 8, 2, 3), (256, 4, 1, 5)])
-def test_attention_of_one_token(head_dim, heads, kv_heads, batch, kv):
+@pytest.mark.parametrize("head_dim,heads,kv_heads,batch,room", [
+    (64, 1, 1, 1, 0), (64, 8, 1, 1, 0), (128, 4, 1, 1, 0), (256, 2, 2, 1, 0), (256, 8, 1, 1, 0), (128, 16, 8, 1, 0), (64, 8, 2, 3, 0), (256, 4, 1, 5, 0),
+    # tables with room for so many positions that the other kernel attends in the global layer: with four and sixteen warps per CTA
+    (64, 1, 1, 1, 20000), (128, 4, 2, 1, 20000), (256, 8, 1, 5, 20000), (64, 8, 2, 3, 20000), (256, 2, 2, 1, 20000), (256, 8, 2, 24, 600)])
+def test_attention_of_one_token(head_dim, heads, kv_heads, batch, room, kv):
     cfg = small_cfg(hidden=128, layers=2, heads=heads, kv_heads=kv_heads, head_dim=head_dim, inter=128, vocab=600, window=40,
                     layer_types=["sliding_attention", "full_attention"])
     gpu, oracle = build_pair(cfg, "f32", kv_bf16=(kv == "bf16"), norm_jitter=0.1)
     n = 300
     seqs = [syn.prompt_ids(600, n, seed=10 * head_dim + b) for b in range(batch)]
     # a table for more positions than are used (sixteen splits) and, for one sequence, one for a handful (a split or two)
-    table = gpu.new_cache_table([n + 30 * b for b in range(batch)], batch=batch, page_tokens=16, kv_dtype=pkg.F32 if kv == "f32" else pkg.BF16)
+    table = gpu.new_cache_table([n + room + 30 * b for b in range(batch)], batch=batch, page_tokens=16, kv_dtype=pkg.F32 if kv == "f32" else pkg.BF16)
     small = gpu.new_cache_table(20, page_tokens=16, kv_dtype=pkg.F32 if kv == "f32" else pkg.BF16) if batch == 1 else None
     caches = [oracle.new_cache(n) for _ in range(batch)]
     look = {0, 1, 7, 15, 16, 17, 31, 32, 33, 39, 40, 41, 127, 128, 129, 255, 256, 257, 299}
@@ -80,3 +82,22 @@ def test_attention_of_one_token(head_dim, heads, kv_heads, batch, kv):
         if small is not None and t < 20:
             off = gpu.decode_token(tokens, small) - want[0]
             assert np.abs(off).max() <= 1e-3 if kv == "f32" else np.linalg.norm(off) <= 2.0 ** -6 * np.linalg.norm(want), t
+
+
+@pytest.mark.parametrize("head_dim,heads,kv_heads,batch,room", [
+    (64, 2, 2, 2, 0), (64, 2, 2, 2, 5000), (128, 8, 1, 5, 2000), (256, 2, 1, 3, 9000), (256, 8, 2, 8, 0), (64, 8, 1, 5, 9000)])
+def test_one_launch_or_three_beside_tcgen05(head_dim, heads, kv_heads, batch, room):
+    """Batches whose global layer attends by attn_step_kernel, attn_decode_kernel (with BF16 output) or the tensor-core attention, by
+    what the table has room for: the same logits to the rounding of BF16 operands."""
+    cfg = small_cfg(hidden=256, layers=1, heads=heads, kv_heads=kv_heads, head_dim=head_dim, inter=128, vocab=600, window=40, layer_types=["full_attention"])
+    gpu, oracle = build_pair(cfg, "bf16", kv_bf16=True, norm_jitter=0.1)
+    n = 40
+    seqs = [syn.prompt_ids(600, n, seed=40 * head_dim + b) for b in range(batch)]
+    table = gpu.new_cache_table([n + room] * batch, batch=batch, page_tokens=16, kv_dtype=pkg.BF16)
+    caches = [oracle.new_cache(n) for _ in range(batch)]
+    for t in range(n):
+        tokens = np.array([s[t] for s in seqs], dtype=np.uint32)
+        want = np.stack([c.decode_logits(int(x)) for c, x in zip(caches, tokens)])
+        got = gpu.decode_token(tokens, table)
+        # with the bound on the attention's output above
+        assert (np.linalg.norm(got - want, axis=1) / np.linalg.norm(want, axis=1)).max() <= TOL + 2.0 ** -6, t
