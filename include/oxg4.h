@@ -321,10 +321,13 @@ int32_t oxg4_smoke_cached_attention(oxg4_model* model, oxg4_cache* cache, uint32
  * polls (kind 2): the kernel returns, the status word is raised and the call returns OXG4_TIMEOUT; later calls work.
  * oxg4_debug_set_status sets the status word of the table's tensor-core kernels as a failed wait would: the launches of the next
  * call return without output, the call reports OXG4_TIMEOUT and clears the word.
+ * oxg4_debug_long_launches switches the one-row projections of a BF16 model between the kernel of long launches (1) and the one of
+ * short ones (0), whatever the model's sizes; tables that have made a step keep what they had.
  * oxg4_debug_fail_alloc_after makes the n-th device allocation of the next oxg4_cache_create report
  * OXG4_OOM (0 switches it off); the failed create must release everything it had allocated. */
 int32_t oxg4_debug_wait_timeout(oxg4_model* model, oxg4_cache* cache, int32_t kind, uint32_t spin_limit);
 int32_t oxg4_debug_set_status(oxg4_model* model, oxg4_cache* cache, int32_t code);
+int32_t oxg4_debug_long_launches(oxg4_model* model, int32_t on);
 void oxg4_debug_fail_alloc_after(int32_t n);
 
 /* Measurement aid (no counterpart in the reference): marks lens[b] positions of every sequence of an EMPTY cache

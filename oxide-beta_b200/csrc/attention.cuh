@@ -568,8 +568,11 @@ DEVINL void attn_cta(const AttnArgs& a, float* sm, const int s, const int kvh, c
 // Decode steps of many units over many positions (attn_step_kernel takes the others). CL: the splits of one (sequence, kv head) form a
 // thread-block cluster (gridDim.x <= 16 CTAs); partials stay in shared memory and are merged through distributed shared memory after one
 // cluster barrier; the CTA that owns the current position also norms, rotates and appends its K and V.
+// CTAs per SM that the registers are cut for. Head size 256 with rows ahead: one, its own choice of 64 registers spilled 800 bytes. 128 with a
+// BF16 cache: two, so that a launch behind one that fills its SMs starts on the first half of them that are free (5 us a layer of the ~27B widths).
+template <typename KT, int D, bool DEEP> constexpr int decode_ctas() { return !DEEP ? 0 : D == 256 ? 1 : D == 128 && sizeof(KT) == 2 ? 2 : 0; }
 template <typename KT, int D, int G, bool DEEP>
-__global__ void __launch_bounds__(kAttnThreads, DEEP && D == 256) attn_decode_kernel(const AttnArgs a) {
+__global__ void __launch_bounds__(kAttnThreads, decode_ctas<KT, D, DEEP>()) attn_decode_kernel(const AttnArgs a) {
     extern __shared__ __align__(16) float attn_sm[];
     attn_cta<KT, D, G, true, DEEP>(a, attn_sm, blockIdx.x, blockIdx.y, blockIdx.z, blockDim.x, BarCta{});
 }

@@ -1,5 +1,5 @@
-// Projections of small batches: what a launch does, and the kernel for f32 weights (1..4 activation rows per pass; BF16 weights:
-// gemv_mma.cuh).
+// Projections of small batches: what a launch does, and the kernel for f32 weights (1..4 activation rows per pass) and for one row of
+// models whose launches are long (other BF16 weights: gemv_mma.cuh, gemv_rows.cuh).
 //
 // One launch covers what the reference spreads over rms_norm[_bf16] + f32_to_bf16 + cublasGemmEx
 // (+ slice / gelu_mul / add / mul_bf16_scalar) launches — crates/oxide-torch-models/src/
@@ -29,7 +29,7 @@
 // that ends inside a row leaves a partial sum; the pieces of a row meet in shared memory and are
 // added in a fixed order, which keeps the split-K reduction deterministic without atomics.
 //
-// The kernel is HBM-bound: bytes per launch = N * K * 4.
+// The kernel is HBM-bound: bytes per launch = N * K * sizeof(weight); 6.0 TB/s over a step of the ~27B widths.
 #pragma once
 #include "common.cuh"
 #include "tc_gemm.cuh"
@@ -101,16 +101,35 @@ struct GemvArgs {
     float* best_scores;      // LOGITS: [B]
 };
 
-// acc[b] += dot(w (four weights), x (matching activations of row b))
-template <int NB>
-DEVINL void fma16(float (&acc)[NB], const uint4& w, const float* xs, int K, int k) {
+// an activation as the kernel keeps it in shared memory: BF16 beside BF16 weights, f32 beside f32 weights
+DEVINL void put_x(float* p, float v) { *p = v; }
+DEVINL void put_x(uint16_t* p, float v) { *p = (uint16_t)f32_to_bf16_bits(v); }
+
+// acc[b] += dot(w (16 bytes of weights), x (matching activations of row b))
+template <typename WT, int NB>
+DEVINL void fma16(float (&acc)[NB], const uint4& w, const WT* xs, int K, int k) {
+    if constexpr (sizeof(WT) == 2) {
+        const float w0 = bf16lo(w.x), w1 = bf16hi(w.x), w2 = bf16lo(w.y), w3 = bf16hi(w.y);
+        const float w4 = bf16lo(w.z), w5 = bf16hi(w.z), w6 = bf16lo(w.w), w7 = bf16hi(w.w);
 #pragma unroll
-    for (int b = 0; b < NB; ++b) {
-        const float4 x = *reinterpret_cast<const float4*>(xs + (size_t)b * K + k);
-        float a = acc[b];
-        a = fmaf(__uint_as_float(w.x), x.x, a); a = fmaf(__uint_as_float(w.y), x.y, a);
-        a = fmaf(__uint_as_float(w.z), x.z, a); a = fmaf(__uint_as_float(w.w), x.w, a);
-        acc[b] = a;
+        for (int b = 0; b < NB; ++b) {
+            const uint4 x = *reinterpret_cast<const uint4*>(xs + (size_t)b * K + k);
+            float a = acc[b];
+            a = fmaf(w0, bf16lo(x.x), a); a = fmaf(w1, bf16hi(x.x), a);
+            a = fmaf(w2, bf16lo(x.y), a); a = fmaf(w3, bf16hi(x.y), a);
+            a = fmaf(w4, bf16lo(x.z), a); a = fmaf(w5, bf16hi(x.z), a);
+            a = fmaf(w6, bf16lo(x.w), a); a = fmaf(w7, bf16hi(x.w), a);
+            acc[b] = a;
+        }
+    } else {
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            const float4 x = *reinterpret_cast<const float4*>(xs + (size_t)b * K + k);
+            float a = acc[b];
+            a = fmaf(__uint_as_float(w.x), x.x, a); a = fmaf(__uint_as_float(w.y), x.y, a);
+            a = fmaf(__uint_as_float(w.z), x.z, a); a = fmaf(__uint_as_float(w.w), x.w, a);
+            acc[b] = a;
+        }
     }
 }
 
@@ -138,18 +157,17 @@ DEVINL void block_range(int total, int parts, int idx, int& first, int& count) {
     count = base + (idx < rem ? 1 : 0);
 }
 
-template <int NB, int PRO, int EPI>
+template <typename WT, int NB, int PRO, int EPI>
 __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a) {
-    typedef float WT;
-    constexpr int EPL = 4;                             // weights per 16-byte load
+    constexpr int EPL = WTraits<WT>::EPL;              // weights per 16-byte load
     constexpr int STEP = 32 * EPL;                     // elements per chunk
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int K = a.K;
     constexpr bool SEGS = (PRO == PRO_SHIFT || PRO == PRO_PLAIN) && EPI == EPI_STORE;  // may have several inputs
     constexpr bool STORES = EPI == EPI_STORE || EPI == EPI_STORE_GLU;
     const int nseg = SEGS ? max(1, a.nseg) : 1;
-    float* xs = reinterpret_cast<float*>(smem_raw);                                        // [nseg][NB][K]
-    float* red = reinterpret_cast<float*>(smem_raw + (size_t)nseg * NB * K * sizeof(float));   // [NB*32]
+    WT* xs = reinterpret_cast<WT*>(smem_raw);                                              // [nseg][NB][K]
+    float* red = reinterpret_cast<float*>(smem_raw + (size_t)nseg * NB * K * sizeof(WT));  // [NB*32]
     float* pieces = red + NB * 32;                     // [rows_cta][slots][NB] / Cand scratch
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int b0 = blockIdx.y * NB;
@@ -229,12 +247,12 @@ __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a)
         for (int sg = 0; sg < nseg; ++sg)
             for (int b = 0; b < nb; ++b)
                 for (int i = tid; i < K; i += kSimtThreads)
-                    xs[((size_t)sg * NB + b) * K + i] = a.in[((size_t)sg * a.B + b0 + b) * K + i];
+                    put_x(xs + ((size_t)sg * NB + b) * K + i, a.in[((size_t)sg * a.B + b0 + b) * K + i]);
     } else if constexpr (PRO == PRO_GNORM) {
         auto put = [&](int i, float v) {
             if (a.gn_w) v *= a.gn_w[i];
             if (a.gn_gate) v *= a.act == ACT_SILU ? silu(a.gn_gate[i]) : sigmoid(a.gn_gate[i]);
-            xs[i] = v;
+            put_x(xs + i, v);
         };
         if (a.gn_group == 0 || a.gn_group == a.gn_n) {
             float r = 1.0f;
@@ -255,11 +273,11 @@ __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a)
             }
         }
         if (a.gn_tail != nullptr) {
-            for (int i = a.gn_n + tid; i < a.gn_tail_at; i += kSimtThreads) xs[i] = 0.0f;
+            for (int i = a.gn_n + tid; i < a.gn_tail_at; i += kSimtThreads) put_x(xs + i, 0.0f);
             for (int i = a.gn_tail_at + tid; i < K; i += kSimtThreads)
-                xs[i] = i < a.gn_tail_at + a.gn_tail_n ? a.gn_tail[i - a.gn_tail_at] : 0.0f;
+                put_x(xs + i, i < a.gn_tail_at + a.gn_tail_n ? a.gn_tail[i - a.gn_tail_at] : 0.0f);
         } else {
-            for (int i = a.gn_n + tid; i < K; i += kSimtThreads) xs[i] = 0.0f;
+            for (int i = a.gn_n + tid; i < K; i += kSimtThreads) put_x(xs + i, 0.0f);
         }
     } else {
         const bool writer = (blockIdx.x == 0);
@@ -274,7 +292,7 @@ __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a)
 #pragma unroll
                 for (int j = 0; j < kSimtMaxJ; ++j) {
                     const int i = tid + j * kSimtThreads;
-                    hv[j] = (i < K) ? ((const float*)a.embed)[(size_t)tok * K + i] * a.embed_scale : 0.0f;
+                    hv[j] = (i < K) ? WTraits<WT>::elem(a.embed, (size_t)tok * K + i) * a.embed_scale : 0.0f;
                 }
             } else if (a.raw == nullptr) {
                 // nothing pending: h_in already is the layer's input (layer-wise tracing)
@@ -323,13 +341,13 @@ __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a)
                     const float c = hv[j] * r2 * wnorm[j], p = first ? 0.0f : a.shift_state[i];
                     if (writer) a.x_f32[i] = c;
                     for (int sg = 0; sg < nseg; ++sg)
-                        xs[(size_t)sg * K + i] = c + (p - c) * a.mu[(size_t)sg * K + i];
+                        put_x(xs + (size_t)sg * K + i, c + (p - c) * a.mu[(size_t)sg * K + i]);
                 }
             } else {
 #pragma unroll
                 for (int j = 0; j < kSimtMaxJ; ++j) {
                     const int i = tid + j * kSimtThreads;
-                    if (i < K) xs[(size_t)b * K + i] = hv[j] * r2 * wnorm[j];
+                    if (i < K) put_x(xs + (size_t)b * K + i, hv[j] * r2 * wnorm[j]);
                 }
             }
         }
@@ -337,7 +355,7 @@ __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a)
     // rows of a partial batch chunk that do not exist read zeros
     for (int sg = 0; sg < nseg; ++sg)
         for (int b = nb; b < NB; ++b)
-            for (int i = tid; i < K; i += kSimtThreads) xs[((size_t)sg * NB + b) * K + i] = 0.0f;
+            for (int i = tid; i < K; i += kSimtThreads) put_x(xs + ((size_t)sg * NB + b) * K + i, 0.0f);
     __syncthreads();
     pdl_launch();
     stamp(a.ts, 2);
@@ -356,7 +374,7 @@ __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a)
             const int nfull = has_tail ? ncs - 1 : ncs;
             const WT* p = row_ptr(row_first + rl) + (size_t)cc * STEP + lane * EPL;
             int k = cc * STEP + lane * EPL;
-            const float* xr = xs;                         // the input of this row's segment
+            const WT* xr = xs;                            // the input of this row's segment
             if constexpr (SEGS) {
                 if (nseg > 1) xr = xs + (size_t)((row_first + rl) / a.seg_rows) * NB * K;
             }
@@ -369,7 +387,7 @@ __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a)
 #pragma unroll
                 for (int q = 0; q < 8; ++q) w[q] = ldg_stream16(p + q * STEP);
 #pragma unroll
-                for (int q = 0; q < 8; ++q) fma16<NB>(acc, w[q], xr, K, k + q * STEP);
+                for (int q = 0; q < 8; ++q) fma16<WT, NB>(acc, w[q], xr, K, k + q * STEP);
                 p += 8 * STEP;
                 k += 8 * STEP;
             }
@@ -378,15 +396,15 @@ __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a)
 #pragma unroll
                 for (int q = 0; q < 4; ++q) w[q] = ldg_stream16(p + q * STEP);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) fma16<NB>(acc, w[q], xr, K, k + q * STEP);
+                for (int q = 0; q < 4; ++q) fma16<WT, NB>(acc, w[q], xr, K, k + q * STEP);
                 p += 4 * STEP;
                 k += 4 * STEP;
                 j += 4;
             }
             if (j + 2 <= nfull) {
                 uint4 w0 = ldg_stream16(p), w1 = ldg_stream16(p + STEP);
-                fma16<NB>(acc, w0, xr, K, k);
-                fma16<NB>(acc, w1, xr, K, k + STEP);
+                fma16<WT, NB>(acc, w0, xr, K, k);
+                fma16<WT, NB>(acc, w1, xr, K, k + STEP);
                 p += 2 * STEP;
                 k += 2 * STEP;
                 j += 2;
@@ -394,7 +412,7 @@ __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a)
             for (; j < ncs; ++j) {
                 if (k < K) {
                     uint4 w0 = ldg_stream16(p);
-                    fma16<NB>(acc, w0, xr, K, k);
+                    fma16<WT, NB>(acc, w0, xr, K, k);
                 }
                 p += STEP;
                 k += STEP;
@@ -462,15 +480,15 @@ __global__ void __launch_bounds__(kSimtThreads, 1) gemv_kernel(const GemvArgs a)
                 }
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    fma16<NB>(acc0, wa[j], xs, K, k + j * STEP);
-                    fma16<NB>(acc1, wb[j], xs, K, k + j * STEP);
+                    fma16<WT, NB>(acc0, wa[j], xs, K, k + j * STEP);
+                    fma16<WT, NB>(acc1, wb[j], xs, K, k + j * STEP);
                 }
             }
             for (; k < K; k += STEP) {
                 uint4 wa = ldg_stream16(p0 + k);
                 uint4 wb = ldg_stream16(p1 + k);
-                fma16<NB>(acc0, wa, xs, K, k);
-                fma16<NB>(acc1, wb, xs, K, k);
+                fma16<WT, NB>(acc0, wa, xs, K, k);
+                fma16<WT, NB>(acc1, wb, xs, K, k);
             }
 #pragma unroll
             for (int b = 0; b < NB; ++b) { acc0[b] = warp_sum(acc0[b]); acc1[b] = warp_sum(acc1[b]); }

@@ -1028,7 +1028,7 @@ struct LayeredPass {
             a.W1 = x.gateup.w1;
             residual_args(a, x.norm2);
             a.act = m->ff_act;
-            uint16_t* gu_x = m->es == 2 && x.gateup.gp.N % 64 == 0 ? (uint16_t*)c->gu_part : nullptr;     // the down projection's operand
+            uint16_t* gu_x = hands_over_x(m, x.gateup.gp, x.down.gp, R) ? (uint16_t*)c->gu_part : nullptr;     // the down projection's operand
             a.out = c->gu_part;
             a.out_x = gu_x;
             launch_gemv(ln, "gateup", c, R, a, x.gateup.gp, PRO_NORM, EPI_GATEUP);

@@ -152,6 +152,7 @@ struct oxg4_model {
     int num_sms = 148;
     bool use_pdl = true;
     bool timeline = false;        // OXG4_TIMELINE: kernels stamp the global timer into the cache's buffer     // pull later kernels' weights into L2 during latency-bound kernels
+    bool long_launches = false;   // one-row projections through gemv_kernel, see pick_one_row_path
     bool finalized = false;
     std::map<std::string, Tensor> tensors;
     // upload path: two pinned staging slots; the host copy into one overlaps the DMA out of the other
@@ -466,9 +467,9 @@ static int32_t shared_sm_attrs(F* kernel) {
     CK(cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
     return OXG4_OK;
 }
-template <int NB>
+template <typename WT, int NB>
 static int32_t set_gemv_attrs() {
-#define SETA(PRO, EPI) TRY((allow_big_smem(gemv_kernel<NB, PRO, EPI>)))
+#define SETA(PRO, EPI) TRY((allow_big_smem(gemv_kernel<WT, NB, PRO, EPI>)))
     SETA(PRO_NORM, EPI_STORE);
     SETA(PRO_NORM, EPI_GATEUP);
     SETA(PRO_NORM, EPI_LOGITS);
@@ -478,7 +479,7 @@ static int32_t set_gemv_attrs() {
         SETA(PRO_GNORM, EPI_STORE);
     }
     SETA(PRO_PLAIN, EPI_STORE);
-    SETA(PRO_PLAIN, EPI_STORE_GLU);
+    if constexpr (sizeof(WT) == 4) SETA(PRO_PLAIN, EPI_STORE_GLU);     // several rows of listed layers
 #undef SETA
     return OXG4_OK;
 }
@@ -501,6 +502,27 @@ static int32_t set_attn_attrs() {
 }
 
 static int32_t finalize_layered(oxg4_model* m);
+// One activation row, BF16 weights: gemv_mma_kernel hides the gaps between launches but streams at 5.0 - 5.2 TB/s, gemv_kernel fills its
+// SMs and streams at 6.0. The second takes the models whose projections are long: 1 MB per SM and launch on average over the layers. Steps
+// at 100 positions with the first / the second, us: ~1B widths (0.09 MB) 893 / 1059, ~4B (0.32) 1877 / 1961, twelve listed layers of width
+// 2560 (0.4) 821 / 878, ~12B (0.76) 1452 / 1388 and at 1000 positions 1514 / 1602 (its evict-first copies leave K/V rows in L2), six layers of
+// ~27B (1.4) 1502 / 1286, twelve listed layers of width 4096 (1.6) 1252 / 1132. Not launch by launch: behind one that fills its SMs the
+// CTAs of one that takes half an SM gather two by two (~27B, only the feed-forward and the head through gemv_kernel: 1457).
+static void pick_one_row_path(oxg4_model* m) {
+    double bytes = 0;
+    int launches = 0;
+    auto add = [&](const GemvPlan& p) {
+        if (p.N > 0) { bytes += (double)p.N * p.K * m->es; ++launches; }
+    };
+    for (const LayerPlan& l : m->layers) {
+        if (m->layered) {
+            for (const Proj* x : {&l.mix.in, &l.mix.uq, &l.mix.o, &l.mix.gateup, &l.mix.down}) add(x->gp);
+        } else {
+            add(l.p_qkv); add(l.p_o); add(m->p_gateup); add(m->p_down);
+        }
+    }
+    m->long_launches = m->es == 2 && bytes >= 1e6 * launches * m->num_sms;
+}
 template <typename F>
 static bool each_mma(const F& f);
 template <int MB>
@@ -516,10 +538,11 @@ static int32_t set_projection_attrs(oxg4_model* m) {
         int32_t status = OXG4_OK;
         each_mma([&](int, int, int, auto* k) { return (status = shared_sm_attrs(k)) != OXG4_OK; });
         TRY(status);
+        TRY((set_gemv_attrs<uint16_t, 1>()));
         TRY(set_rows_attrs<8>());
         TRY(set_rows_attrs<16>());
     } else {
-        TRY((set_gemv_attrs<1>())); TRY((set_gemv_attrs<2>())); TRY((set_gemv_attrs<4>()));
+        TRY((set_gemv_attrs<float, 1>())); TRY((set_gemv_attrs<float, 2>())); TRY((set_gemv_attrs<float, 4>()));
     }
     return allow_big_smem(topk_stage2_kernel);
 }
@@ -535,6 +558,7 @@ extern "C" int32_t oxg4_model_finalize(oxg4_model* m) {
     }
     if (m->layered) {
         TRY(finalize_layered(m));
+        pick_one_row_path(m);
         TRY(set_projection_attrs(m));
         CK(cudaDeviceSynchronize());
         m->finalized = true;
@@ -652,6 +676,7 @@ extern "C" int32_t oxg4_model_finalize(oxg4_model* m) {
     m->p_down = make_plan(H, m->I, m->es, m->num_sms, 1);
     m->p_lm = make_plan(m->Vloc, H, m->es, m->num_sms, 1);
     m->p_lm_simt_grid = std::min(m->num_sms, std::max(1, (m->Vloc + 2 * kSimtWarps - 1) / (2 * kSimtWarps)));
+    pick_one_row_path(m);
     TRY(set_projection_attrs(m));
 #define SA1(D, G) TRY((set_attn_attrs<uint16_t, D, G>())); TRY((set_attn_attrs<float, D, G>()));
 #define SA(D) SA1(D, 1) SA1(D, 2) SA1(D, 4) SA1(D, 8)
@@ -1523,10 +1548,10 @@ struct Launcher {
     }
 };
 
-template <int NB>
+template <typename WT, int NB>
 static void (*pick_gemv(int pro, int epi))(const GemvArgs) {
 #define PG(PRO, EPI) \
-    if (pro == PRO && epi == EPI) return gemv_kernel<NB, PRO, EPI>;
+    if (pro == PRO && epi == EPI) return gemv_kernel<WT, NB, PRO, EPI>;
     PG(PRO_NORM, EPI_STORE)
     PG(PRO_PLAIN, EPI_STORE)
     PG(PRO_NORM, EPI_GATEUP)
@@ -1536,7 +1561,7 @@ static void (*pick_gemv(int pro, int epi))(const GemvArgs) {
         PG(PRO_SHIFT, EPI_STORE)
         PG(PRO_GNORM, EPI_STORE)
     }
-    PG(PRO_PLAIN, EPI_STORE_GLU)
+    if constexpr (sizeof(WT) == 4) { PG(PRO_PLAIN, EPI_STORE_GLU) }
 #undef PG
     return nullptr;
 }
@@ -1603,6 +1628,22 @@ static bool gemv_mma_ring(GemvArgs* a, const GemvPlan& p, int nb, int pro, int e
     return nx <= kGmMaxRows && (a->places >= 2 || (nb == 1 && a->places == 1));     // the A operand's half that is kept has eight rows
 }
 
+// The kernel of a projection of `rows` rows outside the tcgen05 path, and for the ring its geometry
+enum GemvPath { GEMV_SIMT, GEMV_RING, GEMV_ROWS };
+static GemvPath gemv_path(const oxg4_model* m, const GemvPlan& p, int rows, int pro, int epi, GemvArgs* a, size_t* smem) {
+    if (m->es == 4 || (rows == 1 && m->long_launches)) return GEMV_SIMT;
+    for (a->bpp = rows; rows <= kGmMaxRows && a->bpp > 0; --a->bpp)      // as many activation rows per pass as shared memory allows
+        if (gemv_mma_ring(a, p, a->bpp, pro, epi, smem)) return GEMV_RING;
+    return rows <= kGmMaxRows ? GEMV_RING : GEMV_ROWS;
+}
+// Whether the gate/up launch may leave the down projection's BF16 operand
+static bool hands_over_x(const oxg4_model* m, const GemvPlan& gateup, const GemvPlan& down, int rows) {
+    GemvArgs g{}, d{};
+    size_t smem;
+    return gateup.N % 64 == 0 && gemv_path(m, gateup, rows, PRO_NORM, EPI_GATEUP, &g, &smem) == GEMV_RING &&
+           gemv_path(m, down, rows, PRO_PLAIN, EPI_STORE, &d, &smem) == GEMV_RING;
+}
+
 static void launch_gemv(Launcher& ln, const char* kind, oxg4_cache* c, int rows, GemvArgs a, const GemvPlan& p, int pro,
                         int epi) {
     oxg4_model* m = c->m;
@@ -1620,7 +1661,9 @@ static void launch_gemv(Launcher& ln, const char* kind, oxg4_cache* c, int rows,
                          kMaxHidden);
         return;
     }
-    if (m->es == 2 && B > kGmMaxRows) {
+    size_t ring_smem = 0;
+    const GemvPath path = gemv_path(m, p, B, pro, epi, &a, &ring_smem);
+    if (path == GEMV_ROWS) {
         // as many activation rows per pass as shared memory allows (at most 16)
         auto need = [&](int nb) { return (((size_t)nb * mma_x_stride(p.K) * 2 + 15) & ~(size_t)15) + 128 + (size_t)2 * mma_rows_per_pass(nb > 8 ? 16 : 8) * kGrWarps * nb * 4; };
         int bpp = std::min(B, 16);
@@ -1633,28 +1676,21 @@ static void launch_gemv(Launcher& ln, const char* kind, oxg4_cache* c, int rows,
         ln.go(kind, bpp <= 8 ? pick_rows<8>(pro, epi) : pick_rows<16>(pro, epi), dim3(p.grid, (B + bpp - 1) / bpp, 1), dim3(kGrThreads), need(bpp), a);
         return;
     }
-    if (m->es == 2) {
-        // as many activation rows per pass as shared memory allows
-        size_t smem = 0;
-        int bpp = B;
-        while (!gemv_mma_ring(&a, p, bpp, pro, epi, &smem)) {
-            if (bpp == 1) {
-                ln.status = fail(OXG4_UNSUPPORTED, "projection %s needs %zu bytes of shared memory", kind, smem);
-                return;
-            }
-            --bpp;
+    if (path == GEMV_RING) {
+        if (a.bpp == 0) {
+            ln.status = fail(OXG4_UNSUPPORTED, "projection %s needs %zu bytes of shared memory", kind, ring_smem);
+            return;
         }
-        a.bpp = bpp;
         CUtensorMap map0, map1;
         const uint64_t rows = epi == EPI_GATEUP ? p.N / 2 : p.N;
         ln.status = encode_bf16_2d(&map0, a.W0, rows, (uint64_t)p.K, (uint32_t)a.box_rows);
         if (ln.status != OXG4_OK) return;
         ln.status = encode_bf16_2d(&map1, epi == EPI_GATEUP ? a.W1 : a.W0, rows, (uint64_t)p.K, (uint32_t)a.box_rows);
         if (ln.status != OXG4_OK) return;
-        ln.go(kind, pick_mma(pro, epi, p.K > 3 * 4 * kGmThreads), dim3(p.grid, (B + bpp - 1) / bpp, 1), dim3(kGmThreads), smem, map0, map1, a);
+        ln.go(kind, pick_mma(pro, epi, p.K > 3 * 4 * kGmThreads), dim3(p.grid, (B + a.bpp - 1) / a.bpp, 1), dim3(kGmThreads), ring_smem, map0, map1, a);
         return;
     }
-    // f32 weights: SIMT kernel
+    // 16-byte loads into registers
     a.cpr = p.cpr;
     a.slots = p.slots;
     const size_t limit = 226 * 1024;
@@ -1670,7 +1706,8 @@ static void launch_gemv(Launcher& ln, const char* kind, oxg4_cache* c, int rows,
         ln.status = fail(OXG4_UNSUPPORTED, "projection %s needs %zu bytes of shared memory", kind, smem);
         return;
     }
-    auto fn = nb == 1 ? pick_gemv<1>(pro, epi) : nb == 2 ? pick_gemv<2>(pro, epi) : pick_gemv<4>(pro, epi);
+    auto fn = m->es == 2 ? pick_gemv<uint16_t, 1>(pro, epi) : nb == 1 ? pick_gemv<float, 1>(pro, epi)
+            : nb == 2 ? pick_gemv<float, 2>(pro, epi) : pick_gemv<float, 4>(pro, epi);
     dim3 grid(epi == EPI_LOGITS ? m->p_lm_simt_grid : p.grid, (B + nb - 1) / nb, 1);
     ln.go(kind, fn, grid, dim3(kSimtThreads), smem, a);
 }
@@ -1800,6 +1837,7 @@ static QkvPostFn pick_qkv_post(int kv_dtype, int D, bool few) {
 //     size 256 up to 1.1 there and 1.2 at 9000
 //   fewer: eight heads 0.65 - 0.9 below 16 positions per CTA, 1.0 - 1.4 at 30 - 50; four 0.84 - 1.0 at 30 - 50, 1.1 at 100; one or two 0.83 -
 //     1.0 at 100, 1.1 - 1.2 at 300
+// Steps of one sequence between launches that fill their SMs (gemv_kernel) keep the second (six layers of ~27B widths 1277 / 1350 us).
 // `vis` is what the table has room for, as everywhere in the geometry of a step: the captured step serves all positions.
 static bool step_kernel(bool dealt, int ctas, int sms, int splits, int G, int D, int vis, int kv_dtype) {
     const bool bf16 = kv_dtype == OXG4_BF16;
@@ -1916,7 +1954,7 @@ static void launch_attention(Launcher& ln, oxg4_cache* c, const RowSet& rs, int 
     const bool few = ctas <= m->num_sms;
     int unit = p.G;                              // query heads of a unit (attn_step_kernel)
     while (unit > 1 && 2 * a.n_splits * p.Nkv * (p.G / unit) * R <= m->num_sms) unit /= 2;
-    const bool step = !kv_in_cache && step_kernel(unit < p.G, ctas, m->num_sms, a.n_splits, p.G, D, vis, c->kv_dtype);
+    const bool step = !kv_in_cache && !(m->long_launches && R == 1) && step_kernel(unit < p.G, ctas, m->num_sms, a.n_splits, p.G, D, vis, c->kv_dtype);
     const int NW = !few ? 4 : step ? kAttnStepThreads / 32 : kAttnWarps;
     // attn_decode_kernel: more K/V rows in flight per warp when latency is all that counts (with more than two query heads
     // per kv head the extra rows would spill registers)
@@ -1927,9 +1965,11 @@ static void launch_attention(Launcher& ln, oxg4_cache* c, const RowSet& rs, int 
     auto fn = c->kv_dtype == OXG4_BF16 ? pick_attn<uint16_t>(p.D, step ? unit : p.G, attn_kind, NW, a.n_splits, &floats)
                                        : pick_attn<float>(p.D, step ? unit : p.G, attn_kind, NW, a.n_splits, &floats);
     ln.cluster_x = kv_in_cache ? 0 : a.n_splits;
-    // attn_decode_kernel with an SM per CTA asks for the shared memory that it needs, no more: behind a launch that left its SM the least L1
-    // there is, the instances that spill registers (f32 caches of head size 256, eight heads) took up to 1.45 times as long
-    ln.carveout = kv_in_cache || step || !few ? -1 : std::min<int>(100, (int)((sizeof(float) * floats + 3 * 1024) * 100 / (228 * 1024)) + 1);
+    // Instances of attn_decode_kernel that spill registers, with an SM per CTA, ask for the shared memory that they need, no more: behind a
+    // launch that left its SM the least L1 there is, they took up to 1.45 times as long. The others don't: the change waits for an empty SM
+    // (5 us a layer of the ~27B widths).
+    const bool spills = D == 256 && (c->kv_dtype == OXG4_F32 || p.G == 8);
+    ln.carveout = kv_in_cache || step || !few || !spills ? -1 : std::min<int>(100, (int)((sizeof(float) * floats + 3 * 1024) * 100 / (228 * 1024)) + 1);
     ln.go("attn", fn, dim3(a.n_splits, step ? p.Nkv * (p.G / unit) : p.Nkv, R), dim3(NW * 32), sizeof(float) * floats, a);
     ln.cluster_x = 0;
     ln.carveout = -1;
@@ -2071,7 +2111,7 @@ static Pending run_layers(oxg4_cache* c, Launcher& ln, const RowSet& rs, bool us
     int s_down = rs.chunk ? c->ps_down : c->s_down;
     const bool wide = rs.chunk && c->wide && R > kWideRows;
     // small batches of BF16 models: the feed-forward's values leave the gate/up launch as the down projection's operand
-    uint16_t* gu_x = m->es == 2 && R <= kGmMaxRows && m->I % 32 == 0 ? (uint16_t*)c->gu_raw : nullptr;
+    uint16_t* gu_x = !use_tc && hands_over_x(m, m->p_gateup, m->p_down, R) ? (uint16_t*)c->gu_raw : nullptr;
     if (m->P > 0) ple_prepare(c, ln, rs);
     for (int l = 0; l < L; ++l) {
         const LayerPlan& p = m->layers[l];
@@ -3393,6 +3433,13 @@ extern "C" int32_t oxg4_debug_wait_timeout(oxg4_model* m, oxg4_cache* c, int32_t
         if (err == 23) return fail(OXG4_CUDA, "mbarrier wait: the lanes of a warp got different answers");
         return fail(OXG4_TIMEOUT, "%s: a bounded wait ran out (code %d)", err == 21 ? "mbarrier wait" : "peer flag wait", err);
     }
+    return OXG4_OK;
+}
+
+// Test hook: one-row projections as in a model of long launches (1), of short ones (0), for tables made from now on.
+extern "C" int32_t oxg4_debug_long_launches(oxg4_model* m, int32_t on) {
+    if (!m || !m->finalized) return fail(OXG4_INVALID_ARGUMENT, "null model, or not finalized");
+    m->long_launches = m->es == 2 && on != 0;
     return OXG4_OK;
 }
 

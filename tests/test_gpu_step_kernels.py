@@ -4,6 +4,7 @@ heads than a key/value head has, positions around split and window edges."""
 import numpy as np
 import pytest
 
+import layered_util
 from util import build_pair, pkg, small_cfg, syn
 
 pytestmark = pytest.mark.gpu
@@ -11,6 +12,15 @@ pytestmark = pytest.mark.gpu
 # relative 2-norm of a row's logits: a layer and the head round four operands to BF16 (2^-9 each), and two orders of the same sums
 # may round any of them the other way
 TOL = 4 * 2.0 ** -9
+
+
+@pytest.fixture(params=["short", "long"])
+def launches(request):
+    """Makes a BF16 model take the one-row projections of short or of long launches."""
+    def choose(state):
+        pkg._native.check(pkg._native.lib().oxg4_debug_long_launches(state._h, int(request.param == "long")))
+        return request.param
+    return choose
 
 
 @pytest.mark.parametrize("hidden,inter,heads,head_dim,vocab,batch,tcgen05", [
@@ -28,10 +38,12 @@ TOL = 4 * 2.0 ** -9
     (264, 136, 2, 64, 301, 9, False), (1160, 2080, 2, 128, 20011, 15, False),   # csrc/gemv_rows.cuh
     (264, 96, 2, 64, 301, 17, False),       # sixteen rows and one
     (264, 20000, 2, 64, 300, 9, False)])    # nine rows, of the down projection five at a time
-def test_projections_of_few_rows(hidden, inter, heads, head_dim, vocab, batch, tcgen05, monkeypatch):
+def test_projections_of_few_rows(hidden, inter, heads, head_dim, vocab, batch, tcgen05, launches, monkeypatch):
     cfg = small_cfg(hidden=hidden, layers=1, heads=heads, kv_heads=1 if heads != 8 else 4, head_dim=head_dim, inter=inter, vocab=vocab,
                     window=64, layer_types=["full_attention"])
     gpu, oracle = build_pair(cfg, "bf16", kv_bf16=True, norm_jitter=0.1)
+    if launches(gpu) == "long" and batch > 1:
+        pytest.skip("one row only")
     if not tcgen05:
         monkeypatch.setenv("OXG4_DISABLE_TCGEN05", "1")        # looked at when a table is made
     table = gpu.new_cache_table([8] * batch, batch=batch, page_tokens=16, kv_dtype=pkg.BF16)
@@ -41,8 +53,9 @@ def test_projections_of_few_rows(hidden, inter, heads, head_dim, vocab, batch, t
         want = np.stack([c.decode_logits(int(x)) for c, x in zip(caches, tokens)])
         got = np.atleast_2d(gpu.decode_token(tokens, table))
         assert (np.linalg.norm(got - want, axis=1) / np.linalg.norm(want, axis=1)).max() <= TOL
-        if batch > 1 and t == 0:                               # the fused arg-max, one position on
-            best = gpu.decode_topk(tokens, table, 1, 1.0, False)[0].astype(np.int64)
+        if t == 0:                                             # the fused arg-max, one position on
+            best = gpu.decode_topk(tokens, table, 1, 1.0, False)
+            best = np.array([[best[0][0]]]) if batch == 1 else best[0].astype(np.int64)
             want = np.stack([c.decode_logits(int(x)) for c, x in zip(caches, tokens)])
             top = np.take_along_axis(want, best, 1)[:, 0]
             assert (want.max(1) - top <= 2 * TOL * np.linalg.norm(want, axis=1)).all()
@@ -101,3 +114,14 @@ def test_one_launch_or_three_beside_tcgen05(head_dim, heads, kv_heads, batch, ro
         got = gpu.decode_token(tokens, table)
         # with the bound on the attention's output above
         assert (np.linalg.norm(got - want, axis=1) / np.linalg.norm(want, axis=1)).max() <= TOL + 2.0 ** -6, t
+
+
+# a mechanism alone: BF16 operands of its projections and of the head, recurrent state or cache beside them
+@pytest.mark.parametrize("layer", [
+    layered_util.wkv(2, 64, ff=96), layered_util.lightning(2, 32, 64, (0.9, 0.99), ff=72), layered_util.latent(3, 32, 48, 64, 80, 16, ff=136),
+    layered_util.retention(3, 32, 64, (0.8, 0.95, 0.99), ff=200), layered_util.attention(4, 2, 32, 64, ff=104)], ids=lambda x: x["type"])
+def test_one_row_of_listed_layers(layer, launches):
+    pair = layered_util.Pair(layered_util.config([layer], width=100), "bf16", seed=5)
+    launches(pair.state)
+    tokens = pair.prompt(30, 6)
+    assert layered_util.error(layered_util.feed(pair, pair.table(40), tokens, [1]), pair.want(tokens)) <= 3e-2
