@@ -357,9 +357,11 @@ def main():
     peak, peak_kind = peaks()
     gu_ms = r["prof"].get("gateup", float("nan"))
     achieved = r["parts"]["gateup_launch"] / (gu_ms * 1e-3) / 1e9
-    roofline = {"bound": "hbm", "kernel": ("gemv_mma_kernel<PRO_NORM, EPI_GATEUP>" if B == 1 else
-                           "tc_gemm_kernel (tcgen05, gate and up maps)" if B <= 64 else
-                           "gemv_mma_kernel<PRO_NORM, EPI_GATEUP>") + " (gate/up projection)",
+    # as the library picks it for BF16 weights (one sequence with projections of more than 1 MB per SM, which take gemv_kernel, is no workload)
+    gu_kernel = ("gemv_mma_kernel<PRO_NORM, EPI_GATEUP>" if B < (8 if tp > 1 else 2) else
+                 "tc_gemm_kernel (tcgen05, gate and up maps)" if B <= 256 else
+                 "gemv_rows_kernel<PRO_NORM, EPI_GATEUP>")
+    roofline = {"bound": "hbm", "kernel": gu_kernel + " (gate/up projection)",
                 "achieved": achieved, "peak": peak, "peak_kind": f"of {peak_kind}", "unit": "GB/s",
                 "frac": achieved / peak, "traffic": NCU_TRAFFIC_BYTES.get(args.workload) if tp == 1 else None,
                 "bytes_per_launch": r["parts"]["gateup_launch"], "ms_per_launch": gu_ms,

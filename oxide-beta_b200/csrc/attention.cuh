@@ -55,7 +55,7 @@ struct AttnArgs {
     unsigned int* ticket;    // [B, Nkv]
     float* out;              // [B, Nq * D]
     unsigned long long* ts;  // optional timeline slots of this launch (4 entries) or null
-    unsigned long long* ts_mid;  // optional: one more stamp, taken when the CTA's own partial is complete
+    unsigned long long* ts_mid;  // optional: further stamps inside the kernel (attn_step_kernel three, attn_decode_kernel one to four)
 };
 
 template <typename KT, int EPT> struct KVec;

@@ -151,7 +151,7 @@ struct oxg4_model {
     cudaStream_t stream = nullptr;
     int num_sms = 148;
     bool use_pdl = true;
-    bool timeline = false;        // OXG4_TIMELINE: kernels stamp the global timer into the cache's buffer     // pull later kernels' weights into L2 during latency-bound kernels
+    bool timeline = false;        // OXG4_TIMELINE: kernels stamp the global timer into the cache's buffer
     bool long_launches = false;   // one-row projections through gemv_kernel, see pick_one_row_path
     bool finalized = false;
     std::map<std::string, Tensor> tensors;
@@ -460,7 +460,7 @@ static int32_t allow_big_smem(F* kernel) {
     return OXG4_OK;
 }
 
-// SIMT projections: two successive launches share an SM, so the split of its memory must not change between them
+// gemv_mma_kernel and attn_step_kernel: two successive launches share an SM, so the split of its memory must not change between them
 template <typename F>
 static int32_t shared_sm_attrs(F* kernel) {
     TRY(allow_big_smem(kernel));
@@ -1427,7 +1427,7 @@ struct Launcher {
     int carveout = -1;            // >= 0: the next kernel prefers this percentage of an SM's memory as shared memory
     int cluster_x = 0;            // > 0: launch the next kernel with thread-block clusters of this many CTAs along x
     bool coop = false;            // launch the next kernel cooperatively (all CTAs resident at once), without PDL
-    bool early = false;           // decode step: SIMT projections let their successor start before they wait (see gemv.cuh)
+    bool early = false;           // decode step: gemv_mma_kernel and attn_step_kernel let their successor start before they wait (see gemv_mma.cuh)
     int kernels = 0;
     unsigned long long* ts() const { return (ts_base && kernels < kMaxTimeline) ? ts_base + (size_t)kernels * 4 : nullptr; }
     int32_t status = OXG4_OK;
@@ -1603,7 +1603,9 @@ static void (*pick_rows(int pro, int epi))(const GemvArgs) {
 // Shared memory of a small-batch projection. Two launches in a row share an SM, so that the second one's weights arrive while the
 // first still runs, but no SM may get two CTAs of one launch: the launch would run on some of the SMs only (seen as gate/up and down
 // launches of the ~4B model that took 11 us longer). A launch that may find SMs empty beside others that an attention or row kernel
-// fills, that is an output projection, therefore claims more than half an SM, and the others leave room for one of these.
+// fills, that is an output projection, therefore claims more than half an SM, and the others leave room for one of these. (With the 1 KB
+// that the hardware keeps per CTA and the static parts, 108 KB fit beside 116: a ring that comes closer to kShareBoth than that starts
+// only when the output projection ahead of it has left the SM.)
 constexpr size_t kShareBoth = 110 * 1024, kShareAlone = 116 * 1024, kSmemMost = 226 * 1024;
 static size_t sm_share(int pro, int epi) { return epi == EPI_STORE && (pro == PRO_PLAIN || pro == PRO_GNORM) ? kShareAlone : kShareBoth; }
 
