@@ -153,11 +153,15 @@ DEVINL void norm_rotate(float (&t)[EPT], const float (&w)[EPT], const C& cs, con
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     const NT r = (NT)1 / sqrt(ss / (NT)(32 * EPT) + (NT)eps);
+    if (rotate) {                                      // one branch around the shuffles, not one for each of them
 #pragma unroll
-    for (int e = 0; e < EPT; ++e) {
-        NT v = (NT)t[e] * r * (NT)w[e];
-        if (rotate) v = v * (NT)cs(e) + __shfl_xor_sync(0xffffffffu, v, 16) * (NT)sn(e);
-        t[e] = (float)v;
+        for (int e = 0; e < EPT; ++e) {
+            const NT v = (NT)t[e] * r * (NT)w[e];
+            t[e] = (float)(v * (NT)cs(e) + __shfl_xor_sync(0xffffffffu, v, 16) * (NT)sn(e));
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < EPT; ++e) t[e] = (float)((NT)t[e] * r * (NT)w[e]);
     }
 }
 // With an f32 cache norm and rotation of a step's token are done in doubles: their roundings in q and k were most of the error of
