@@ -1057,7 +1057,8 @@ static int32_t cache_build(oxg4_cache* c) {
     }
     // From two sequences on the tcgen05 path (up to 256: row blocks of 128 / 256, UMMA N). Steps at 250 positions with it / with
     // gemv_mma.cuh, us: ~4B model, 2 sequences 2330 / 2346, 4 2354 / 2704, 7 2440 / 2800; ~1B model, 4 1084 / 1341; ~12B widths, 4 1637 / 1660;
-    // ~27B widths, 4 1437 / 1560. Tensor-parallel ranks from eight on: theirs has not been timed below
+    // ~27B widths, 4 1437 / 1560. At 230 positions, vocabulary of 32768: eight layers of ~4B widths, 2 sequences 537 / 570, 3 539 / 644; eight of
+    // ~12B, 935 / 962 and 925 / 1068; six of ~27B, 1019 / 1125 and 1028 / 1264. Tensor-parallel ranks from eight on: theirs has not been timed below
     c->use_tc = c->tc_ok && B >= (m->tp > 1 ? 8 : 2) && B <= kPrefillRows;
     c->ls_qkv.assign(L, 1);
     c->ls_o.assign(L, 1);
